@@ -1,15 +1,10 @@
-// Attention kernels that are not tcgen05-shaped.
-//
-// 1. attention_decode_bf16: one query token per sequence against a long KV cache.  HBM-bound (every K and V byte is
-//    read once, the query heads of a KV group share it), so the design goal is streaming the cache: a producer warp
-//    keeps a ring of TMA tile copies in flight (data in flight costs no registers) and four consumer warps run the
-//    arithmetic on warp-level mma.sync tiles fed by ldmatrix (a 128-row tcgen05 tile would be 97 % padding for 4 query
-//    heads).  Split over the sequence only when B * Hkv alone cannot fill the GPU; every consumer warp takes 16
-//    keys of each 64-key tile with an online softmax, warps are merged through shared memory, per-chunk partials
-//    (m, l, O) go to scratch and a second kernel merges chunks.
-// 2. attention_generic<T>: any head_dim <= 256, f32 or bf16, one warp per query row, sequential online softmax --
-//    the reference kernel's own recurrence; used for the f32 entry point and for shapes the tcgen05 kernel
-//    does not cover.
+// Decode attention, which is not tcgen05-shaped: one query token per sequence against a long KV cache.  HBM-bound (every K and V byte is
+// read once, the query heads of a KV group share it), so the design goal is streaming the cache: a producer warp
+// keeps a ring of TMA tile copies in flight (data in flight costs no registers) and four consumer warps run the
+// arithmetic on warp-level mma.sync tiles fed by ldmatrix (a 128-row tcgen05 tile would be 97 % padding for 4 query
+// heads).  Split over the sequence only when B * Hkv alone cannot fill the GPU; every consumer warp takes 16
+// keys of each 64-key tile with an online softmax, warps are merged through shared memory, per-chunk partials
+// (m, l, O) go to scratch and a second kernel merges chunks.
 #include <atomic>
 
 #include "common.cuh"
@@ -409,68 +404,6 @@ __global__ void attention_decode_combine_kernel(const float* __restrict__ part_o
   o[b * o_sb + h * o_sh + d] = __float2bfloat16_rn(oo / ll);
 }
 
-// ------------------------------------------------------------------------------------------------
-template <typename T> __device__ __forceinline__ float ld_as_f(const T* p);
-template <> __device__ __forceinline__ float ld_as_f<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ld_as_f<bf16>(const bf16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void st_from_f(float* p, float v) { *p = v; }
-__device__ __forceinline__ void st_from_f(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
-
-// one warp per (query row, head, batch); lane owns d = lane, lane + 32, ... (up to 8 values: D <= 256)
-template <typename T>
-__global__ void attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                                         T* __restrict__ o, float* __restrict__ lse, const AttnShape s) {
-  pdl_wait();
-  const long long wid = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long rows = static_cast<long long>(s.B) * s.Hq * s.Sq;
-  if (wid >= rows) return;
-  const int i = static_cast<int>(wid % s.Sq);
-  const int h = static_cast<int>((wid / s.Sq) % s.Hq);
-  const int b = static_cast<int>(wid / (static_cast<long long>(s.Sq) * s.Hq));
-  const int hk = h / (s.Hq / s.Hkv);
-  const T* qr = q + b * s.q_sb + h * s.q_sh + i * s.q_ss;
-  const T* kb = k + b * s.k_sb + hk * s.k_sh;
-  const T* vb = v + b * s.v_sb + hk * s.v_sh;
-  float qv[8], acc[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int d = lane + 32 * e;
-    qv[e] = d < s.D ? ld_as_f(qr + d) : 0.0f;
-    acc[e] = 0.0f;
-  }
-  float m = -INFINITY, l = 0.0f;
-  const int last = s.causal ? min(s.Skv - 1, i + (s.Skv - s.Sq)) : s.Skv - 1;
-  for (int j = 0; j <= last; ++j) {
-    const T* kr = kb + j * s.k_ss;
-    const T* vr = vb + j * s.v_ss;
-    float dot = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int d = lane + 32 * e;
-      if (d < s.D) dot += qv[e] * ld_as_f(kr + d);
-    }
-    dot = warp_sum(dot) * s.scale;
-    const float m_new = fmaxf(m, dot);
-    const float corr = expf(m - m_new);
-    const float p = expf(dot - m_new);
-    l = corr * l + p;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const int d = lane + 32 * e;
-      if (d < s.D) acc[e] = corr * acc[e] + p * ld_as_f(vr + d);
-    }
-    m = m_new;
-  }
-  T* orow = o + b * s.o_sb + h * s.o_sh + i * s.o_ss;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int d = lane + 32 * e;
-    if (d < s.D) st_from_f(orow + d, acc[e] / l);
-  }
-  if (lse && lane == 0) lse[(static_cast<long long>(b) * s.Hq + h) * s.Sq + i] = m + logf(l);
-}
-
 }  // namespace
 
 // Raises the decode kernel's dynamic shared-memory limit once per device.
@@ -651,19 +584,5 @@ int attention_decode_bf16_static(const bf16* q, const bf16* k, const bf16* v, bf
   return attention_decode_bf16(q, k, v, o, s, kv_len, kv_len_dev, g_static_decode_scratch_ptr[dev],
                                kStaticDecodeScratchBytes, stream);
 }
-
-template <typename T>
-int attention_generic(const T* q, const T* k, const T* v, T* o, float* lse, const AttnShape& s, cudaStream_t stream) {
-  if (!q || !k || !v || !o || s.B <= 0 || s.Hq <= 0 || s.Hkv <= 0 || s.Sq <= 0 || s.Skv <= 0 || s.D <= 0)
-    return TEENY_ERR_BAD_ARG;
-  if (s.D > 256 || s.Hq % s.Hkv != 0 || (s.causal && s.Skv < s.Sq)) return TEENY_ERR_BAD_ARG;
-  const long long rows = static_cast<long long>(s.B) * s.Hq * s.Sq;
-  const long long blocks = (rows + 3) / 4;
-  if (blocks > 0x7fffffffLL) return TEENY_ERR_BAD_ARG;
-  launch_kernel(attention_generic_kernel<T>, dim3(static_cast<int>(blocks)), dim3(128), 0, stream, 1, q, k, v, o, lse, s);
-  return static_cast<int>(cudaGetLastError());
-}
-template int attention_generic<float>(const float*, const float*, const float*, float*, float*, const AttnShape&, cudaStream_t);
-template int attention_generic<bf16>(const bf16*, const bf16*, const bf16*, bf16*, float*, const AttnShape&, cudaStream_t);
 
 }  // namespace teeny
