@@ -443,29 +443,6 @@ struct SkinnyCfg {
   static constexpr int kSmemBytes = kBarOffset + 1024 + 256;
 };
 
-// Four FP8 E4M3 bytes (k ascending from the low byte) -> two bf16 pairs, exactly.  A byte's seven magnitude bits,
-// placed four bits below the top of a bf16's exponent field, read as the bf16 number 2^-120 times the E4M3 value --
-// also for E4M3 subnormals, which land on bf16 subnormals -- so one multiplication by 2^120 finishes the job.  (The two
-// NaN bytes 0x7f / 0xff decode as +-480; the loader refuses tensors that contain them.)
-// The conversion is what bounds this kernel, and the integer pipe (logic, shifts, byte permutes: half the rate of the
-// FMA pipe) is what bounds the conversion.  So the placement is done by integer multiply-adds, which run on the FMA
-// pipe: with the byte in the low half of a halfword (one permute), x * 16 puts the magnitude at bits 10..4 and the sign
-// at bit 11, and adding 240 * (x & 0x80) carries the sign from bit 11 to bit 15 without touching the rest.  `mul16`
-// is the constant 16 handed in through a register, so that the compiler keeps the multiply-add instead of turning it
-// into a shift on the integer pipe.
-__device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t mul16, uint32_t& lo, uint32_t& hi) {
-  const uint32_t x0 = __byte_perm(w, 0u, 0x4140), x1 = __byte_perm(w, 0u, 0x4342);
-  const uint32_t s0 = x0 & 0x00800080u, s1 = x1 & 0x00800080u;
-  uint32_t t0, t1;
-  asm("mad.lo.u32 %0, %1, %2, 0;\n\tmad.lo.u32 %0, %3, 240, %0;" : "=&r"(t0) : "r"(x0), "r"(mul16), "r"(s0));
-  asm("mad.lo.u32 %0, %1, %2, 0;\n\tmad.lo.u32 %0, %3, 240, %0;" : "=&r"(t1) : "r"(x1), "r"(mul16), "r"(s1));
-  const __nv_bfloat162 k = __halves2bfloat162(__ushort_as_bfloat16(0x7b80), __ushort_as_bfloat16(0x7b80));  // 2^120
-  const __nv_bfloat162 r0 = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&t0), k);
-  const __nv_bfloat162 r1 = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&t1), k);
-  lo = *reinterpret_cast<const uint32_t*>(&r0);
-  hi = *reinterpret_cast<const uint32_t*>(&r1);
-}
-
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -994,6 +971,17 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
   if (swiglu && (w_is_kn || bias || N % 128 != 0)) return TEENY_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (ldx & 7) || (ldw & 7))
     return TEENY_ERR_ALIGNMENT;
+
+  if (!w_is_kn && !push && gemm_rows_takes(M, N, K, ldw, false, kRowsNormNone)) {
+    RowsGemm g{};
+    g.x = x; g.ldx = ldx;
+    g.w = w; g.ldw = ldw;
+    g.bias = bias;
+    g.glu = swiglu;
+    g.y = y; g.ldy = ldy;
+    g.M = M; g.N = N; g.K = K;
+    return gemm_rows(g, stream);
+  }
 
   GemmArgs a{};
   a.M = M; a.N = N; a.K = K; a.ldy = ldy; a.y = y; a.y32 = y32; a.bias = bias;

@@ -260,6 +260,16 @@ struct teeny_hybrid : DecoderBase {
 
 namespace {
 
+RowsGemm rows_call(const void* x, int ldx, const void* w, int ldw, int M, int N, int K, int glu, const void* bias) {
+  RowsGemm g{};
+  g.x = x; g.ldx = ldx;
+  g.w = w; g.ldw = ldw;
+  g.bias = static_cast<const bf16*>(bias);
+  g.glu = glu;
+  g.M = M; g.N = N; g.K = K;
+  return g;
+}
+
 // y[M, N] = x[M, K] W^T (+ bias), in the model's element type; glu: act(gate) * up with N counting both.
 int linear(teeny_hybrid* m, const void* x, int ldx, const void* w, int ldw, void* y, int ldy, int M, int N, int K, cudaStream_t st,
            int glu = 0, const void* bias = nullptr) {
@@ -574,15 +584,46 @@ int norm(teeny_hybrid* m, const float* w, int T, cudaStream_t st) {
                            m->cfg.f32 != 0, st, m->pending_post, m->cfg.residual_mult);
 }
 
+// y[T, N] = norm(residual) W^T: the norm goes along with the projection where nothing is pending and the rows are few.
+int normed_linear(teeny_hybrid* m, const float* norm_w, const void* w, void* y, int ldy, int T, int N, int glu, const void* bias, cudaStream_t st) {
+  const Plan& p = m->p;
+  const int d = m->cfg.width;
+  if (!m->cfg.f32 && !m->pending_delta && d % 8 == 0 && !(reinterpret_cast<uintptr_t>(norm_w) & 15) &&
+      gemm_rows_takes(T, N, d, p.width_ld, false, kRowsNormF32)) {
+    RowsGemm g = rows_call(m->at<float>(p.x), d, w, p.width_ld, T, N, d, glu, bias);
+    g.norm = kRowsNormF32; g.norm_w = norm_w; g.eps = m->cfg.eps;
+    g.y = static_cast<bf16*>(y); g.ldy = ldy;
+    return gemm_rows(g, st);
+  }
+  TEENY_TRY(norm(m, norm_w, T, st));
+  return linear(m, m->at<void>(p.y), p.width_ld, w, p.width_ld, y, ldy, T, N, d, st, glu, bias);
+}
+
+// A sublayer's output x W^T: added into the residual stream at once where the rows are few and no norm comes in between; otherwise
+// (and for the last sublayer, whose output the head's norm and the caller look for there) it is pending in `delta`.
+int sublayer_out(teeny_hybrid* m, const void* x, const void* w, int K, const float* post, bool last, int T, cudaStream_t st) {
+  const Plan& p = m->p;
+  const int d = m->cfg.width;
+  if (!m->cfg.f32 && !post && !last && gemm_rows_takes(T, d, K, K, false, kRowsNormNone)) {
+    RowsGemm g = rows_call(x, K, w, K, T, d, K, 0, nullptr);
+    g.add32 = m->at<float>(p.x); g.ldy = d;
+    m->pending_delta = false;
+    return gemm_rows(g, st);
+  }
+  m->pending_delta = true;
+  m->pending_post = post;
+  return linear(m, x, K, w, K, m->at<void>(p.delta), p.width_ld, T, d, K, st);
+}
+
 int run_layers(teeny_hybrid* m, const int* ids, const StepShape& s, cudaStream_t st) {
   const Plan& p = m->p;
   const int d = m->cfg.width;
-  void *y = m->at<void>(p.y), *delta = m->at<void>(p.delta), *act = m->at<void>(p.act);
+  void* act = m->at<void>(p.act);
   TEENY_TRY(embedding_scaled(ids, m->embed, m->at<float>(p.x), s.T, d, m->cfg.vocab, m->cfg.embed_scale, m->cfg.f32 != 0, st));
   m->pending_delta = false;
   for (const Layer& L : p.layers) {
-    TEENY_TRY(norm(m, L.norm1, s.T, st));
-    TEENY_TRY(linear(m, y, p.width_ld, L.w_in, p.width_ld, m->at<void>(p.proj), L.n_in, s.T, L.n_in, d, st, 0, L.in_bias));
+    const bool last = &L == &p.layers.back();
+    TEENY_TRY(normed_linear(m, L.norm1, L.w_in, m->at<void>(p.proj), L.n_in, s.T, L.n_in, 0, L.in_bias, st));
     for (const Branch& b : L.branches) {
       if (b.full()) TEENY_TRY(run_full_attention(m, L, b, s, st));
       else if (b.c.kind == TEENY_HYBRID_ATTENTION) TEENY_TRY(run_attention(m, L, b, s, st));
@@ -590,15 +631,10 @@ int run_layers(teeny_hybrid* m, const int* ids, const StepShape& s, cudaStream_t
       else if (b.c.kind == TEENY_HYBRID_MIN_GRU) TEENY_TRY(run_min_gru(m, L, b, s, st));
       else TEENY_TRY(run_matrix_state(m, L, b, s, st));
     }
-    TEENY_TRY(linear(m, m->at<void>(p.mix), L.n_out, L.w_out, L.n_out, delta, p.width_ld, s.T, d, L.n_out, st));
-    m->pending_delta = true;
-    m->pending_post = L.norm1_post;
+    TEENY_TRY(sublayer_out(m, m->at<void>(p.mix), L.w_out, L.n_out, L.norm1_post, last && !L.ff, s.T, st));
     if (L.ff) {
-      TEENY_TRY(norm(m, L.norm2, s.T, st));
-      TEENY_TRY(linear(m, y, p.width_ld, L.gate_up, p.width_ld, act, L.ff, s.T, 2 * L.ff, d, st, L.act));
-      TEENY_TRY(linear(m, act, L.ff, L.down, L.ff, delta, p.width_ld, s.T, d, L.ff, st));
-      m->pending_delta = true;
-      m->pending_post = L.norm2_post;
+      TEENY_TRY(normed_linear(m, L.norm2, L.gate_up, act, L.ff, s.T, 2 * L.ff, L.act, nullptr, st));
+      TEENY_TRY(sublayer_out(m, act, L.down, L.ff, L.norm2_post, last, s.T, st));
     }
   }
   return 0;
@@ -690,6 +726,7 @@ int teeny_hybrid_create(const teeny_hybrid_config* cfg, const teeny_hybrid_layer
   if (rc == 0 && workspace_bytes < m->p.total) rc = TEENY_ERR_SCRATCH;
   // function attributes (dynamic shared memory) are set once per device here, outside any stream capture
   if (rc == 0) rc = gemm_bf16_prepare();
+  if (rc == 0) rc = gemm_rows_prepare();
   if (rc == 0) rc = gemm_bf16_2cta_prepare();
   if (rc == 0) rc = state_scan_prepare();
   if (rc == 0) rc = window_attention_prepare();

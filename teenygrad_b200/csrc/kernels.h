@@ -86,6 +86,37 @@ int linear_w8a16(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float
                  const bf16* bias, bf16* y, int ldy, int M, int N, int K, void* scratch, size_t scratch_bytes,
                  cudaStream_t st, bool swiglu = false, const GemmPush* push = nullptr);
 
+// Decode-shaped linear layer for few rows (M <= 16), its neighbours in the layer folded in (gemm_rows.cu):
+//   in   x [M, K] bf16; or the rows of a residual stream, RMS-normalised on the way in: kRowsNormBf16 as rms_norm_bf16 does it
+//        (bf16 rows, bf16 norm_w), kRowsNormF32 as residual_rms_norm does it (f32 rows, f32 norm_w)
+//   out  y [M, N] (+ bias); glu (kGluSilu, kGluGelu; weight rows interleaved in blocks of 64): y [M, N / 2]; add16 / add32: the
+//        rounded product is added into the residual rows there instead (row stride ldy)
+// w: bf16 [N, K], or with w_scale FP8 E4M3 bytes (scale kind 0 or 1, see above; no NaN bytes).
+constexpr int kRowsMaxM = 16;
+constexpr int kRowsNormNone = 0, kRowsNormBf16 = 1, kRowsNormF32 = 2;
+struct RowsGemm {
+  const void* x;
+  int ldx;
+  int norm;
+  const void* norm_w;
+  float eps;
+  const void* w;
+  int ldw;
+  const float* w_scale;
+  int w_scale_kind;
+  const bf16* bias;
+  int glu;
+  bf16* y;
+  bf16* add16;
+  float* add32;
+  int ldy;
+  int M, N, K;
+  uint32_t w_mul16;  // set by gemm_rows
+};
+bool gemm_rows_takes(int M, int N, int K, int ldw, bool w8, int norm);
+int gemm_rows_prepare();
+int gemm_rows(const RowsGemm& g, cudaStream_t stream);
+
 // Large-M path on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles); same contract as gemm_bf16 without the options.
 // With `qkv` the GEMM is the fused [q | k | v] projection of a prefill (N = (Hq + 2 Hkv) * 128, token t = sequence
 // t / S at position pos0 + t % S) and its epilogue does what qk_norm_rope_kv_bf16 does in a pass of its own: per-head

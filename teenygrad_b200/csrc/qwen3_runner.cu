@@ -487,6 +487,21 @@ bool qkv_fuse_enabled() {
   return on;
 }
 
+// Whether a decode step's projection of T rows runs in the kernel for few rows (gemm_rows.cu), with `norm` in front of it.
+// FP8 weights: per-tensor and per-channel scales.
+bool rows_take(const teeny_qwen3* m, const Weight& w, int T, int N, int K, int norm = kRowsNormNone) {
+  return !m->tp && T <= kRowsMaxM && (!w.q || w.kind <= 1) && gemm_rows_takes(T, N, K, K, w.q != nullptr, norm);
+}
+RowsGemm rows_call(const Weight& w, const void* x, int ldx, int T, int N, int K) {
+  RowsGemm g{};
+  g.x = x; g.ldx = ldx;
+  g.w = w.q ? static_cast<const void*>(w.q) : w.w; g.ldw = K;
+  g.w_scale = w.q ? w.scale : nullptr;
+  g.w_scale_kind = w.kind;
+  g.M = T; g.N = N; g.K = K;
+  return g;
+}
+
 // The shared layer loop.  T tokens arranged [B, S]; pos0 is the position of the first token of every sequence
 // (device value when pos_dev != null).  decode selects the split-KV attention kernel (S == 1).
 int run_layers(teeny_qwen3* m, int B, int S, int pos0, const int* pos_dev, const int* len_dev, bool decode,
@@ -500,24 +515,56 @@ int run_layers(teeny_qwen3* m, int B, int S, int pos0, const int* pos_dev, const
   const float scale = 1.0f / sqrtf(static_cast<float>(D));
   // (Asking the QKV and gate/up weights into L2 while the norm in front of them waits for the other ranks' partial sums
   // was measured under tensor parallelism: 3.29 ms per decode step against 3.25 ms without, 2 ranks.  Not used.)
+  // Decode with few rows: a projection takes its norm along, and the output of a sublayer goes straight into the residual
+  // stream (`held`: it is still in `delta` instead; the last layer's always is, the head's norm adds it).
+  bool held = false;
   for (int l = 0; l < c.num_layers; ++l) {
     const LayerWeights& w = m->layers[l];
     bf16* kc = m->at<bf16>(m->off.kcache) + static_cast<size_t>(l) * m->off.cache_layer_elems;
     bf16* vc = m->at<bf16>(m->off.vcache) + static_cast<size_t>(l) * m->off.cache_layer_elems;
-    const bool qkv8 = wants_x8(m, w.qkv, T), mlp8 = wants_x8(m, w.gate_up, T);
-    if (l == 0)
-      TEENY_TRY(rms_norm_bf16(h, H, y, H, w.input_ln, nullptr, T, H, c.eps, st, qkv8 ? m->at<uint8_t>(m->off.y8) : nullptr, H,
-                              qkv8 ? m->at<float>(m->off.y8_scale) : nullptr));
-    else TEENY_TRY(residual_norm(m, delta, h, H, y, w.input_ln, T, st, qkv8));
+    const bool qkv_rows = decode && rows_take(m, w.qkv, T, qkv_n, H), mlp_rows = decode && rows_take(m, w.gate_up, T, 2 * I, H);
+    const bool qkv8 = !qkv_rows && wants_x8(m, w.qkv, T), mlp8 = !mlp_rows && wants_x8(m, w.gate_up, T);
+    // y[T, N] = norm(h) W^T
+    auto normed = [&](const bf16* norm_w, const Weight& pw, bool rows, bool x8, bf16* out, int N, int glu) -> int {
+      const bool fold = rows && !held && rows_take(m, pw, T, N, H, kRowsNormBf16);
+      if (!fold) {
+        if (held) TEENY_TRY(residual_norm(m, delta, h, H, y, norm_w, T, st, x8));
+        else
+          TEENY_TRY(rms_norm_bf16(h, H, y, H, norm_w, nullptr, T, H, c.eps, st, x8 ? m->at<uint8_t>(m->off.y8) : nullptr, H,
+                                  x8 ? m->at<float>(m->off.y8_scale) : nullptr));
+        held = false;
+      }
+      const int ldo = glu ? N / 2 : N;
+      if (!rows) return project(m, y, H, pw, out, ldo, T, N, H, st, glu != 0, nullptr, nullptr, x8);
+      RowsGemm g = rows_call(pw, fold ? h : y, H, T, N, H);
+      if (fold) { g.norm = kRowsNormBf16; g.norm_w = norm_w; g.eps = c.eps; }
+      g.y = out; g.ldy = ldo;
+      g.glu = glu;
+      return gemm_rows(g, st);
+    };
+    // h += x W^T, or delta = x W^T
+    auto sublayer_out = [&](const bf16* x, const Weight& pw, int K, bool into_h, bool x8) -> int {
+      if (!decode || !rows_take(m, pw, T, H, K)) {
+        held = true;
+        return row_parallel(m, x, K, pw, delta, T, H, K, decode, st, x8);
+      }
+      RowsGemm g = rows_call(pw, x, K, T, H, K);
+      g.ldy = H;
+      if (into_h) g.add16 = h; else g.y = delta;
+      held = !into_h;
+      return gemm_rows(g, st);
+    };
     // Head norms, RoPE and the cache fill: in a large prefill they run in the epilogue of the QKV projection itself (k
     // and v never pass through the projection buffer); in a small one as one pass over the projection; in decode the
     // attention kernel does them for its own (sequence, kv head) on the way in.
     if (!decode && !pos_dev && qkv_fuse_enabled() && gemm_bf16_uses_2cta(T, qkv_n)) {
+      if (held) TEENY_TRY(residual_norm(m, delta, h, H, y, w.input_ln, T, st));
+      else TEENY_TRY(rms_norm_bf16(h, H, y, H, w.input_ln, nullptr, T, H, c.eps, st));
       const QkvEpilogue fuse{w.q_norm, w.k_norm, m->at<bf16>(m->off.cos), m->at<bf16>(m->off.sin), kc, vc,
                              S, Hq, Hkv, c.max_len, pos0, c.eps};
       TEENY_TRY(project(m, y, H, w.qkv, qkv, qkv_n, T, qkv_n, H, st, false, nullptr, &fuse));
     } else {
-      TEENY_TRY(project(m, y, H, w.qkv, qkv, qkv_n, T, qkv_n, H, st, false, nullptr, nullptr, qkv8));
+      TEENY_TRY(normed(w.input_ln, w.qkv, qkv_rows, qkv8, qkv, qkv_n, 0));
       if (!decode)
         TEENY_TRY(qk_norm_rope_kv_bf16(qkv, qkv_n, w.q_norm, w.k_norm, m->at<bf16>(m->off.cos), m->at<bf16>(m->off.sin),
                                        kc, vc, T, S, Hq, Hkv, D, c.max_len, pos0, pos_dev, c.eps, st));
@@ -546,14 +593,14 @@ int run_layers(teeny_qwen3* m, int B, int S, int pos0, const int* pos_dev, const
       a.Sq = S; a.Skv = pos0 + S; a.causal = 1;
       TEENY_TRY(attention_prefill_bf16(qkv, kc, vc, attn, nullptr, a, st));
     }
-    TEENY_TRY(row_parallel(m, attn, Hq * D, w.o, delta, T, H, Hq * D, decode, st));
-    TEENY_TRY(residual_norm(m, delta, h, H, y, w.post_ln, T, st, mlp8));
-    TEENY_TRY(project(m, y, H, w.gate_up, act, I, T, 2 * I, H, st, /*swiglu=*/true, nullptr, nullptr, mlp8));
+    TEENY_TRY(sublayer_out(attn, w.o, Hq * D, true, false));
+    TEENY_TRY(normed(w.post_ln, w.gate_up, mlp_rows, mlp8, act, 2 * I, kGluSilu));
     // (one GPU, FP8 down projection: its input as two-term FP8 costs a small kernel and saves the conversion of 50 M
     // weight bytes next to the tensor core)
-    const bool down8 = down8_enabled() && wants_x8(m, w.down, T) && m->off.a8 != m->off.a8_scale;
+    const bool down8 = down8_enabled() && wants_x8(m, w.down, T) && m->off.a8 != m->off.a8_scale &&
+                       !(decode && rows_take(m, w.down, T, H, I));
     if (down8) TEENY_TRY(split_e4m3(act, I, m->at<uint8_t>(m->off.a8), I, m->at<float>(m->off.a8_scale), T, I, st));
-    TEENY_TRY(row_parallel(m, act, I, w.down, delta, T, H, I, decode, st, down8));
+    TEENY_TRY(sublayer_out(act, w.down, I, l + 1 < c.num_layers, down8));
   }
   return 0;
 }
@@ -751,6 +798,7 @@ int teeny_qwen3_create(const teeny_qwen3_config* cfg, void* workspace, size_t wo
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // function attributes (dynamic shared memory) are set once per device here, outside any stream capture
   int prc = gemm_bf16_prepare();
+  if (prc == 0) prc = gemm_rows_prepare();
   if (prc == 0) prc = gemm_bf16_2cta_prepare();
   if (prc == 0) prc = attention_prefill_prepare();
   if (prc == 0) prc = attention_decode_prepare();
