@@ -3,8 +3,9 @@
 // keeps a ring of TMA tile copies in flight (data in flight costs no registers) and four consumer warps run the
 // arithmetic on warp-level mma.sync tiles fed by ldmatrix (a 128-row tcgen05 tile would be 97 % padding for 4 query
 // heads).  Split over the sequence only when B * Hkv alone cannot fill the GPU; every consumer warp takes 16
-// keys of each 64-key tile with an online softmax, warps are merged through shared memory, per-chunk partials
-// (m, l, O) go to scratch and a second kernel merges chunks.
+// keys of each 64-key tile with an online softmax, warps are merged through shared memory.  A sequence split in up to eight parts
+// is one cluster, whose CTAs hand each other their parts (m, l, O) through distributed shared memory; of more parts they go to
+// scratch, merged by the last CTA to arrive or by a second kernel.
 #include <atomic>
 
 #include "common.cuh"
@@ -43,6 +44,7 @@ struct DecodeArgs {
   // dependency wait.  < 0: nothing is known, read everything after the wait.
   int fresh_rows;
   int stages;          // ring depth of this launch
+  int clustered;       // the CTAs of a sequence are one cluster and merge there (no scratch, no counters)
   unsigned* counters;  // [B * Hkv] arrival counters (zero between calls) for the in-kernel merge, or null
   float scale_log2;
   int* err;
@@ -64,7 +66,13 @@ constexpr int kDecStagesAlone = 6;   // ring depth when the grid has at most one
 constexpr int kDecBox = kDecTile * 64 * 2;       // 8 KB: [64 keys][64 d]
 constexpr int dec_stage_bytes(int hd) { return 2 * (hd / 64) * kDecBox; }  // K and V boxes: 32 KB for head size 128
 constexpr int dec_smem_bytes(int stages, int hd) { return stages * dec_stage_bytes(hd) + 1024 + 128; }
+constexpr int kDecMaxCluster = 8;
 constexpr int kDecThreads = 160;                 // 4 consumer warps + 1 producer warp
+
+__device__ __forceinline__ void st_cluster_f32(const void* local, unsigned rank, float v) {
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}"
+               :: "r"(smem_u32(local)), "r"(rank), "f"(v) : "memory");
+}
 
 template <int G, int HD>
 __global__ void __launch_bounds__(kDecThreads, 2)
@@ -75,6 +83,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   constexpr int kDecStageBytes = dec_stage_bytes(HD), kVTile = (HD / 64) * kDecBox;
   __shared__ float sm_o[4][G][HD];
   __shared__ __align__(16) bf16 sm_q[4][G][HD];  // normed, rotated q heads, one copy per consumer warp (fused front end)
+  // clustered merge: this CTA's slice of the outputs from every CTA of the cluster, and everyone's (m, l)
+  __shared__ float cl_o[G * HD + kDecMaxCluster], cl_ml[kDecMaxCluster][G][2];
   const uint32_t base = (smem_u32(dec_smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = dec_smem_raw + (base - smem_u32(dec_smem_raw));
   const int n_stages = a.stages;
@@ -93,6 +103,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     mbar_fence_init();
   }
   __syncthreads();
+  if (a.clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
   // the live keys are divided evenly (in whole 64-key tiles) over the gridDim.x CTAs of this (batch, kv head)
   int L = 0, span = 0, key_begin = 0, key_end = 0, n_tiles = 0;
   int cb = b, newest = 0;  // row of the cache tensors; cache row of the newest key
@@ -123,14 +134,29 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   };
   int pre = 0;  // tiles requested ahead of the wait (producer thread only)
   int rope_pos = 0;
+  // Fused front end (per-head RMSNorm + RoPE + cache append), one 128-wide head per half-warp, no CTA-wide barrier: every consumer
+  // warp prepares its own copy of the G query heads, and the warp that owns the newest key norms / rotates it, appends it and the
+  // new value to the caches and writes both into the tile in shared memory, which was requested with whatever the caches held there.
+  const bool fused = HD == kHD && a.rope.k_new != nullptr;
+  const int sub = lane & 15, hw = lane >> 4;
+  uint4 wq_raw = {}, wk_raw = {}, craw = {}, sraw = {};  // norm weights and table rows of this lane's eight elements
+  auto rope_constants = [&]() {
+    if (!fused || warp == 4) return;
+    const int tp = rope_pos < a.rope.max_len ? rope_pos : a.rope.max_len - 1;
+    wq_raw = __ldg(reinterpret_cast<const uint4*>(a.rope.q_w + sub * 8));
+    wk_raw = __ldg(reinterpret_cast<const uint4*>(a.rope.k_w + sub * 8));
+    craw = __ldg(reinterpret_cast<const uint4*>(a.rope.cos_t + static_cast<size_t>(tp) * kHD + sub * 8));
+    sraw = __ldg(reinterpret_cast<const uint4*>(a.rope.sin_t + static_cast<size_t>(tp) * kHD + sub * 8));
+  };
   if (a.fresh_rows >= 0) {
     plan();
     if (a.rope.k_new) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
+    rope_constants();
     if (threadIdx.x == 128) {
       // first ring of tiles that hold none of the rows the previous kernel is still writing
-      // (the fresh rows end at the newest key; in a ring older rows may follow it)
+      // (the fresh rows end at the newest key; in a ring older rows may follow it; the fused front end has none)
       while (pre < n_tiles && pre < n_stages &&
-             (key_begin + (pre + 1) * kDecTile <= newest + 1 - a.fresh_rows || key_begin + pre * kDecTile > newest)) {
+             (fused || key_begin + (pre + 1) * kDecTile <= newest + 1 - a.fresh_rows || key_begin + pre * kDecTile > newest)) {
         load_tile(pre, pre);
         ++pre;
       }
@@ -140,43 +166,15 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   if (a.fresh_rows < 0) {
     plan();
     if (a.rope.k_new) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
+    rope_constants();
   }
   const int g = lane >> 2, c = lane & 3;
   float acc[HD / 8][4];
   float m = -INFINITY, l = 0.0f;
-  if (n_tiles == 0) return;  // chunk lies beyond the live length (uniform for the CTA)
-
-  // Fused front end (per-head RMSNorm + RoPE + cache append), one 128-wide head per half-warp.  No CTA-wide barrier:
-  // the producer warp norms / rotates the new key, appends it and the new value to the caches and goes on streaming;
-  // every consumer warp prepares its own copy of the G query heads.
-  const bool fused = HD == kHD && a.rope.k_new != nullptr;
-  const int sub = lane & 15, hw = lane >> 4;
-  auto rope_head = [&](const bf16* src, const bf16* w, uint4& raw) {
-    raw = *reinterpret_cast<const uint4*>(src + sub * 8);
-    const uint4 wraw = __ldg(reinterpret_cast<const uint4*>(w + sub * 8));
-    const int tp = rope_pos < a.rope.max_len ? rope_pos : a.rope.max_len - 1;
-    const uint4 craw = __ldg(reinterpret_cast<const uint4*>(a.rope.cos_t + static_cast<size_t>(tp) * kHD + sub * 8));
-    const uint4 sraw = __ldg(reinterpret_cast<const uint4*>(a.rope.sin_t + static_cast<size_t>(tp) * kHD + sub * 8));
-    return head_norm_rope(raw, wraw, craw, sraw, sub, a.rope.eps);
-  };
+  if (n_tiles == 0 && !a.clustered) return;  // chunk lies beyond the live length (uniform for the CTA)
 
   if (warp == 4) {
     // ---------------- producer ----------------
-    if (fused) {
-      // half-warp 0: key head (normed, rotated); half-warp 1: value head (copied)
-      uint4 raw;
-      const uint4 outv = rope_head((hw == 0 ? a.rope.k_new : a.rope.v_new) + b * a.rope.new_sb + hk * kHD, a.rope.k_w, raw);
-      if (rope_pos >= key_begin && rope_pos < key_end && rope_pos < a.rope.max_len) {
-        if (hw == 0)
-          *reinterpret_cast<uint4*>(a.rope.k_cache + b * a.kc_sb + hk * a.kc_sh + rope_pos * a.kc_ss + sub * 8) = outv;
-        else
-          *reinterpret_cast<uint4*>(a.rope.v_cache + b * a.vc_sb + hk * a.vc_sh + rope_pos * a.vc_ss + sub * 8) = raw;
-      }
-      // the appended rows are read back by this warp's own TMA loads (async proxy): order them behind the stores
-      __threadfence();
-      asm volatile("fence.proxy.async;" ::: "memory");
-      __syncwarp();
-    }
     if (lane == 0) {
       int st = pre == n_stages ? 0 : pre;
       uint32_t ph = pre == n_stages ? 1 : 0;
@@ -192,13 +190,25 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     for (int i = 0; i < HD / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
     // Q fragments: head hk * G + g; a0 = d 16 ks + 2c.., a2 = d 16 ks + 8 + 2c..; rows >= G are zero
     uint32_t qa[HD / 16][2];
+    // the newest key and value, held by the half-warps of the one warp that owns them (fused front end)
+    const int new_rel = rope_pos - key_begin;
+    const bool has_new = fused && rope_pos < a.rope.max_len && rope_pos >= key_begin && rope_pos < key_end && ((new_rel >> 4) & 3) == warp;
+    uint4 new_row = make_uint4(0u, 0u, 0u, 0u);
     {
+      if (has_new) {
+        const uint4 raw = *reinterpret_cast<const uint4*>((hw == 0 ? a.rope.k_new : a.rope.v_new) + b * a.rope.new_sb + hk * kHD + sub * 8);
+        const uint4 turned = head_norm_rope(raw, wk_raw, craw, sraw, sub, a.rope.eps);
+        new_row = hw == 0 ? turned : raw;
+        bf16* dst = hw == 0 ? a.rope.k_cache + b * a.kc_sb + hk * a.kc_sh + rope_pos * a.kc_ss
+                            : a.rope.v_cache + b * a.vc_sb + hk * a.vc_sh + rope_pos * a.vc_ss;
+        *reinterpret_cast<uint4*>(dst + sub * 8) = new_row;
+      }
       if (fused) {
 #pragma unroll
         for (int h0 = 0; h0 < G; h0 += 2) {  // two heads per pass (a lone last head is done twice)
           const int hsel = h0 + hw < G ? h0 + hw : G - 1;
-          uint4 raw;
-          const uint4 outv = rope_head(a.q + b * a.q_sb + (hk * G + hsel) * a.q_sh, a.rope.q_w, raw);
+          const uint4 raw = *reinterpret_cast<const uint4*>(a.q + b * a.q_sb + (hk * G + hsel) * a.q_sh + sub * 8);
+          const uint4 outv = head_norm_rope(raw, wq_raw, craw, sraw, sub, a.rope.eps);
           *reinterpret_cast<uint4*>(&sm_q[warp][hsel][sub * 8]) = outv;
         }
         __syncwarp();
@@ -221,6 +231,12 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       const uint32_t kt = base + st * kDecStageBytes, vt = kt + kVTile;
       const int kb = key_begin + t * kDecTile + 16 * warp;  // first key of this warp's slice
       if (kb < key_end) {
+        if (has_new && (new_rel >> 6) == t) {
+          const int rr = new_rel & 63;  // row of the tile; 128-byte swizzle as TMA wrote it
+          *reinterpret_cast<uint4*>(gen + st * kDecStageBytes + (hw == 0 ? 0 : kVTile) + (sub >> 3) * kDecBox + rr * 128 +
+                                    (((sub & 7) ^ (rr & 7)) << 4)) = new_row;
+          __syncwarp();
+        }
         if (kb + 16 > key_end) {
           // rows past the live length hold whatever the cache had (possibly NaN patterns): their probabilities are
           // zero, but 0 * NaN is NaN inside the MMA, so clear those V rows first
@@ -323,6 +339,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     a.o[b * a.o_sb + (hk * G + gg) * a.o_sh + d] = __float2bfloat16_rn(oo);
   };
   const size_t slot = (static_cast<size_t>(b) * a.Hkv + hk) * a.max_chunks + chunk;
+  const int n_cta = gridDim.x, slice = (G * HD + n_cta - 1) / n_cta;  // clustered: CTA i finishes outputs i * slice ..
+  if (a.clustered) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster is running
   for (int idx = threadIdx.x; idx < G * HD; idx += kDecThreads) {
     const int gg = idx / HD, d = idx - gg * HD;
     float mm = -INFINITY;
@@ -336,6 +354,16 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       ll += sm_ml[w][gg][1] * sc;
       oo += sm_o[w][gg][d] * sc;
     }
+    if (a.clustered) {
+      const unsigned owner = idx / slice;
+      st_cluster_f32(&cl_o[chunk * slice + idx - owner * slice], owner, oo);
+      if (d == 0)
+        for (int to = 0; to < n_cta; ++to) {
+          st_cluster_f32(&cl_ml[chunk][gg][0], to, mm);
+          st_cluster_f32(&cl_ml[chunk][gg][1], to, ll);
+        }
+      continue;
+    }
     if (gridDim.x == 1) {  // whole sequence in this CTA: finish here, no partials
       finish(gg, d, mm, ll, oo);
       continue;
@@ -346,7 +374,24 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       a.part_ml[(slot * G + gg) * 2 + 1] = ll;
     }
   }
-  if (gridDim.x > 1 && a.counters) {
+  __syncwarp();
+  if (a.clustered) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < slice; i += kDecThreads) {
+      const int idx = chunk * slice + i;
+      if (idx >= G * HD) break;
+      const int gg = idx / HD, d = idx - gg * HD;
+      float mm = -INFINITY, ll = 0.0f, oo = 0.0f;
+      for (int ch = 0; ch < n_cta; ++ch) mm = fmaxf(mm, cl_ml[ch][gg][0]);  // CTAs without keys hold -inf
+      for (int ch = 0; ch < n_cta; ++ch) {
+        const float cm = cl_ml[ch][gg][0];
+        const float sc = cm == -INFINITY ? 0.0f : ex2(cm - mm);
+        ll = fmaf(cl_ml[ch][gg][1], sc, ll);
+        oo = fmaf(cl_o[ch * slice + i], sc, oo);
+      }
+      finish(gg, d, mm, ll, oo);
+    }
+  } else if (gridDim.x > 1 && a.counters) {
     // The last CTA of this (sequence, kv head) to have stored its partial merges them all: no second kernel.
     __shared__ unsigned sm_last;
     __threadfence();
@@ -522,12 +567,30 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
     if (n_split > max_chunks) n_split = max_chunks;
     if (n_split < 1) n_split = 1;
   }
-  a.counters = n_split > 1 ? counters : nullptr;
+  // Parts of two tiles are worth a CTA of their own when the merge stays inside a cluster: 0.6 us instead of 3 through scratch, fence
+  // and counter.  Decode step of a 28-layer model, batch 1, 8 kv heads, 576 rows (nine tiles): 675 us with one CTA for each head,
+  // 601, 588 and 562 with parts of five, three and two tiles.  Three tiles in all are faster in one CTA (4k model, batch 8: 576 us a
+  // step against 581 with two parts).  The ring is no deeper than a part's tiles, which leaves room for the next kernel's CTAs.
+  const int tiles = (s.Skv + kDecTile - 1) / kDecTile;
+  if (a.stages == kDecStagesAlone && n_split <= kDecMaxCluster) {
+    int n = sms / bh;
+    n = n < kDecMaxCluster ? n : kDecMaxCluster;
+    const int most = tiles < 4 ? 1 : (tiles + 1) / 2;
+    n = n < most ? n : most;
+    if (n > 1) {
+      n_split = n;
+      a.clustered = 1;
+      const int part = (tiles + n - 1) / n;
+      if (part < a.stages) a.stages = part;
+    }
+  }
+  a.counters = n_split > 1 && !a.clustered ? counters : nullptr;
   const int smem = dec_smem_bytes(a.stages, HD);
   dim3 grid(n_split, s.Hkv, s.B);
+  const unsigned cl = a.clustered ? n_split : 1;
 #define TEENY_DEC(GG)                                                                                                     \
-  if (HD == 64) launch_kernel(attention_decode_kernel<GG, 64>, grid, dim3(kDecThreads), smem, stream, 1, mk, mv, a);      \
-  else launch_kernel(attention_decode_kernel<GG, 128>, grid, dim3(kDecThreads), smem, stream, 1, mk, mv, a)
+  if (HD == 64) launch_kernel(attention_decode_kernel<GG, 64>, grid, dim3(kDecThreads), smem, stream, cl, mk, mv, a);      \
+  else launch_kernel(attention_decode_kernel<GG, 128>, grid, dim3(kDecThreads), smem, stream, cl, mk, mv, a)
   switch (G) {
     case 1: TEENY_DEC(1); break;
     case 2: TEENY_DEC(2); break;
@@ -537,7 +600,7 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
 #undef TEENY_DEC
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (n_split == 1 || a.counters) return 0;
+  if (n_split == 1 || a.counters || a.clustered) return 0;
   launch_kernel(attention_decode_combine_kernel, dim3(s.Hq, s.B), dim3(kHD), 0, stream, 1, a.part_o, a.part_ml, o,
                 s.o_sb, s.o_sh, s.Hkv, G, max_chunks, n_split, kv_len, kv_len_dev);
   return static_cast<int>(cudaGetLastError());
