@@ -187,11 +187,12 @@ int teeny_device_error(int clear) {
 // ---- GEMM ----
 int matmul_forward_entry_point_f32(const float* a, const float* b, float* c, int M, int N, int K, void* scratch,
                                    size_t scratch_bytes, teeny_stream_t stream) {
-  // with scratch for the split operands: the tensor-core path (bf16 x 3, f32 accuracy); else f32 FMAs on the CUDA cores
+  // with scratch for the split operands, and where that is faster: two bf16 terms per operand, 1e-5; else at the accuracy of f32 multiply-adds
   if (a && b && c && scratch && M > 0 && N > 0 && K > 0 && !(K & 7) && !(N & 7) &&
       !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
          reinterpret_cast<uintptr_t>(scratch)) & 15) &&
-      scratch_bytes >= gemm_f32_split_scratch_bytes(M, N, K))
+      scratch_bytes >= gemm_f32_split_scratch_bytes(M, N, K) &&
+      gemm_f32_split_clocks(M, N, K) < gemm_f32_clocks(a, K, 1, b, N, 1, M, N, K))
     return gemm_f32_split(a, b, c, M, N, K, scratch, scratch_bytes, S(stream));
   return gemm_f32(a, K, 1, b, N, 1, nullptr, c, N, 1, M, N, K, S(stream));
 }

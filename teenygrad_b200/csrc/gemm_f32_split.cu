@@ -59,6 +59,13 @@ size_t gemm_f32_split_scratch_bytes(int M, int N, int K) {
   return align256(static_cast<size_t>(M) * 3 * K * 2) + align256(static_cast<size_t>(3) * K * N * 2);
 }
 
+// Clocks: two passes over the operands and three launches (14000), and 590 for each 64 of the threefold K of a 128 x 128 tile.
+// 512^3: 15.2 us (9.8 with three terms and no scratch); 1000 x 2048 x 2048: 43 (60); 4096^3: 430 (757).
+double gemm_f32_split_clocks(int M, int N, int K) {
+  const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + 127) / 128), sms = sm_count();
+  return 14000.0 + static_cast<double>((tiles + sms - 1) / sms) * ((3LL * K + 63) / 64) * 590.0;
+}
+
 int gemm_f32_split(const float* a, const float* b, float* c, int M, int N, int K, void* scratch, size_t scratch_bytes,
                    cudaStream_t stream) {
   if (!a || !b || !c || !scratch || M <= 0 || N <= 0 || K <= 0) return TEENY_ERR_BAD_ARG;

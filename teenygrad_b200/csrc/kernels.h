@@ -142,9 +142,17 @@ bool gemm_bf16_uses_2cta(int M, int N);
 // GEMM over the concatenated K (A' = [hi | mid | hi], B' = [hi ; hi ; mid]).  scratch holds A' and B':
 // gemm_f32_split_scratch_bytes(M, N, K).  Needs K and N multiples of 8 and 16-byte aligned pointers.
 size_t gemm_f32_split_scratch_bytes(int M, int N, int K);
+double gemm_f32_split_clocks(int M, int N, int K);  // estimated
 int gemm_f32_split(const float* a, const float* b, float* c, int M, int N, int K, void* scratch, size_t scratch_bytes,
                    cudaStream_t stream);
-// f32 GEMM with true f32 accuracy.  b_is_nk: B given as [N, K] (linear layout) instead of [K, N].
+// The same accuracy as f32 multiply-adds from the tensor cores (gemm_f32_tc.cu): three bf16 terms per operand.  sam = row stride of A
+// (k contiguous); B with either index contiguous.
+bool gemm_f32_tc_takes(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K);
+double gemm_f32_tc_clocks(long long sbk, int M, int N, int K);  // estimated
+int gemm_f32_tc(const float* a, long long sam, const float* b, long long sbk, long long sbn, const float* bias, float* c, long long scm,
+                long long scn, int M, int N, int K, cudaStream_t stream);
+// f32 GEMM with true f32 accuracy, on the tensor cores or the CUDA cores, whichever is estimated to end first (gemm_f32_clocks).  b_is_nk: B given as [N, K] (linear layout) instead of [K, N].
+double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K);
 int gemm_f32(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn,
              const float* bias, float* c, long long scm, long long scn, int M, int N, int K, cudaStream_t stream);
 // bf16 GEMM on CUDA cores for shapes the TMA path cannot take (unaligned strides / pointers).

@@ -1,0 +1,65 @@
+"""GPU: f32 products on the tensor cores (three bf16 terms per operand, sums of 64 k) against float64: tile widths, K splits, ragged edges
+and numbers that the split does not hold."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from teenygrad_b200 import ops as o
+    return o
+
+
+def bound(x, w, K):
+    """Per element: a sum of 64 k is cut off at most 24 times by 2^-23 of the products' sizes, the sums of K / 64 such and of up to eight parts
+    are rounded, and the terms left out are below 3 * 2^-24."""
+    return (48 + K // 64 + 12) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 1000, 1000), (4, 4096, 4096), (64, 4096, 2052), (300, 700, 2000), (2000, 100, 4000), (512, 512, 512), (129, 4100, 68),
+                                   (1000, 4096, 1024), (1100, 2300, 36), (4000, 64, 516)])
+def test_shapes(ops, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    wide = [torch.full((r, K + 4), float("nan"), device="cuda") for r in (M, N)]  # what lies between the rows is not read
+    x, w = wide[0][:, :K], wide[1][:, :K]
+    x.copy_(torch.randn(M, K, generator=g, device="cuda"))
+    w.copy_(torch.randn(N, K, generator=g, device="cuda"))
+    bias = torch.randn(N, generator=g, device="cuda")
+    e, b = x.double() @ w.double().T, bound(x, w, K)
+    out = torch.empty(M, N, device="cuda")
+    ops.linear_forward(x, w, bias, out=out)
+    assert bool(((out.double() - e - bias.double()).abs() <= b + 2.0 ** -23 * (e.abs() + bias.abs())).all())
+    kn = w.T.contiguous()
+    assert bool(((ops.matmul_forward(x.contiguous(), kn).double() - e).abs() <= b).all())
+    rel = float((out.double() - e - bias.double()).norm() / e.norm())
+    assert rel < 3e-7  # f32 multiply-adds in one chain: 2.4e-7 at K = 1000, 1.2e-6 at K = 4096
+    assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 1500, 320), (40, 1000, 1600)])
+@pytest.mark.parametrize("kn", [False, True])
+def test_numbers_at_the_limits(ops, M, N, K, kn):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    x[3, 7] = float("inf")
+    x[5, 9] = float("nan")
+    x[7, 1], w[:, 1] = 3.4028e38, w[:, 1].clamp(-0.9, 0.9)  # rounds to infinity as bf16
+    x[9] *= 1e-36
+    x[11] = 0.0
+    w[4, 7] = 0.0
+    w[6, 3] = -float("inf")
+    w[8] = 1e-3
+    w[12] *= 1e20
+    y = ops.matmul_forward(x, w.T.contiguous()) if kn else ops.linear_forward(x, w, None)
+    e = x.double() @ w.double().T
+    f = e.float()
+    assert torch.equal(torch.isnan(y), torch.isnan(f)) and torch.equal(torch.isinf(y), torch.isinf(f))
+    ok = torch.isfinite(f)
+    # products below the smallest number that f32 holds with all its bits are off by up to 2^-149 each
+    b = (48 + K // 64 + 12) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
+    assert bool(((y.double() - e).abs() <= b)[ok].all())
+    assert ops.device_error() == 0
