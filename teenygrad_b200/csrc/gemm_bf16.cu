@@ -467,7 +467,7 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t
   return v;
 }
 
-// grid (S, tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile.
+// grid (S, tiles, token tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile, blockIdx.z = BN tokens.
 template <int BN, bool W8 = false, bool F8 = false>
 __global__ void __launch_bounds__((SkinnyCfg<BN, W8, F8>::kThreads), 2)
 gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -494,6 +494,8 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   int* err = args.err;
   const uint32_t S = cluster_size(), rank = cluster_rank();
   const int tile = blockIdx.y;
+  const int m0 = blockIdx.z * BN, rows = args.M - m0;  // this CTA's tokens
+  bf16* const y = args.y + static_cast<size_t>(m0) * args.ldy;
   const int kb0 = static_cast<int>(rank) * args.kb_per_split;
   const int kb1 = min(args.k_blocks, kb0 + args.kb_per_split);
   // W8: what the accumulator of weight row n is multiplied by on the way out (per-group scales are already in the
@@ -545,9 +547,9 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
       pdl_wait();
       auto load_x = [&](uint32_t sq, uint32_t bar, int kb) {  // the activation tile(s) of one stage: 64 k each
-        tma_load_2d(sq, &tmap_x, bar, kb * Cfg::kKB, 0);
-        if constexpr (F8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB, args.x_lo_row);  // the lo terms
-        else if constexpr (W8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB + kBK, 0);
+        tma_load_2d(sq, &tmap_x, bar, kb * Cfg::kKB, m0);
+        if constexpr (F8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB, args.x_lo_row + m0);  // the lo terms
+        else if constexpr (W8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB + kBK, m0);
       };
       for (int i = 0; i < pre; ++i) load_x(smem_base + i * Cfg::kStageBytes + Cfg::kStageP, full_bar(i), kb0 + i);
       int stage = pre == Cfg::kStages ? 0 : pre;
@@ -704,7 +706,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
           for (int e = 0; e < kChunk; ++e) {
             if constexpr (F8) {
-              const float xs = (c0 + e < args.M) ? __ldg(args.x_scale + c0 + e) : 0.0f;
+              const float xs = (c0 + e < rows) ? __ldg(args.x_scale + m0 + c0 + e) : 0.0f;
               r[e] = __float_as_uint(fmaf(__uint_as_float(r1[e]), 0.0625f, __uint_as_float(r[e])) * xs);
             } else {
               r[e] = __float_as_uint(__uint_as_float(r[e]) + __uint_as_float(r1[e]));
@@ -718,7 +720,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
             for (int e = 0; e < kChunk; ++e) {
               const int c = c0 + e;
-              if (c < args.M) {
+              if (c < rows) {
                 const float v = W8 ? fmaf(__uint_as_float(r[e]), wsc, bias) : __uint_as_float(r[e]) + bias;
                 if (args.push_recv) {
                   const size_t off = static_cast<size_t>(c) * args.N + n;
@@ -727,7 +729,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
                   for (int p = p0; p < p1; ++p)  // NVLink stores, one 64-bit word per {value, stamp}
                     st_stamped(args.push_recv[p] + off, __float_as_uint(v), stamp);
                 } else {
-                  args.y[static_cast<size_t>(c) * args.ldy + n] = __float2bfloat16_rn(v);
+                  y[static_cast<size_t>(c) * args.ldy + n] = __float2bfloat16_rn(v);
                 }
               }
             }
@@ -759,7 +761,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int epi = (warp - 2) * 32 + lane;
     if (args.swiglu) {
       // the tile holds 64 gate rows then the 64 up rows of the same channels: a unit = 4 channels of one column
-      const bool vec_ok = (args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(args.y) & 7) == 0);
+      const bool vec_ok = (args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(y) & 7) == 0);
       for (int u = epi; u < ncols * 16; u += kEpilogueThreads) {
         const int c = c_begin + (u >> 4), j = u & 15;
         const uint32_t ga = part_base + static_cast<uint32_t>((c * kBM + 4 * j) * 4);
@@ -781,10 +783,10 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           gs.x *= row_scale(wr); gs.y *= row_scale(wr + 1); gs.z *= row_scale(wr + 2); gs.w *= row_scale(wr + 3);
           us.x *= row_scale(wr + 64); us.y *= row_scale(wr + 65); us.z *= row_scale(wr + 66); us.w *= row_scale(wr + 67);
         }
-        if (c < args.M) {
+        if (c < rows) {
           const float o[4] = {glu_f(args.swiglu, gs.x, us.x), glu_f(args.swiglu, gs.y, us.y), glu_f(args.swiglu, gs.z, us.z),
                               glu_f(args.swiglu, gs.w, us.w)};
-          bf16* dst = args.y + static_cast<size_t>(c) * args.ldy + n_out;
+          bf16* dst = y + static_cast<size_t>(c) * args.ldy + n_out;
           if (vec_ok && n_out + 3 < args.N / 2) {
             *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
           } else {
@@ -795,7 +797,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
     } else {
       const bool vec_ok = args.push_recv ? (args.N % 4 == 0)
-                                         : ((args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(args.y) & 7) == 0));
+                                         : ((args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(y) & 7) == 0));
       const unsigned stamp = args.push_recv ? __ldcg(args.push_epoch) * 1024u + args.push_round + 1u : 0u;
       for (int u = epi; u < ncols * 32; u += kEpilogueThreads) {
         const int c = c_begin + (u >> 5), j = u & 31;
@@ -808,7 +810,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
         for (int q = 1; q < 8; ++q) { acc.x += v[q].x; acc.y += v[q].y; acc.z += v[q].z; acc.w += v[q].w; }
         const int n = tile * kBM + 4 * j;
-        if (c < args.M && n < args.N) {
+        if (c < rows && n < args.N) {
           float o[4] = {acc.x, acc.y, acc.z, acc.w};
           if constexpr (W8) {
 #pragma unroll
@@ -834,7 +836,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
               }
             }
           } else {
-            bf16* dst = args.y + static_cast<size_t>(c) * args.ldy + n;
+            bf16* dst = y + static_cast<size_t>(c) * args.ldy + n;
             if (vec_ok && n + 3 < args.N) {
               *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
             } else {
@@ -902,10 +904,10 @@ int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, const GemmArgs&
 
 template <int BN, bool W8 = false, bool F8 = false>
 int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int split, int tiles,
-                  cudaStream_t st) {
+                  cudaStream_t st, int token_tiles = 1) {
   const int rc = prepare_skinny<BN, W8, F8>();
   if (rc) return rc;
-  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8>, dim3(split, tiles, 1),
+  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8>, dim3(split, tiles, token_tiles),
                        dim3(SkinnyCfg<BN, W8, F8>::kThreads, 1, 1), SkinnyCfg<BN, W8, F8>::kSmemBytes, st,
                        static_cast<unsigned>(split), tw, tx, a);
 }
@@ -927,6 +929,34 @@ int skinny_split(int tiles, int k_blocks, int sms) {
 // Largest token count that takes the swapped (weights on the 128-row MMA side) assignment.
 constexpr int kSwapMaxM = 128;
 int swap_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
+
+// More than kSwapMaxM tokens: the kernel that is estimated to end first.  Microseconds: a start, and the rounds of tiles over the SMs
+// times the 64-k blocks of a tile times what a block takes.  Fitted to calls with 129 to 4500 tokens (M x N x K; narrow 128 x 128
+// tiles / wide 128 x 256 / CTA pairs with 256 x 256 / K of 128 x 128 tiles over clusters):
+//   800 x 4096 x 4096 40.0 / 30.9 / 28.6 / 41.6     300 x 12288 x 1024 16.3 / 16.6 / 22.1 / 24.6     512 x 1024 x 3072 17.4 / 21.0 / 21.4 / 11.7
+//   200 x 4096 x 12288 54.5 / 75.3 / 62.7 / 32.5    4500 x 1024 x 3072 33.3 / 24.5 / 24.3 / -        200 x 520 x 8192 39.3 / 46.4 / 46.8 / 12.5
+// (By tile counts alone, wide tiles only with one for every SM and no K split, these took 40.7, 22.0, 17.4, 54.4, 33.1 and 41.7.)
+enum { kLargeNone, kLargeNarrow, kLargeWide, kLargePair, kLargeSplit };
+struct LargeChoice { int kind, split; };
+LargeChoice choose_large(int M, int N, int k_blocks, int sms) {
+  auto rounds = [](long long tiles, long long slots) { return static_cast<double>((tiles + slots - 1) / slots); };
+  const long long m128 = ceil_div(M, 128), n128 = ceil_div(N, 128), n256 = ceil_div(N, 256);
+  LargeChoice best{kLargeNarrow, 0};
+  double least = 5.0 + rounds(m128 * n128, sms) * k_blocks * 0.28;
+  const double wide = 6.5 + rounds(m128 * n256, sms) * k_blocks * 0.385;
+  if (N > 128 && wide < least) { best.kind = kLargeWide; least = wide; }
+  const double pair = 7.5 + rounds(static_cast<long long>(ceil_div(M, 256)) * n256, sms / 2) * k_blocks * 0.345;
+  if (pair < least) { best.kind = kLargePair; least = pair; }
+  for (int split = 2; split <= 8; ++split) {
+    const int per = ceil_div(k_blocks, split);
+    // all of them resident, two on an SM; clusters do not find place on every SM (300 x 4096 x 4096 in 288 CTAs: 30.5 us, in 192: 22.7)
+    const long long ctas = m128 * n128 * split;
+    if (ctas * 100 > 2LL * sms * 87 || per < 4 || per * (split - 1) >= k_blocks || n128 > 65535) continue;
+    const double t = ctas <= sms ? 6.5 + per * 0.45 : 9.0 + per * 0.47;
+    if (t < least) { best = LargeChoice{kLargeSplit, split}; least = t; }
+  }
+  return best;
+}
 
 }  // namespace
 
@@ -1007,14 +1037,17 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
   const int sms = sm_count();
 
   CUtensorMap tmx, tmw;
-  const bool swap = (!w_is_kn) && (M <= kSwapMaxM);
+  const LargeChoice large = (w_is_kn || M <= kSwapMaxM) ? LargeChoice{} : choose_large(M, N, a.k_blocks, sms);
+  // Enough 256 x 256 tiles for the SM pairs: the CTA-pair kernel.
+  if (large.kind == kLargePair) return gemm_bf16_2cta(x, ldx, w, ldw, bias, y, ldy, M, N, K, stream, swiglu);
+  const bool swap = !w_is_kn && (M <= kSwapMaxM || large.kind == kLargeSplit);
   int bn;
   if (swap) {
     bn = swap_bn(M);
   } else if (w_is_kn) {
     bn = (N <= 64) ? 64 : 128;
   } else {
-    bn = (N <= 128 || (static_cast<long long>(ceil_div(M, kBM)) * ceil_div(N, 256) < sms)) ? 128 : 256;
+    bn = large.kind == kLargeWide ? 256 : 128;
   }
 
   // activations X: K-major rows; box = 64 k x (128 rows normally, bn rows when swapped)
@@ -1041,11 +1074,12 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
 
   if (swap) {
     const int tiles = ceil_div(N, kBM);
-    if ((tiles < 4 * sms || swiglu || push) && tiles <= 65535) {
+    if ((tiles < 4 * sms || swiglu || push || large.split) && tiles <= 65535) {
       // Few weight tiles: cluster split-K.  Measured on B200 (batch 32, K = 4096 / 12288): the kernel is fastest
       // when all its CTAs are resident at once (two per SM) and share HBM evenly -- about 0.85 of the slots -- and a
       // wider cluster than that only adds barrier and reduction cost; with at least as many tiles as SMs no split.
-      const int split = skinny_split(tiles, a.k_blocks, sms);
+      const int split = large.split ? large.split : skinny_split(tiles, a.k_blocks, sms);
+      const int token_tiles = ceil_div(M, bn);
       a.kb_per_split = ceil_div(a.k_blocks, split);
       {  // what the CTAs ask into L2 ahead of time must stay well inside it (126 MB): at most 48 MB over the grid
         const long long per_cta = (48ll << 20) / (static_cast<long long>(kBM * kBK * 2) * split * tiles);
@@ -1055,7 +1089,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
         case 16: return launch_skinny<16>(tmw, tmx, a, split, tiles, stream);
         case 32: return launch_skinny<32>(tmw, tmx, a, split, tiles, stream);
         case 64: return launch_skinny<64>(tmw, tmx, a, split, tiles, stream);
-        default: return launch_skinny<128>(tmw, tmx, a, split, tiles, stream);
+        default: return launch_skinny<128>(tmw, tmx, a, split, tiles, stream, token_tiles);
       }
     }
     a.tiles_p = tiles;
@@ -1069,9 +1103,6 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
     }
   }
 
-  // Enough 256 x 256 tiles to occupy every SM pair: the CTA-pair kernel (about a fifth faster at these sizes).
-  if (!w_is_kn && gemm_bf16_uses_2cta(M, N))
-    return gemm_bf16_2cta(x, ldx, w, ldw, bias, y, ldy, M, N, K, stream, swiglu);
   a.tiles_p = ceil_div(M, kBM);
   a.tiles_q = ceil_div(N, bn);
   const int work = a.tiles_p * a.tiles_q;
