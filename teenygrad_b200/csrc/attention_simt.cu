@@ -7,8 +7,9 @@
 // and the multiply-adds are packed pairs of keys (or of output dimensions), which halves their issue slots.  A row's eight
 // threads sit side by side in one warp: the probabilities pass through shared memory behind a __syncwarp, the row maximum takes
 // three shuffles, the row sum is only added up at the end.  Two or more CTAs per SM hide each other's tile loads, which hit L2.
-// Measured on B200, f32, 32 heads x 1000 x 1000: 274 us at D = 64 (30 TFLOP/s of the pipe's 74), 546 us at D = 128; a warp per query row
-// with a chain of shuffles and exponentials per key took 6250 us at D = 64.
+// Measured on B200, f32, 32 heads x 1000 x 1000: 279 us at D = 64 (29 TFLOP/s of the pipe's 74), 562 us at D = 128 (error against 64 bits
+// 6.0e-7 either way); a warp per query row
+// with a chain of shuffles and exponentials per key took 6250 us at D = 64 (7.4e-7).
 #include <atomic>
 
 #include "common.cuh"
@@ -155,20 +156,34 @@ attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int j = 0; j < 4; ++j) sc[r][j] = pack2(0.0f, 0.0f);
-#pragma unroll 4
-    for (int d = 0; d < Cfg::kD; ++d) {
-      float a[R];
-      read_rows<R>(a, qt + d * Cfg::kRows + ty * R);
-      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(kt + d * kTile + 4 * tx);
-      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(kt + d * kTile + 32 + 4 * tx);
+    // 32 dimensions at a time: a shorter chain of roundings than the whole head
+#pragma unroll 1
+    for (int d0 = 0; d0 < Cfg::kD; d0 += 32) {
+      f32x2 part[R][4];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const f32x2 aa = pack2(a[r], a[r]);
-        sc[r][0] = fma2(aa, b0.x, sc[r][0]);
-        sc[r][1] = fma2(aa, b0.y, sc[r][1]);
-        sc[r][2] = fma2(aa, b1.x, sc[r][2]);
-        sc[r][3] = fma2(aa, b1.y, sc[r][3]);
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[r][j] = pack2(0.0f, 0.0f);
+#pragma unroll 4
+      for (int d = d0; d < d0 + 32; ++d) {
+        float a[R];
+        read_rows<R>(a, qt + d * Cfg::kRows + ty * R);
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(kt + d * kTile + 4 * tx);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(kt + d * kTile + 32 + 4 * tx);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const f32x2 aa = pack2(a[r], a[r]);
+          part[r][0] = fma2(aa, b0.x, part[r][0]);
+          part[r][1] = fma2(aa, b0.y, part[r][1]);
+          part[r][2] = fma2(aa, b1.x, part[r][2]);
+          part[r][3] = fma2(aa, b1.y, part[r][3]);
+        }
       }
+      const f32x2 one = pack2(1.0f, 1.0f);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sc[r][j] = fma2(part[r][j], one, sc[r][j]);
     }
 
     const bool edge = k0 + kTile > s.Skv || (s.causal && k0 + kTile - 1 > row0 + shift);

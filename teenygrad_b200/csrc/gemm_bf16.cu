@@ -943,7 +943,7 @@ LargeChoice choose_large(int M, int N, int k_blocks, int sms) {
   const long long m128 = ceil_div(M, 128), n128 = ceil_div(N, 128), n256 = ceil_div(N, 256);
   LargeChoice best{kLargeNarrow, 0};
   double least = 5.0 + rounds(m128 * n128, sms) * k_blocks * 0.28;
-  const double wide = 6.5 + rounds(m128 * n256, sms) * k_blocks * 0.385;
+  const double wide = 8.0 + rounds(m128 * n256, sms) * k_blocks * 0.385;
   if (N > 128 && wide < least) { best.kind = kLargeWide; least = wide; }
   const double pair = 7.5 + rounds(static_cast<long long>(ceil_div(M, 256)) * n256, sms / 2) * k_blocks * 0.345;
   if (pair < least) { best.kind = kLargePair; least = pair; }
