@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
 }
 
 template <int BN, bool KN>
-int launch_tc(F32Args g, int grid, cudaStream_t st) {
+int prepare_tc() {
   static std::atomic<unsigned long long> done{0};  // one bit per device; threads may race to set it
   int dev = 0;
   cudaGetDevice(&dev);
@@ -363,6 +363,13 @@ int launch_tc(F32Args g, int grid, cudaStream_t st) {
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
   }
+  return 0;
+}
+
+template <int BN, bool KN>
+int launch_tc(const F32Args& g, int grid, cudaStream_t st) {
+  const int rc = prepare_tc<BN, KN>();
+  if (rc) return rc;
   return launch_kernel(gemm_f32_tc_kernel<BN, KN>, dim3(grid), dim3(kThreads), Cfg<BN>::kSmem, st, g.split, g);
 }
 
@@ -396,6 +403,14 @@ bool gemm_f32_tc_takes(const float* a, long long sam, long long sak, const float
   if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) || sak != 1 || sam % 4 || K % 4) return false;
   if (static_cast<long long>((M + kBM - 1) / kBM) * ((N + 31) / 32) > 0x7fffffffLL) return false;
   return (sbk == 1 && sbn % 4 == 0) || (sbn == 1 && sbk % 4 == 0 && N % 4 == 0);
+}
+
+int gemm_f32_tc_prepare() {
+  int rc = 0;
+  if ((rc = prepare_tc<128, false>()) || (rc = prepare_tc<64, false>()) || (rc = prepare_tc<32, false>()) || (rc = prepare_tc<128, true>()) ||
+      (rc = prepare_tc<64, true>()))
+    return rc;
+  return 0;
 }
 
 double gemm_f32_tc_clocks(long long sbk, int M, int N, int K) { return choose(M, N, K, sbk != 1, sm_count()).clocks; }

@@ -727,6 +727,7 @@ int teeny_hybrid_create(const teeny_hybrid_config* cfg, const teeny_hybrid_layer
   // function attributes (dynamic shared memory) are set once per device here, outside any stream capture
   if (rc == 0) rc = gemm_bf16_prepare();
   if (rc == 0) rc = gemm_rows_prepare();
+  if (rc == 0) rc = gemm_f32_tc_prepare();
   if (rc == 0) rc = gemm_bf16_2cta_prepare();
   if (rc == 0) rc = state_scan_prepare();
   if (rc == 0) rc = window_attention_prepare();
