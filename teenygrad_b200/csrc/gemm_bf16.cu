@@ -47,6 +47,7 @@ struct GemmArgs {
   float* y32;             // when set (persistent kernel, unswapped): the f32 accumulators are stored as they are, to y32[M, ldy]
   const bf16* bias;       // [N] or null
   int tiles_p, tiles_q;   // tiles along P rows and along Q rows
+  int w_after_wait;       // skinny kernel: the weights are not to be read before the dependency wait
   int k_blocks;           // ceil(K / 64)
   int group;              // persistent kernel: P-tiles per raster group
   int kb_per_split;       // skinny kernel: k-blocks per cluster rank
@@ -536,7 +537,8 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     if (lane == 0) {
       // Weights are never written by a kernel of the stream, so the first ring of weight tiles is requested while
       // the previous kernel may still be running; the activation tiles follow once it has finished.
-      const int pre = min(kb1 - kb0, Cfg::kStages);
+      // (w_after_wait: a prefill's weights may be a copy that the kernel in front converts)
+      const int pre = args.w_after_wait ? 0 : min(kb1 - kb0, Cfg::kStages);
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), Cfg::kStageBytes);
         tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, full_bar(i), (kb0 + i) * Cfg::kKB, tile * kBM);
@@ -1080,6 +1082,8 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
       // wider cluster than that only adds barrier and reduction cost; with at least as many tiles as SMs no split.
       const int split = large.split ? large.split : skinny_split(tiles, a.k_blocks, sms);
       const int token_tiles = ceil_div(M, bn);
+      a.w_after_wait = large.split != 0;
+      if (a.w_after_wait) a.l2_ahead = 0;
       a.kb_per_split = ceil_div(a.k_blocks, split);
       {  // what the CTAs ask into L2 ahead of time must stay well inside it (126 MB): at most 48 MB over the grid
         const long long per_cta = (48ll << 20) / (static_cast<long long>(kBM * kBK * 2) * split * tiles);
