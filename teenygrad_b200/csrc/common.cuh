@@ -59,8 +59,8 @@ __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
 // programmatic dependent launch
 // ------------------------------------------------------------------------------------------------
 // Every kernel of this library calls pdl_wait() before it first touches memory that an earlier kernel in the
-// stream may still be writing; whatever it does before that (barrier init, TMEM allocation, fetching weights,
-// which no kernel writes) overlaps the tail of its predecessor.  pdl_trigger() lets the next kernel become resident:
+// stream may still be writing; whatever it does before that (barrier init, TMEM allocation, in a runner fetching a
+// model's weights, which no kernel of its steps writes) overlaps the tail of its predecessor.  pdl_trigger() lets the next kernel become resident:
 // the long kernels call it when their main loop is done, the short ones (norms, rope) right after their own wait, so
 // that the GEMM or attention kernel behind them streams its first ring of weights or cache tiles while they run.
 // No kernel triggers before its own wait has returned: at most two later kernels are ever resident beside the

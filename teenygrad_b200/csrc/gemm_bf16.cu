@@ -47,11 +47,11 @@ struct GemmArgs {
   float* y32;             // when set (persistent kernel, unswapped): the f32 accumulators are stored as they are, to y32[M, ldy]
   const bf16* bias;       // [N] or null
   int tiles_p, tiles_q;   // tiles along P rows and along Q rows
-  int w_after_wait;       // skinny kernel: the weights are not to be read before the dependency wait
+  int w_early;            // skinny kernel: the weights may be read before the dependency wait
   int k_blocks;           // ceil(K / 64)
   int group;              // persistent kernel: P-tiles per raster group
   int kb_per_split;       // skinny kernel: k-blocks per cluster rank
-  int l2_ahead;           // skinny kernel: weight k-blocks asked into L2 beyond the shared-memory ring at start
+  int l2_ahead;           // skinny kernel: weight k-blocks asked into L2 beyond the shared-memory ring at start; -1: not the ring's either
   int swiglu;             // GLU kind (glu_f): W rows interleave 64 gate / 64 up channels; Y[M, N/2] = act(gate) * up
   // Tensor-parallel push (skinny kernel only): instead of Y, the f32 row sums go to slot `rank` of every rank's
   // receive buffer (peer-mapped memory, [M][N] f32 each) and each CTA then bumps every rank's arrival counter.
@@ -535,17 +535,18 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 
   if (warp == 0) {
     if (lane == 0) {
-      // Weights are never written by a kernel of the stream, so the first ring of weight tiles is requested while
-      // the previous kernel may still be running; the activation tiles follow once it has finished.
-      // (w_after_wait: a prefill's weights may be a copy that the kernel in front converts)
-      const int pre = args.w_after_wait ? 0 : min(kb1 - kb0, Cfg::kStages);
+      // A model's weights are not written by any kernel of its steps (w_early), so the first ring of weight tiles is requested
+      // while the previous kernel may still be running; the activation tiles follow once it has finished.  Weights that
+      // the kernel in front may be writing (an operator's, a prefill's converted copy) are only asked into L2, where its
+      // stores arrive, too.
+      const int ring = min(kb1 - kb0, Cfg::kStages), pre = args.w_early ? ring : 0;
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), Cfg::kStageBytes);
         tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, full_bar(i), (kb0 + i) * Cfg::kKB, tile * kBM);
       }
       // ... and the weight tiles behind them are asked into L2, so that HBM keeps streaming this kernel's weights for
       // as long as the predecessor's tail lasts, not just until the ring is full
-      for (int kb = kb0 + pre; kb < min(kb1, kb0 + pre + args.l2_ahead); ++kb)
+      for (int kb = kb0 + pre; kb < min(kb1, kb0 + (args.l2_ahead < 0 ? 0 : ring + args.l2_ahead)); ++kb)
         tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
       pdl_wait();
       auto load_x = [&](uint32_t sq, uint32_t bar, int kb) {  // the activation tile(s) of one stage: 64 k each
@@ -996,7 +997,7 @@ size_t gemm_bf16_scratch_bytes(int, int, int) { return 0; }
 // Y[M,N] = X[M,K] W^T (+bias).  w_is_kn: W given as [K, N] row-major (matmul_forward's B) instead of [N, K].
 int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, const bf16* bias, bf16* y, int ldy,
               int M, int N, int K, void*, size_t, cudaStream_t stream, int swiglu, const GemmPush* push, float* y32,
-              int l2_ahead) {
+              int l2_ahead, bool w_early) {
   if (!x || !w || (!y && !y32) || M <= 0 || N <= 0 || K <= 0) return TEENY_ERR_BAD_ARG;
   if (y32 && (!w_is_kn || swiglu || push || bias)) return TEENY_ERR_BAD_ARG;  // f32 output: the [K, N] form only
   if (swiglu < 0 || swiglu > kGluGelu) return TEENY_ERR_BAD_ARG;
@@ -1012,6 +1013,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
     g.glu = swiglu;
     g.y = y; g.ldy = ldy;
     g.M = M; g.N = N; g.K = K;
+    g.w_early = w_early;
     return gemm_rows(g, stream);
   }
 
@@ -1082,8 +1084,8 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
       // wider cluster than that only adds barrier and reduction cost; with at least as many tiles as SMs no split.
       const int split = large.split ? large.split : skinny_split(tiles, a.k_blocks, sms);
       const int token_tiles = ceil_div(M, bn);
-      a.w_after_wait = large.split != 0;
-      if (a.w_after_wait) a.l2_ahead = 0;
+      a.w_early = w_early && !large.split;
+      if (large.split) a.l2_ahead = -1;
       a.kb_per_split = ceil_div(a.k_blocks, split);
       {  // what the CTAs ask into L2 ahead of time must stay well inside it (126 MB): at most 48 MB over the grid
         const long long per_cta = (48ll << 20) / (static_cast<long long>(kBM * kBK * 2) * split * tiles);
@@ -1123,7 +1125,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
 // weight tile where the tiles alone fill the GPU).
 int gemm_w8a16_skinny(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float* w_scale, int scale_kind,
                       int group, const bf16* bias, bf16* y, int ldy, int M, int N, int K, cudaStream_t stream, bool swiglu,
-                      const GemmPush* push) {
+                      const GemmPush* push, bool w_early) {
   if (!x || !wq || !w_scale || !y || M <= 0 || M > kSwapMaxM || N <= 0 || K <= 0) return TEENY_ERR_BAD_ARG;
   if (scale_kind < 0 || scale_kind > 2 || (scale_kind == 2 && (group <= 0 || group % kBK != 0))) return TEENY_ERR_BAD_ARG;
   if (swiglu && (bias || N % 128 != 0)) return TEENY_ERR_BAD_ARG;
@@ -1134,6 +1136,7 @@ int gemm_w8a16_skinny(const bf16* x, int ldx, const uint8_t* wq, int ldw, const 
   a.k_blocks = ceil_div(K, 2 * kBK);  // a stage of the W8 variant is 128 k wide
   a.swiglu = swiglu ? 1 : 0;
   a.w_scale = w_scale; a.w_scale_kind = scale_kind; a.w_group = group; a.w_mul16 = 16u;
+  a.w_early = w_early;
   if (push) {
     if (swiglu || !push->recv || !push->epoch || push->world < 2 || push->round >= 1023) return TEENY_ERR_BAD_ARG;
     a.push_recv = push->recv;
@@ -1177,7 +1180,7 @@ int gemm_w8a16_skinny(const bf16* x, int ldx, const uint8_t* wq, int ldw, const 
 // rows; row stride ldx8 bytes), x_scale[M].  Nothing is converted inside: kind::f8f6f4 on the bytes as they are.
 int gemm_w8a8x2_skinny(const uint8_t* x8, int ldx8, const float* x_scale, const uint8_t* wq, int ldw, const float* w_scale,
                        int scale_kind, const bf16* bias, bf16* y, int ldy, int M, int N, int K, cudaStream_t stream,
-                       bool swiglu, const GemmPush* push) {
+                       bool swiglu, const GemmPush* push, bool w_early) {
   if (!x8 || !x_scale || !wq || !w_scale || !y || M <= 0 || M > kSwapMaxM || N <= 0 || K <= 0) return TEENY_ERR_BAD_ARG;
   if (scale_kind < 0 || scale_kind > 1) return TEENY_ERR_BAD_ARG;  // per-group weight scales need the converting variant
   if (swiglu && (bias || N % 128 != 0)) return TEENY_ERR_BAD_ARG;
@@ -1188,6 +1191,7 @@ int gemm_w8a8x2_skinny(const uint8_t* x8, int ldx8, const float* x_scale, const 
   a.k_blocks = ceil_div(K, 2 * kBK);
   a.swiglu = swiglu ? 1 : 0;
   a.w_scale = w_scale; a.w_scale_kind = scale_kind; a.w_group = 0; a.w_mul16 = 16u;
+  a.w_early = w_early;
   a.x_scale = x_scale; a.x_lo_row = M;
   if (push) {
     if (swiglu || !push->recv || !push->epoch || push->world < 2 || push->round >= 1023) return TEENY_ERR_BAD_ARG;

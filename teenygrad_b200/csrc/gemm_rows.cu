@@ -3,7 +3,8 @@
 // What bounds these calls is the way from one kernel to the next, not the bytes: at M = 1 a layer of a 1024-wide model has 31 MB of
 // weights, 5 us at HBM rate, and its seven kernels took 33 us.  So the kernel is built for a short chain:
 //   * the weights of a CTA (all of them: at most kMaxSmem) are requested by bulk copies at its very start, before the wait for
-//     the kernel in front, so that only the activations are left to fetch when that has ended;
+//     the kernel in front, so that only the activations are left to fetch when that has ended (weights that the kernel in front may
+//     have computed are asked into L2 instead, and copied behind the wait);
 //   * what stood between two GEMMs is part of them: the RMSNorm of the input rows in front (every CTA norms the few rows for
 //     itself), bias, gated linear unit or the addition into the residual stream behind;
 //   * little code: a short rolled loop of mma.m16n8k16 with the tokens as the 16-row A operand and 8 weight rows as B; no tensor
@@ -86,7 +87,12 @@ __global__ void __launch_bounds__(kThreads, 3) gemm_rows_kernel(const __grid_con
       mbar_expect_tx(bar, rows * g.K * kEs);
     }
     __syncwarp();
-    if (mine) bulk_load(smem_u32(smem) + lane * wp, static_cast<const uint8_t*>(g.w) + static_cast<size_t>(n) * g.ldw * kEs, g.K * kEs, bar);
+    const uint8_t* src = static_cast<const uint8_t*>(g.w) + static_cast<size_t>(n) * g.ldw * kEs;
+    if (!g.w_early) {
+      if (mine) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(src), "r"(g.K * kEs) : "memory");
+      pdl_wait();
+    }
+    if (mine) bulk_load(smem_u32(smem) + lane * wp, src, g.K * kEs, bar);
   }
   // columns behind K up to a whole block: zeros on both sides
   if (g.K & 63) {
@@ -325,7 +331,7 @@ int gemm_rows(const RowsGemm& in, cudaStream_t st) {
   RowsGemm g = in;
   const bool two = g.M > 8, w8 = g.w_scale != nullptr;
   if (!g.x || !g.w || !(g.y || g.add16 || g.add32) || !gemm_rows_takes(g.M, g.N, g.K, g.ldw, w8, g.norm)) return TEENY_ERR_BAD_ARG;
-  if (g.norm != kRowsNormNone && !g.norm_w) return TEENY_ERR_BAD_ARG;
+  if (g.norm != kRowsNormNone && (!g.norm_w || !g.w_early)) return TEENY_ERR_BAD_ARG;  // norm_w is always read ahead of the wait
   if (g.glu && (g.bias || g.add16 || g.add32 || g.N % 128)) return TEENY_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(g.x) | reinterpret_cast<uintptr_t>(g.w) | reinterpret_cast<uintptr_t>(g.norm_w)) & 15 || g.ldx % 8) return TEENY_ERR_ALIGNMENT;
   g.w_mul16 = 16u;

@@ -237,8 +237,8 @@ size_t linear_w8a16_scratch_bytes(int M, int N, int K) {
 
 int linear_w8a16(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float* scale, int kind, int group,
                  const bf16* bias, bf16* y, int ldy, int M, int N, int K, void* scratch, size_t scratch_bytes,
-                 cudaStream_t st, bool swiglu, const GemmPush* push) {
-  if (M <= 128) return gemm_w8a16_skinny(x, ldx, wq, ldw, scale, kind, group, bias, y, ldy, M, N, K, st, swiglu, push);
+                 cudaStream_t st, bool swiglu, const GemmPush* push, bool w_early) {
+  if (M <= 128) return gemm_w8a16_skinny(x, ldx, wq, ldw, scale, kind, group, bias, y, ldy, M, N, K, st, swiglu, push, w_early);
   if (push) return TEENY_ERR_BAD_ARG;
   if (!scratch || scratch_bytes < linear_w8a16_scratch_bytes(M, N, K)) return TEENY_ERR_SCRATCH;
   if (reinterpret_cast<uintptr_t>(scratch) & 15) return TEENY_ERR_ALIGNMENT;

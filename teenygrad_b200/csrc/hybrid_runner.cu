@@ -267,6 +267,7 @@ RowsGemm rows_call(const void* x, int ldx, const void* w, int ldw, int M, int N,
   g.bias = static_cast<const bf16*>(bias);
   g.glu = glu;
   g.M = M; g.N = N; g.K = K;
+  g.w_early = true;
   return g;
 }
 
@@ -280,7 +281,7 @@ int linear(teeny_hybrid* m, const void* x, int ldx, const void* w, int ldw, void
     return glu ? glu_interleaved_f32(out, ldo, static_cast<float*>(y), ldy, M, N / 2, glu, st) : 0;
   }
   return gemm_bf16(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, false, static_cast<const bf16*>(bias), static_cast<bf16*>(y), ldy, M, N,
-                   K, nullptr, 0, st, glu);
+                   K, nullptr, 0, st, glu, nullptr, nullptr, -1, /*w_early=*/true);
 }
 
 struct StepShape {

@@ -38,7 +38,10 @@ struct GemmPush {
 };
 int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, const bf16* bias, bf16* y, int ldy,
               int M, int N, int K, void* scratch, size_t scratch_bytes, cudaStream_t stream, int swiglu = 0,
-              const GemmPush* push = nullptr, float* y32 = nullptr, int l2_ahead = -1);
+              const GemmPush* push = nullptr, float* y32 = nullptr, int l2_ahead = -1, bool w_early = false);
+// w_early (here and below): no kernel that may still run writes the weights, so a decode-shaped GEMM (M <= 128) may fetch them before it
+// waits for its predecessor.  True of a model's weights in the runners; not of a public operator's w, which the kernel in front may have
+// computed.
 // y32 (w_is_kn only): store the f32 accumulators to y32[M, ldy] instead of rounding them to bf16 into y.
 // l2_ahead (decode-shaped GEMMs, M <= 128): how many of its 16 KB weight tiles beyond the shared-memory ring each CTA
 // asks into L2 before it waits for its predecessor (-1: the library default, none).  Worth it only where the
@@ -65,13 +68,13 @@ int gather_add_rms_norm_owner_bf16(const uint2* recv, size_t slot_elems, int wor
 // larger M: converted once into `scratch` (linear_w8a16_scratch_bytes) as bf16(value * scale), then the bf16 GEMM.
 int gemm_w8a16_skinny(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float* w_scale, int scale_kind,
                       int group, const bf16* bias, bf16* y, int ldy, int M, int N, int K, cudaStream_t stream,
-                      bool swiglu = false, const GemmPush* push = nullptr);
+                      bool swiglu = false, const GemmPush* push = nullptr, bool w_early = false);
 // FP8 weights AND two-term FP8 activations (split_e4m3 writes them: x = (hi + lo / 16) * x_scale[row], exact for
 // elements within 2^10 of their row's maximum): kind::f8f6f4 on the bytes as they are, M <= 128, scale kinds 0 and 1.
 int split_e4m3(const bf16* x, long long ldx, uint8_t* out, long long ldo, float* scale, int M, int K, cudaStream_t st);
 int gemm_w8a8x2_skinny(const uint8_t* x8, int ldx8, const float* x_scale, const uint8_t* wq, int ldw, const float* w_scale,
                        int scale_kind, const bf16* bias, bf16* y, int ldy, int M, int N, int K, cudaStream_t stream,
-                       bool swiglu = false, const GemmPush* push = nullptr);
+                       bool swiglu = false, const GemmPush* push = nullptr, bool w_early = false);
 int dequant_e4m3_bf16(const uint8_t* wq, long long ldw, const float* scale, int kind, int group, bf16* out, long long ldo,
                       int N, int K, cudaStream_t st);
 // out[N, K] = bf16((q - zero point) * scale) for the integer schemes: bits 8 (int8 [N, K]) or 4 (nibbles packed two per
@@ -84,7 +87,7 @@ int e4m3_count_nan(const uint8_t* p, size_t n, unsigned* count, cudaStream_t st)
 size_t linear_w8a16_scratch_bytes(int M, int N, int K);
 int linear_w8a16(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float* scale, int kind, int group,
                  const bf16* bias, bf16* y, int ldy, int M, int N, int K, void* scratch, size_t scratch_bytes,
-                 cudaStream_t st, bool swiglu = false, const GemmPush* push = nullptr);
+                 cudaStream_t st, bool swiglu = false, const GemmPush* push = nullptr, bool w_early = false);
 
 // Decode-shaped linear layer for few rows (M <= 16), its neighbours in the layer folded in (gemm_rows.cu):
 //   in   x [M, K] bf16; or the rows of a residual stream, RMS-normalised on the way in: kRowsNormBf16 as rms_norm_bf16 does it
@@ -111,6 +114,7 @@ struct RowsGemm {
   float* add32;
   int ldy;
   int M, N, K;
+  bool w_early;      // of w; a norm asks for it, of norm_w too
   uint32_t w_mul16;  // set by gemm_rows
 };
 bool gemm_rows_takes(int M, int N, int K, int ldw, bool w8, int norm);

@@ -416,16 +416,16 @@ int project(teeny_qwen3* m, const bf16* x, int ldx, const Weight& w, bf16* y, in
   if (w.q && x8 && T <= 128 && w.kind <= 1)
     return gemm_w8a8x2_skinny(m->at<uint8_t>(mlp_act ? m->off.a8 : m->off.y8), K,
                               m->at<float>(mlp_act ? m->off.a8_scale : m->off.y8_scale), w.q, K, w.scale, w.kind, nullptr, y,
-                              ldy, T, N, K, st, swiglu, push);
+                              ldy, T, N, K, st, swiglu, push, /*w_early=*/true);
   if (w.q) {
-    if (T <= 128) return linear_w8a16(x, ldx, w.q, K, w.scale, w.kind, w.group, nullptr, y, ldy, T, N, K, nullptr, 0, st, swiglu, push);
+    if (T <= 128) return linear_w8a16(x, ldx, w.q, K, w.scale, w.kind, w.group, nullptr, y, ldy, T, N, K, nullptr, 0, st, swiglu, push, /*w_early=*/true);
     const size_t need = static_cast<size_t>(w_rows) * K * sizeof(bf16);
     if (!m->fp8_scratch || m->fp8_scratch_bytes < need || (K & 7)) return TEENY_ERR_SCRATCH;
     TEENY_TRY(dequant_e4m3_bf16(w.q, K, w.scale, w.kind, w.group, static_cast<bf16*>(m->fp8_scratch), K, w_rows, K, st));
     wb = static_cast<const bf16*>(m->fp8_scratch);
   }
   if (fuse) return gemm_bf16_2cta(x, ldx, wb, K, nullptr, y, ldy, T, N, K, st, false, fuse);
-  return gemm_bf16(x, ldx, wb, K, false, nullptr, y, ldy, T, N, K, gs, m->off.gemm_scratch_bytes, st, swiglu, push);
+  return gemm_bf16(x, ldx, wb, K, false, nullptr, y, ldy, T, N, K, gs, m->off.gemm_scratch_bytes, st, swiglu, push, nullptr, -1, /*w_early=*/!w.q);
 }
 
 // Row-parallel projection delta = x W^T followed by the cross-rank sum.  Decode with peer buffers: the GEMM pushes
@@ -499,6 +499,7 @@ RowsGemm rows_call(const Weight& w, const void* x, int ldx, int T, int N, int K)
   g.w_scale = w.q ? w.scale : nullptr;
   g.w_scale_kind = w.kind;
   g.M = T; g.N = N; g.K = K;
+  g.w_early = true;
   return g;
 }
 
