@@ -176,7 +176,7 @@ __device__ __forceinline__ void rotate_tail(const HeadLinear& a, int h, int r0, 
 }
 
 // CTA = 32 output columns of one head for 16 MT rows.  MT = 1: the four warps split K and are summed through shared memory;
-// MT = 4: each warp 16 rows.  The weights (no kernel writes them) are requested before the dependency wait.
+// MT = 4: each warp 16 rows.  A model's weights (w_early: no kernel of its steps writes them) are requested before the dependency wait.
 constexpr int kHlCols = 32;
 constexpr int hl_smem_bytes(int mt, int K) { return (kHlCols + 16 * mt) * ((K + 15) / 16 * 16 + 8) * 2; }
 
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(128) head_linear_mma_kernel(const HeadLinear a
     rotate_tail<bf16>(a, h, r0, rows);
     return;
   }
+  if (!a.w_early) pdl_wait();
   const uint32_t sw = smem_u32(hl_smem), sx = sw + kHlCols * LD * 2;
   const bf16* w = static_cast<const bf16*>(a.w) + (static_cast<size_t>(h) * a.N + n0) * a.K;
   for (int idx = threadIdx.x; idx < kHlCols * CH; idx += 128) {
@@ -377,6 +378,7 @@ struct LatTcArgs {
   int tile_slots;      // slots of a tile
   int slots, ahead;    // of the ring; whether it holds two tiles
   uint32_t tmem_cols;
+  bool cache_early;    // see LatentAttn
   float scale_log2;
   int* err;
 };
@@ -549,7 +551,8 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmap_c, const __grid
                         const SeqDesc* __restrict__ seqs) {
   constexpr int HN = N / 2;  // rows whose weights a thread works out
   extern __shared__ uint8_t lat_raw[];
-  const SeqDesc seq = seqs[blockIdx.z];  // written well before the kernel in front of this one
+  if (!a.cache_early) pdl_wait();
+  const SeqDesc seq = seqs[blockIdx.z];
   const int row0 = blockIdx.y * N, n_rows = min(N, seq.len * a.H - row0);
   if (n_rows <= 0) {
     pdl_wait();
@@ -1046,6 +1049,7 @@ int latent_attention(const LatentAttn& a, const SeqDesc* seqs, int n_seqs, int l
     if (n >= 16 && tiles <= 65535) {
       t.out = static_cast<bf16*>(a.out);
       t.row_base = a.row_base;
+      t.cache_early = a.cache_early;
       t.H = a.H; t.D = a.D; t.DV = a.DV;
       t.scale_log2 = a.scale * 1.4426950408889634f;
       t.err = device_error_word();

@@ -847,7 +847,8 @@ __global__ void embedding_scaled_kernel(const int* __restrict__ ids, const T* __
 template <typename T, int VPT, bool POST>
 __global__ void residual_rms_norm_kernel(float* __restrict__ x, const T* __restrict__ delta, long long ldd, T* __restrict__ y,
                                          long long ldy, const float* __restrict__ w, int N, float eps, const int* __restrict__ rows,
-                                         const float* __restrict__ post, float mult) {
+                                         const float* __restrict__ post, float mult, bool w_early) {
+  if (!w_early) pdl_wait();
   const int nv = N >> 2;
   float4 g[VPT], p[POST ? VPT : 1];
 #pragma unroll
@@ -1146,7 +1147,7 @@ int embedding_scaled(const int* ids, const void* table, float* x, int T, int wid
 namespace {
 template <typename T>
 int launch_residual_norm(float* x, const void* delta, long long ldd, void* y, long long ldy, const float* w, int M, int N, float eps,
-                         const int* rows, const float* post, float mult, cudaStream_t st) {
+                         const int* rows, const float* post, float mult, bool w_early, cudaStream_t st) {
   const T* d = static_cast<const T*>(delta);
   T* yo = static_cast<T*>(y);
   const int nv = N / 4;
@@ -1165,9 +1166,9 @@ int launch_residual_norm(float* x, const void* delta, long long ldd, void* y, lo
 #define TEENY_RRN(V)                                                                                                                \
   do {                                                                                                                             \
     if (post) launch_kernel(residual_rms_norm_kernel<T, V, true>, dim3(M), dim3(threads), 0, st, 1, x, d, ldd, yo, ldy, w, N, eps, \
-                            rows, post, mult);                                                                                     \
+                            rows, post, mult, w_early);                                                                                     \
     else launch_kernel(residual_rms_norm_kernel<T, V, false>, dim3(M), dim3(threads), 0, st, 1, x, d, ldd, yo, ldy, w, N, eps,     \
-                       rows, post, mult);                                                                                          \
+                       rows, post, mult, w_early);                                                                                          \
   } while (0)
   if (vpt <= 1) TEENY_RRN(1);
   else if (vpt <= 2) TEENY_RRN(2);
@@ -1179,11 +1180,11 @@ int launch_residual_norm(float* x, const void* delta, long long ldd, void* y, lo
 }  // namespace
 
 int residual_rms_norm(float* x, const void* delta, long long ldd, void* y, long long ldy, const float* w, int M, int N, float eps,
-                      const int* rows, bool f32, cudaStream_t st, const float* post, float mult) {
+                      const int* rows, bool f32, cudaStream_t st, const float* post, float mult, bool w_early) {
   if (!x || !y || !w || M <= 0 || N <= 0) return TEENY_ERR_BAD_ARG;
   if (!delta) post = nullptr;
-  return f32 ? launch_residual_norm<float>(x, delta, ldd, y, ldy, w, M, N, eps, rows, post, mult, st)
-             : launch_residual_norm<bf16>(x, delta, ldd, y, ldy, w, M, N, eps, rows, post, mult, st);
+  return f32 ? launch_residual_norm<float>(x, delta, ldd, y, ldy, w, M, N, eps, rows, post, mult, w_early, st)
+             : launch_residual_norm<bf16>(x, delta, ldd, y, ldy, w, M, N, eps, rows, post, mult, w_early, st);
 }
 
 int tanh_rows(const void* x, long long ldx, void* y, long long ldy, int M, int N, bool f32, cudaStream_t st) {

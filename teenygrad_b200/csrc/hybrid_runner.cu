@@ -369,6 +369,7 @@ int run_latent_absorbed(teeny_hybrid* m, const Layer& L, const Branch& b, int e0
   in.RD = c.rot_dims; in.rot_off = -c.rot_dims;
   in.inv_freq = b.inv_freq; in.rot_scale = c.rot_scale;
   in.seqs = seqs; in.n_seqs = n;
+  in.w_early = true;
   TEENY_TRY(head_linear(in, st));
   LatentAttn a{};
   a.f32 = m->cfg.f32;
@@ -382,6 +383,7 @@ int run_latent_absorbed(teeny_hybrid* m, const Layer& L, const Branch& b, int e0
   a.scale = c.score_scale;
   a.scratch = m->at<void>(p.lat_scratch);
   a.scratch_bytes = p.lat_scratch_bytes;
+  a.cache_early = true;  // the kernel in front makes the queries
   TEENY_TRY(latent_attention(a, seqs, n, longest, st));
   HeadLinear out{};
   out.f32 = m->cfg.f32;
@@ -391,6 +393,7 @@ int run_latent_absorbed(teeny_hybrid* m, const Layer& L, const Branch& b, int e0
   out.y = element(m, p.mix, r0, L.n_out, b.out_col);
   out.ldy = L.n_out; out.y_head = c.vdim;
   out.H = H; out.N = c.vdim; out.K = KR; out.T = rows;
+  out.w_early = true;
   return head_linear(out, st);
 }
 
@@ -582,7 +585,7 @@ int norm(teeny_hybrid* m, const float* w, int T, cudaStream_t st) {
   const void* d = m->pending_delta ? m->at<void>(p.delta) : nullptr;
   m->pending_delta = false;
   return residual_rms_norm(m->at<float>(p.x), d, p.width_ld, m->at<void>(p.y), p.width_ld, w, T, m->cfg.width, m->cfg.eps, nullptr,
-                           m->cfg.f32 != 0, st, m->pending_post, m->cfg.residual_mult);
+                           m->cfg.f32 != 0, st, m->pending_post, m->cfg.residual_mult, /*w_early=*/true);
 }
 
 // y[T, N] = norm(residual) W^T: the norm goes along with the projection where nothing is pending and the rows are few.
@@ -646,7 +649,7 @@ int run_head(teeny_hybrid* m, const int* rows, int n, cudaStream_t st) {
   const Plan& p = m->p;
   void* y = m->at<void>(p.yrows);
   TEENY_TRY(residual_rms_norm(m->at<float>(p.x), m->at<void>(p.delta), p.width_ld, y, p.width_ld, m->final_norm, n, m->cfg.width,
-                              m->cfg.eps, rows, m->cfg.f32 != 0, st, m->pending_post, m->cfg.residual_mult));
+                              m->cfg.eps, rows, m->cfg.f32 != 0, st, m->pending_post, m->cfg.residual_mult, /*w_early=*/true));
   return linear(m, y, p.width_ld, m->lm_head, p.width_ld, m->at<void>(p.logits), p.vocab_ld, n, m->cfg.vocab, m->cfg.width, st);
 }
 

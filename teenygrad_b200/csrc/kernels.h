@@ -446,6 +446,7 @@ struct HeadLinear {
   float rot_scale;
   const SeqDesc* seqs;       // RD > 0: the entries that hold the T rows (row0 of the first is row 0 of x and y)
   int n_seqs;
+  bool w_early;              // of w (see gemm_bf16)
 };
 int head_linear(const HeadLinear& a, cudaStream_t st);
 // Causal attention of H query heads over one shared key per token whose first DV elements are the value: q [q_rows, ldq] with
@@ -464,6 +465,7 @@ struct LatentAttn {
   float scale;
   void* scratch;             // latent_attention_scratch_bytes(DV), or null (the keys are then not split over CTAs)
   size_t scratch_bytes;
+  bool cache_early;          // the kernel launched just before writes neither the cache nor the entries: both are read ahead of the wait
 };
 size_t latent_attention_scratch_bytes(int dv);
 int latent_attention_prepare();
@@ -474,9 +476,9 @@ int embedding_scaled(const int* ids, const void* table, float* x, int T, int wid
                      cudaStream_t st);
 // delta null: nothing is added.  rows null: row i -> y row i, and x is updated; else y row i comes from x row rows[i] (plus
 // its delta) and x stays as it is.
-// post: what is added is rms_norm(delta) * post * mult (post null: delta as it is).
+// post: what is added is rms_norm(delta) * post * mult (post null: delta as it is).  w_early: of w and post (see gemm_bf16).
 int residual_rms_norm(float* x, const void* delta, long long ldd, void* y, long long ldy, const float* w, int M, int N, float eps,
-                      const int* rows, bool f32, cudaStream_t st, const float* post = nullptr, float mult = 1.0f);
+                      const int* rows, bool f32, cudaStream_t st, const float* post = nullptr, float mult = 1.0f, bool w_early = false);
 int tanh_rows(const void* x, long long ldx, void* y, long long ldy, int M, int N, bool f32, cudaStream_t st);
 // act(gate) * up from rows interleaved in blocks of 64 (kGlu* of common.cuh), f32
 int glu_interleaved_f32(const float* gu, long long ld, float* out, long long ldo, int T, int inter, int kind, cudaStream_t st);

@@ -137,3 +137,63 @@ def test_fp8_prefill_converts_each_matrix_in_front_of_its_product(batch, prompt)
         # the head's few rows run in other kernels for other weight types: sums in another order, one rounding of 2^-9
         assert float((a.logits().float() - want.float()).norm() / want.float().norm()) < 2 ** -8
     assert a.device_error() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 16, 40])
+def test_head_linear_weights_just_before(rows):
+    """The matrices of a per-head product that dequant_fp8 has written."""
+    from teenygrad_b200 import ops
+    H, n, k = 16, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, H, k, generator=g, device="cuda").bfloat16()
+    src = [_fp8(g, H * n, k) for _ in range(3)]
+    scale = torch.full((H * n,), 0.001, device="cuda")
+    w, y = torch.zeros(H * n, k, dtype=torch.bfloat16, device="cuda"), torch.zeros(rows, H, n, dtype=torch.bfloat16, device="cuda")
+    _chain(lambda i: ops.dequant_fp8(src[i % 3], scale, out=w), lambda: ops.head_linear(x, w.view(H, n, k), out=y), torch.equal)
+    assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("post", [False, True])
+def test_norm_weights_just_before(post):
+    """The weights of the residual norm that the sum of two vectors has made."""
+    from teenygrad_b200 import ops
+    rows, n = 600, 4096
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x0 = torch.randn(rows, n, generator=g, device="cuda")
+    delta = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    src = [torch.randn(rows, n, generator=g, device="cuda") for _ in range(3)]
+    zero, x, none = torch.zeros(rows, n, device="cuda"), x0.clone(), torch.zeros(rows, n, device="cuda").bfloat16()
+    w = torch.zeros(rows, n, device="cuda")
+
+    def write(i):
+        # one norm in front whose f32 rows w (the last one is used) become src: it lets the next kernel in before it writes
+        w.copy_(src[i % 3])
+        ops.residual_rms_norm(w, delta, zero[0], 1e-6)
+
+    def use():
+        y = ops.residual_rms_norm(x, none, w[rows - 1], 1e-6, w[rows - 2] if post else None)
+        return y
+    _chain(write, use, torch.equal)
+    assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("rows,cached", [(1, 700), (4, 300)])
+def test_latent_cache_written_just_before(rows, cached):
+    """The cached rows of an entry that latent_prepare has written, with nothing between it and the attention."""
+    from teenygrad_b200 import ops
+    H, rank, rot = 16, 256, 64
+    dim, n = rank + rot, cached + rows
+    g = torch.Generator(device="cuda").manual_seed(cached)
+    q = torch.randn(rows, H, dim, generator=g, device="cuda").bfloat16()
+    src = [torch.randn(n, 64 + rank + rot, generator=g, device="cuda").bfloat16() for _ in range(3)]
+    qw, cw = torch.ones(64, device="cuda"), torch.ones(rank, device="cuda")
+    freq = 1.0 / 1e4 ** (torch.arange(rot // 2, device="cuda").float() / (rot // 2))
+    cache = torch.zeros(1, n, dim, dtype=torch.bfloat16, device="cuda")
+    whole, last = ops.seq_table([(0, 0, 0, n)]), ops.seq_table([(0, cached, 0, rows)])
+    scratch = torch.empty(ops.lib.teeny_latent_attention_scratch_bytes(rank), dtype=torch.uint8, device="cuda")
+    y = torch.zeros(rows, H, rank, dtype=torch.bfloat16, device="cuda")
+
+    def write(i):
+        ops.latent_prepare(src[i % 3], (0, 64, 64 + rank), 64, rank, qw, cw, freq, 1e-6, cache, whole, n)
+    _chain(write, lambda: ops.latent_attention(q, cache, rank, dim ** -0.5, last, rows, out=y, scratch=scratch), torch.equal)
+    assert ops.device_error() == 0
