@@ -558,9 +558,9 @@ int window_attention(const WindowAttn& a, const SeqDesc* seqs, int n_seqs, int m
     s.B = n_seqs; s.Sq = 1; s.Skv = a.ring;
     s.gate = static_cast<const bf16*>(a.gate); s.gate_sb = a.ldg;
     const DecodeRing ring{seqs, a.slots};
-    // (the kernel before this one, head_norm_rope_rows, wrote q and each sequence's newest ring row)
     return attention_decode_bf16(static_cast<const bf16*>(a.q), static_cast<const bf16*>(a.k_ring), static_cast<const bf16*>(a.v_ring),
-                                 static_cast<bf16*>(a.out), s, 0, nullptr, a.scratch, a.scratch_bytes, st, 1, nullptr, a.counters, &ring);
+                                 static_cast<bf16*>(a.out), s, 0, nullptr, a.scratch, a.scratch_bytes, st, a.ring_early ? 1 : -1, nullptr, a.counters,
+                                 &ring);
   }
   const bool prefill = rows16 && a.D <= 192 && a.DV <= 128 && a.scale > 0.0f;
   if (prefill && a.keys == kKeysInRing && a.host && a.window >= a.ring && max_len >= kPrefillLen) {

@@ -337,6 +337,7 @@ int run_full_attention(teeny_hybrid* m, const Layer& L, const Branch& b, const S
   a.scale = c.score_scale; a.out_scale = c.out_scale;
   a.slots = m->cfg.max_batch;
   a.keys = kKeysInRing;
+  a.ring_early = true;
   a.scratch = m->at<void>(p.attn_scratch);
   a.scratch_bytes = p.attn_scratch_bytes;
   a.counters = m->at<unsigned>(p.attn_counters);
@@ -518,6 +519,7 @@ int run_attention(teeny_hybrid* m, const Layer& L, const Branch& b, const StepSh
   a.slots = m->cfg.max_batch;
   a.uniform_fresh = s.uniform_fresh;
   a.keys = single ? kKeysInRing : kKeysSplit;
+  a.ring_early = true;
   a.scratch = m->at<void>(p.attn_scratch);
   a.scratch_bytes = p.attn_scratch_bytes;
   a.counters = m->at<unsigned>(p.attn_counters);

@@ -375,6 +375,7 @@ struct WindowAttn {
   long long ldg;
   const SeqDesc* host;       // the entries in host memory, where the caller has them: with kKeysInRing groups of equal long entries,
                              // with kKeysInNew a single long entry, then run on the tcgen05 kernel
+  bool ring_early;           // the kernel launched just before writes nothing that is read here but q and each entry's newest ring row
 };
 // Per-head RMSNorm of q (in place) and k (k_raw -> k_out), then rotary positions on the first rot_dims dimensions
 // (i with i + rot_dims / 2), angles position * inv_freq[i] in f32, cos and sin times rot_scale.  q_w / k_w null: no norm.

@@ -197,3 +197,25 @@ def test_latent_cache_written_just_before(rows, cached):
         ops.latent_prepare(src[i % 3], (0, 64, 64 + rank), 64, rank, qw, cw, freq, 1e-6, cache, whole, n)
     _chain(write, lambda: ops.latent_attention(q, cache, rank, dim ** -0.5, last, rows, out=y, scratch=scratch), torch.equal)
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("cached,cap", [(300, 512), (1500, 1600), (5000, 5120)])
+def test_cached_rows_written_just_before(cached, cap):
+    """All cached rows of an entry, and not only the newest, from the operator in front of its attention (rope_cache over a whole prompt)."""
+    from teenygrad_b200 import ops
+    H, G, D = 16, 8, 128
+    g = torch.Generator(device="cuda").manual_seed(cached)
+    q = torch.randn(1, H, D, generator=g, device="cuda").bfloat16()
+    src = [(torch.randn(cached, G, D, generator=g, device="cuda").bfloat16(), torch.randn(cached, G, D, generator=g, device="cuda").bfloat16()) for _ in range(3)]
+    qs = torch.zeros(cached, H, D, dtype=torch.bfloat16, device="cuda")
+    freq = 1.0 / 1e4 ** (torch.arange(D // 2, device="cuda").float() / (D // 2))
+    kc, vc = (torch.zeros(1, G, cap, D, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    whole = ops.seq_table([(0, 0, 0, cached)])
+    last = (ops.seq_table([(0, cached - 1, 0, 1)]), ops.seq_table([(0, cached - 1, 0, 1)], "cpu"))
+    scratch = (torch.empty(ops.lib.teeny_attn_decode_scratch_bytes(1, H, 128, cap), dtype=torch.uint8, device="cuda"), torch.zeros(G, dtype=torch.int32, device="cuda"))
+    y = torch.zeros(1, H, D, dtype=torch.bfloat16, device="cuda")
+
+    def write(i):
+        ops.rope_cache(qs, *src[i % 3], kc, vc, freq, D, whole, cached)
+    _chain(write, lambda: ops.cached_attention(q, kc, vc, D ** -0.5, last, out=y, scratch=scratch), torch.equal)
+    assert ops.device_error() == 0
