@@ -7,6 +7,7 @@
 // is one cluster, whose CTAs hand each other their parts (m, l, O) through distributed shared memory; of more parts they go to
 // scratch, merged by the last CTA to arrive or by a second kernel.
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -44,7 +45,6 @@ struct DecodeArgs {
   // dependency wait.  < 0: nothing is known, read everything after the wait.
   int fresh_rows;
   int stages;          // ring depth of this launch
-  int clustered;       // the CTAs of a sequence are one cluster and merge there (no scratch, no counters)
   unsigned* counters;  // [B * Hkv] arrival counters (zero between calls) for the in-kernel merge, or null
   float scale_log2;
   int* err;
@@ -74,7 +74,8 @@ __device__ __forceinline__ void st_cluster_f32(const void* local, unsigned rank,
                :: "r"(smem_u32(local)), "r"(rank), "f"(v) : "memory");
 }
 
-template <int G, int HD>
+// CLUSTERED: the CTAs of a sequence are one cluster and merge there (no scratch, no counters).  FUSED: with the front end (a.rope).
+template <int G, int HD, bool CLUSTERED, bool FUSED>
 __global__ void __launch_bounds__(kDecThreads, 2)
 attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         const DecodeArgs a) {
@@ -82,9 +83,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   __shared__ float sm_ml[4][8][2];
   constexpr int kDecStageBytes = dec_stage_bytes(HD), kVTile = (HD / 64) * kDecBox;
   __shared__ float sm_o[4][G][HD];
-  __shared__ __align__(16) bf16 sm_q[4][G][HD];  // normed, rotated q heads, one copy per consumer warp (fused front end)
+  __shared__ __align__(16) bf16 sm_q[FUSED ? 4 : 1][G][FUSED ? HD : 1];  // normed, rotated q heads, one copy per consumer warp (fused front end)
   // clustered merge: this CTA's slice of the outputs from every CTA of the cluster, and everyone's (m, l)
-  __shared__ float cl_o[G * HD + kDecMaxCluster], cl_ml[kDecMaxCluster][G][2];
+  __shared__ float cl_o[CLUSTERED ? G * HD + kDecMaxCluster : 1], cl_ml[CLUSTERED ? kDecMaxCluster : 1][G][2];
   const uint32_t base = (smem_u32(dec_smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = dec_smem_raw + (base - smem_u32(dec_smem_raw));
   const int n_stages = a.stages;
@@ -103,8 +104,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     mbar_fence_init();
   }
   __syncthreads();
-  if (a.clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  if (CLUSTERED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
   // the live keys are divided evenly (in whole 64-key tiles) over the gridDim.x CTAs of this (batch, kv head)
+  const int parts = gridDim.x;
   int L = 0, span = 0, key_begin = 0, key_end = 0, n_tiles = 0;
   int cb = b, newest = 0;  // row of the cache tensors; cache row of the newest key
   auto plan = [&]() {
@@ -117,7 +119,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       L = a.kv_len_dev ? *a.kv_len_dev : a.kv_len;
       newest = L - 1;
     }
-    span = ((L + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x) + kDecTile - 1) / kDecTile * kDecTile;
+    span = ((L + parts - 1) / parts + kDecTile - 1) / kDecTile * kDecTile;
     key_begin = chunk * span;
     key_end = min(L, key_begin + span);
     n_tiles = key_begin < L ? (key_end - key_begin + kDecTile - 1) / kDecTile : 0;
@@ -137,11 +139,10 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   // Fused front end (per-head RMSNorm + RoPE + cache append), one 128-wide head per half-warp, no CTA-wide barrier: every consumer
   // warp prepares its own copy of the G query heads, and the warp that owns the newest key norms / rotates it, appends it and the
   // new value to the caches and writes both into the tile in shared memory, which was requested with whatever the caches held there.
-  const bool fused = HD == kHD && a.rope.k_new != nullptr;
   const int sub = lane & 15, hw = lane >> 4;
   uint4 wq_raw = {}, wk_raw = {}, craw = {}, sraw = {};  // norm weights and table rows of this lane's eight elements
   auto rope_constants = [&]() {
-    if (!fused || warp == 4) return;
+    if (!FUSED || warp == 4) return;
     const int tp = rope_pos < a.rope.max_len ? rope_pos : a.rope.max_len - 1;
     wq_raw = __ldg(reinterpret_cast<const uint4*>(a.rope.q_w + sub * 8));
     wk_raw = __ldg(reinterpret_cast<const uint4*>(a.rope.k_w + sub * 8));
@@ -150,13 +151,13 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   };
   if (a.fresh_rows >= 0) {
     plan();
-    if (a.rope.k_new) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
+    if (FUSED) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
     rope_constants();
     if (threadIdx.x == 128) {
       // first ring of tiles that hold none of the rows the previous kernel is still writing
       // (the fresh rows end at the newest key; in a ring older rows may follow it; the fused front end has none)
       while (pre < n_tiles && pre < n_stages &&
-             (fused || key_begin + (pre + 1) * kDecTile <= newest + 1 - a.fresh_rows || key_begin + pre * kDecTile > newest)) {
+             (FUSED || key_begin + (pre + 1) * kDecTile <= newest + 1 - a.fresh_rows || key_begin + pre * kDecTile > newest)) {
         load_tile(pre, pre);
         ++pre;
       }
@@ -165,13 +166,13 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   pdl_wait();  // the cache rows of this step (and, unless declared stable, the live length) come from earlier kernels
   if (a.fresh_rows < 0) {
     plan();
-    if (a.rope.k_new) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
+    if (FUSED) rope_pos = a.rope.pos_dev ? *a.rope.pos_dev : a.rope.pos;
     rope_constants();
   }
   const int g = lane >> 2, c = lane & 3;
   float acc[HD / 8][4];
   float m = -INFINITY, l = 0.0f;
-  if (n_tiles == 0 && !a.clustered) return;  // chunk lies beyond the live length (uniform for the CTA)
+  if (n_tiles == 0 && !CLUSTERED) return;  // chunk lies beyond the live length (uniform for the CTA)
 
   if (warp == 4) {
     // ---------------- producer ----------------
@@ -192,7 +193,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     uint32_t qa[HD / 16][2];
     // the newest key and value, held by the half-warps of the one warp that owns them (fused front end)
     const int new_rel = rope_pos - key_begin;
-    const bool has_new = fused && rope_pos < a.rope.max_len && rope_pos >= key_begin && rope_pos < key_end && ((new_rel >> 4) & 3) == warp;
+    const bool has_new = FUSED && rope_pos < a.rope.max_len && rope_pos >= key_begin && rope_pos < key_end && ((new_rel >> 4) & 3) == warp;
     uint4 new_row = make_uint4(0u, 0u, 0u, 0u);
     {
       if (has_new) {
@@ -203,7 +204,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                             : a.rope.v_cache + b * a.vc_sb + hk * a.vc_sh + rope_pos * a.vc_ss;
         *reinterpret_cast<uint4*>(dst + sub * 8) = new_row;
       }
-      if (fused) {
+      if constexpr (FUSED) {
 #pragma unroll
         for (int h0 = 0; h0 < G; h0 += 2) {  // two heads per pass (a lone last head is done twice)
           const int hsel = h0 + hw < G ? h0 + hw : G - 1;
@@ -213,7 +214,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         }
         __syncwarp();
       }
-      const bf16* qp = fused ? &sm_q[warp][g < G ? g : 0][0] : a.q + b * a.q_sb + (hk * G + (g < G ? g : 0)) * a.q_sh;
+      const bf16* qp = a.q + b * a.q_sb + (hk * G + (g < G ? g : 0)) * a.q_sh;
+      if constexpr (FUSED) qp = &sm_q[warp][g < G ? g : 0][0];
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks) {
         const int d0 = 16 * ks + 2 * c, d1 = d0 + 8;
@@ -339,8 +341,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     a.o[b * a.o_sb + (hk * G + gg) * a.o_sh + d] = __float2bfloat16_rn(oo);
   };
   const size_t slot = (static_cast<size_t>(b) * a.Hkv + hk) * a.max_chunks + chunk;
-  const int n_cta = gridDim.x, slice = (G * HD + n_cta - 1) / n_cta;  // clustered: CTA i finishes outputs i * slice ..
-  if (a.clustered) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster is running
+  const int slice = CLUSTERED ? (G * HD + parts - 1) / parts : G * HD;  // CTA i of a cluster finishes outputs i * slice ..
+  if (CLUSTERED) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster is running
   for (int idx = threadIdx.x; idx < G * HD; idx += kDecThreads) {
     const int gg = idx / HD, d = idx - gg * HD;
     float mm = -INFINITY;
@@ -354,17 +356,17 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       ll += sm_ml[w][gg][1] * sc;
       oo += sm_o[w][gg][d] * sc;
     }
-    if (a.clustered) {
+    if (CLUSTERED) {
       const unsigned owner = idx / slice;
       st_cluster_f32(&cl_o[chunk * slice + idx - owner * slice], owner, oo);
       if (d == 0)
-        for (int to = 0; to < n_cta; ++to) {
+        for (int to = 0; to < parts; ++to) {
           st_cluster_f32(&cl_ml[chunk][gg][0], to, mm);
           st_cluster_f32(&cl_ml[chunk][gg][1], to, ll);
         }
       continue;
     }
-    if (gridDim.x == 1) {  // whole sequence in this CTA: finish here, no partials
+    if (parts == 1) {  // whole sequence in this CTA: finish here, no partials
       finish(gg, d, mm, ll, oo);
       continue;
     }
@@ -375,15 +377,15 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     }
   }
   __syncwarp();
-  if (a.clustered) {
+  if (CLUSTERED) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     for (int i = threadIdx.x; i < slice; i += kDecThreads) {
       const int idx = chunk * slice + i;
       if (idx >= G * HD) break;
       const int gg = idx / HD, d = idx - gg * HD;
       float mm = -INFINITY, ll = 0.0f, oo = 0.0f;
-      for (int ch = 0; ch < n_cta; ++ch) mm = fmaxf(mm, cl_ml[ch][gg][0]);  // CTAs without keys hold -inf
-      for (int ch = 0; ch < n_cta; ++ch) {
+      for (int ch = 0; ch < parts; ++ch) mm = fmaxf(mm, cl_ml[ch][gg][0]);  // CTAs without keys hold -inf
+      for (int ch = 0; ch < parts; ++ch) {
         const float cm = cl_ml[ch][gg][0];
         const float sc = cm == -INFINITY ? 0.0f : ex2(cm - mm);
         ll = fmaf(cl_ml[ch][gg][1], sc, ll);
@@ -391,7 +393,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       }
       finish(gg, d, mm, ll, oo);
     }
-  } else if (gridDim.x > 1 && a.counters) {
+  } else if (parts > 1 && a.counters) {
     // The last CTA of this (sequence, kv head) to have stored its partial merges them all: no second kernel.
     __shared__ unsigned sm_last;
     __threadfence();
@@ -449,6 +451,30 @@ __global__ void attention_decode_combine_kernel(const float* __restrict__ part_o
   o[b * o_sb + h * o_sh + d] = __float2bfloat16_rn(oo / ll);
 }
 
+// f(kernel) for the variant of a group of g heads of size class hd
+template <typename F>
+void for_variant(int g, int hd, bool clustered, bool fused, F f) {
+  auto kind = [&](auto gg, auto dd) {
+    constexpr int G = decltype(gg)::value, HD = decltype(dd)::value;
+    if constexpr (HD == kHD) {
+      if (fused) {
+        if (clustered) f(attention_decode_kernel<G, HD, true, true>); else f(attention_decode_kernel<G, HD, false, true>);
+        return;
+      }
+    }
+    if (clustered) f(attention_decode_kernel<G, HD, true, false>); else f(attention_decode_kernel<G, HD, false, false>);
+  };
+  auto size = [&](auto gg) {
+    if (hd == 64) kind(gg, std::integral_constant<int, 64>{}); else kind(gg, std::integral_constant<int, 128>{});
+  };
+  switch (g) {
+    case 1: size(std::integral_constant<int, 1>{}); break;
+    case 2: size(std::integral_constant<int, 2>{}); break;
+    case 4: size(std::integral_constant<int, 4>{}); break;
+    default: size(std::integral_constant<int, 8>{}); break;
+  }
+}
+
 }  // namespace
 
 // Raises the decode kernel's dynamic shared-memory limit once per device.
@@ -458,14 +484,12 @@ int attention_decode_prepare() {
   cudaGetDevice(&dev);
   if (dev < 64 && (done.load(std::memory_order_acquire) >> dev) & 1ull) return 0;
   cudaError_t e = cudaSuccess;
-  auto raise = [&](auto kernel, int hd) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem_bytes(kDecStagesAlone, hd));
-  };
-  raise(attention_decode_kernel<1, 128>, 128); raise(attention_decode_kernel<2, 128>, 128);
-  raise(attention_decode_kernel<4, 128>, 128); raise(attention_decode_kernel<8, 128>, 128);
-  raise(attention_decode_kernel<1, 64>, 64); raise(attention_decode_kernel<2, 64>, 64);
-  raise(attention_decode_kernel<4, 64>, 64); raise(attention_decode_kernel<8, 64>, 64);
+  for (int hd : {64, 128})
+    for (int g : {1, 2, 4, 8})
+      for (int kind = 0; kind < (hd == kHD ? 4 : 2); ++kind)
+        for_variant(g, hd, kind & 1, kind & 2, [&](auto kernel) {
+          if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem_bytes(kDecStagesAlone, hd));
+        });
   if (e != cudaSuccess) return static_cast<int>(e);
   if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
   return 0;
@@ -570,8 +594,10 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
   // Parts of two tiles are worth a CTA of their own when the merge stays inside a cluster: 0.6 us instead of 3 through scratch, fence
   // and counter.  Decode step of a 28-layer model, batch 1, 8 kv heads, 576 rows (nine tiles): 675 us with one CTA for each head,
   // 601, 588 and 562 with parts of five, three and two tiles.  Three tiles in all are faster in one CTA (4k model, batch 8: 576 us a
-  // step against 581 with two parts).  The ring is no deeper than a part's tiles, which leaves room for the next kernel's CTAs.
+  // step against 581 with two parts).  The ring is no deeper than a part's tiles, which leaves room for
+  // the next kernel's CTAs.
   const int tiles = (s.Skv + kDecTile - 1) / kDecTile;
+  bool clustered = false;
   if (a.stages == kDecStagesAlone && n_split <= kDecMaxCluster) {
     int n = sms / bh;
     n = n < kDecMaxCluster ? n : kDecMaxCluster;
@@ -579,28 +605,19 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
     n = n < most ? n : most;
     if (n > 1) {
       n_split = n;
-      a.clustered = 1;
+      clustered = true;
       const int part = (tiles + n - 1) / n;
       if (part < a.stages) a.stages = part;
     }
   }
-  a.counters = n_split > 1 && !a.clustered ? counters : nullptr;
+  a.counters = n_split > 1 && !clustered ? counters : nullptr;
   const int smem = dec_smem_bytes(a.stages, HD);
   dim3 grid(n_split, s.Hkv, s.B);
-  const unsigned cl = a.clustered ? n_split : 1;
-#define TEENY_DEC(GG)                                                                                                     \
-  if (HD == 64) launch_kernel(attention_decode_kernel<GG, 64>, grid, dim3(kDecThreads), smem, stream, cl, mk, mv, a);      \
-  else launch_kernel(attention_decode_kernel<GG, 128>, grid, dim3(kDecThreads), smem, stream, cl, mk, mv, a)
-  switch (G) {
-    case 1: TEENY_DEC(1); break;
-    case 2: TEENY_DEC(2); break;
-    case 4: TEENY_DEC(4); break;
-    default: TEENY_DEC(8); break;
-  }
-#undef TEENY_DEC
+  const unsigned cl = clustered ? n_split : 1;
+  for_variant(G, HD, clustered, rope != nullptr, [&](auto kernel) { launch_kernel(kernel, grid, dim3(kDecThreads), smem, stream, cl, mk, mv, a); });
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (n_split == 1 || a.counters || a.clustered) return 0;
+  if (n_split == 1 || a.counters || clustered) return 0;
   launch_kernel(attention_decode_combine_kernel, dim3(s.Hq, s.B), dim3(kHD), 0, stream, 1, a.part_o, a.part_ml, o,
                 s.o_sb, s.o_sh, s.Hkv, G, max_chunks, n_split, kv_len, kv_len_dev);
   return static_cast<int>(cudaGetLastError());
