@@ -475,6 +475,37 @@ void for_variant(int g, int hd, bool clustered, bool fused, F f) {
   }
 }
 
+// Clusters of n CTAs with `stages` tiles of ring each that the GPU holds at once.  Asked from the runtime once per device and variant: it
+// depends on how many SMs each of the GPU's processing clusters has (six-stage rings: 74, 45, 33, 26, 22, 15, 15 of 2 to 8 CTAs).
+int resident_clusters(int g, int hd, bool fused, int n, int stages) {
+  constexpr int kDevices = 16;
+  static std::atomic<short> known[kDevices][4][3][kDecMaxCluster + 1][kDecStagesAlone + 1];  // number + 1
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<short>* slot = dev < kDevices ? &known[dev][g == 8 ? 3 : g >> 1][hd == 64 ? 0 : (fused ? 2 : 1)][n][stages] : nullptr;
+  if (slot)
+    if (const int v = slot->load(std::memory_order_relaxed)) return v - 1;
+  int count = 0;
+  for_variant(g, hd, true, fused, [&](auto kernel) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = n;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(n);
+    config.blockDim = dim3(kDecThreads);
+    config.dynamicSmemBytes = dec_smem_bytes(stages, hd);
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&count, kernel, &config) != cudaSuccess) {
+      cudaGetLastError();
+      count = 0;
+    }
+  });
+  if (slot) slot->store(static_cast<short>(count + 1), std::memory_order_relaxed);
+  return count;
+}
+
 }  // namespace
 
 // Raises the decode kernel's dynamic shared-memory limit once per device.
@@ -596,6 +627,8 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
   // 601, 588 and 562 with parts of five, three and two tiles.  Three tiles in all are faster in one CTA (4k model, batch 8: 576 us a
   // step against 581 with two parts).  The ring is no deeper than a part's tiles, which leaves room for
   // the next kernel's CTAs.
+  // All clusters have to be there at once: 16 of eight such CTAs are one too many, and the call takes two rounds (16 kv heads in all,
+  // 4096 rows: 17.5 us with eight parts, 11.8 with six; 48 kv heads: 34.2 with three, 23.3 with two; through scratch 12.7 and 24.6).
   const int tiles = (s.Skv + kDecTile - 1) / kDecTile;
   bool clustered = false;
   if (a.stages == kDecStagesAlone && n_split <= kDecMaxCluster) {
@@ -603,11 +636,16 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
     n = n < kDecMaxCluster ? n : kDecMaxCluster;
     const int most = tiles < 4 ? 1 : (tiles + 1) / 2;
     n = n < most ? n : most;
+    int stages = kDecStagesAlone;
+    for (; n > 1; --n) {
+      const int part = (tiles + n - 1) / n;
+      stages = part < kDecStagesAlone ? part : kDecStagesAlone;
+      if (resident_clusters(G, HD, rope != nullptr, n, stages) >= bh) break;
+    }
     if (n > 1) {
       n_split = n;
       clustered = true;
-      const int part = (tiles + n - 1) / n;
-      if (part < a.stages) a.stages = part;
+      a.stages = stages;
     }
   }
   a.counters = n_split > 1 && !clustered ? counters : nullptr;
