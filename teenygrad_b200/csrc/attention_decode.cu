@@ -67,6 +67,7 @@ constexpr int kDecBox = kDecTile * 64 * 2;       // 8 KB: [64 keys][64 d]
 constexpr int dec_stage_bytes(int hd) { return 2 * (hd / 64) * kDecBox; }  // K and V boxes: 32 KB for head size 128
 constexpr int dec_smem_bytes(int stages, int hd) { return stages * dec_stage_bytes(hd) + 1024 + 128; }
 constexpr int kDecMaxCluster = 8;
+constexpr int kDecAlone = 4 * kDecTile;          // live keys up to which one CTA of a cluster does them all, see attention_decode_bf16
 constexpr int kDecThreads = 160;                 // 4 consumer warps + 1 producer warp
 
 __device__ __forceinline__ void st_cluster_f32(const void* local, unsigned rank, float v) {
@@ -106,7 +107,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   __syncthreads();
   if (CLUSTERED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
   // the live keys are divided evenly (in whole 64-key tiles) over the gridDim.x CTAs of this (batch, kv head)
-  const int parts = gridDim.x;
+  int parts = gridDim.x;
   int L = 0, span = 0, key_begin = 0, key_end = 0, n_tiles = 0;
   int cb = b, newest = 0;  // row of the cache tensors; cache row of the newest key
   auto plan = [&]() {
@@ -119,6 +120,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       L = a.kv_len_dev ? *a.kv_len_dev : a.kv_len;
       newest = L - 1;
     }
+    if (CLUSTERED && !FUSED && L <= kDecAlone) parts = 1;
     span = ((L + parts - 1) / parts + kDecTile - 1) / kDecTile * kDecTile;
     key_begin = chunk * span;
     key_end = min(L, key_begin + span);
@@ -172,7 +174,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
   const int g = lane >> 2, c = lane & 3;
   float acc[HD / 8][4];
   float m = -INFINITY, l = 0.0f;
-  if (n_tiles == 0 && !CLUSTERED) return;  // chunk lies beyond the live length (uniform for the CTA)
+  if (n_tiles == 0 && !(CLUSTERED && parts > 1)) return;  // chunk lies beyond the live length (uniform for the CTA)
 
   if (warp == 4) {
     // ---------------- producer ----------------
@@ -341,8 +343,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     a.o[b * a.o_sb + (hk * G + gg) * a.o_sh + d] = __float2bfloat16_rn(oo);
   };
   const size_t slot = (static_cast<size_t>(b) * a.Hkv + hk) * a.max_chunks + chunk;
-  const int slice = CLUSTERED ? (G * HD + parts - 1) / parts : G * HD;  // CTA i of a cluster finishes outputs i * slice ..
-  if (CLUSTERED) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster is running
+  const bool exchange = CLUSTERED && parts > 1;
+  const int slice = exchange ? (G * HD + parts - 1) / parts : G * HD;  // CTA i of a cluster finishes outputs i * slice ..
+  if (exchange) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster is running
   for (int idx = threadIdx.x; idx < G * HD; idx += kDecThreads) {
     const int gg = idx / HD, d = idx - gg * HD;
     float mm = -INFINITY;
@@ -356,7 +359,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       ll += sm_ml[w][gg][1] * sc;
       oo += sm_o[w][gg][d] * sc;
     }
-    if (CLUSTERED) {
+    if (exchange) {
       const unsigned owner = idx / slice;
       st_cluster_f32(&cl_o[chunk * slice + idx - owner * slice], owner, oo);
       if (d == 0)
@@ -377,7 +380,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     }
   }
   __syncwarp();
-  if (CLUSTERED) {
+  if (exchange) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     for (int i = threadIdx.x; i < slice; i += kDecThreads) {
       const int idx = chunk * slice + i;
@@ -393,7 +396,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       }
       finish(gg, d, mm, ll, oo);
     }
-  } else if (parts > 1 && a.counters) {
+  } else if (!CLUSTERED && parts > 1 && a.counters) {
     // The last CTA of this (sequence, kv head) to have stored its partial merges them all: no second kernel.
     __shared__ unsigned sm_last;
     __threadfence();
@@ -625,7 +628,9 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
   // Parts of two tiles are worth a CTA of their own when the merge stays inside a cluster: 0.6 us instead of 3 through scratch, fence
   // and counter.  Decode step of a 28-layer model, batch 1, 8 kv heads, 576 rows (nine tiles): 675 us with one CTA for each head,
   // 601, 588 and 562 with parts of five, three and two tiles.  Three tiles in all are faster in one CTA (4k model, batch 8: 576 us a
-  // step against 581 with two parts).  The ring is no deeper than a part's tiles, which leaves room for
+  // step against 581 with two parts).  Without the front end it is four, and counted by the live keys, since there is no work of the
+  // parts' own to share: 16 kv heads, 256 rows 5.3 us in one CTA, 5.7 in two; 128 live of 256 4.3 and 5.2 (with it, 128 + 128 tokens of
+  // the 28-layer model at batch 2 take 78.3 ms that way against 76.6).  The ring is no deeper than a part's tiles, which leaves room for
   // the next kernel's CTAs.
   // All clusters have to be there at once: 16 of eight such CTAs are one too many, and the call takes two rounds (16 kv heads in all,
   // 4096 rows: 17.5 us with eight parts, 11.8 with six; 48 kv heads: 34.2 with three, 23.3 with two; through scratch 12.7 and 24.6).
@@ -634,7 +639,7 @@ int attention_decode_bf16(const bf16* q, const bf16* k, const bf16* v, bf16* o, 
   if (a.stages == kDecStagesAlone && n_split <= kDecMaxCluster) {
     int n = sms / bh;
     n = n < kDecMaxCluster ? n : kDecMaxCluster;
-    const int most = tiles < 4 ? 1 : (tiles + 1) / 2;
+    const int most = tiles <= (rope ? 3 : kDecAlone / kDecTile) ? 1 : (tiles + 1) / 2;
     n = n < most ? n : most;
     int stages = kDecStagesAlone;
     for (; n > 1; --n) {
