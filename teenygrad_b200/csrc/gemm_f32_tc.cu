@@ -113,6 +113,7 @@ __device__ __forceinline__ void store4(const F32Args& g, int m, int n, float4 v,
         if (n + q < g.N) out[q * g.scn] = y[q];
     }
   }
+  __syncwarp();  // what follows stores to the same places
   for (unsigned lanes = __ballot_sync(0xffffffffu, again != 0); lanes; lanes &= lanes - 1) {
     const int from = __ffs(lanes) - 1, mm = __shfl_sync(0xffffffffu, m, from), nn = __shfl_sync(0xffffffffu, n, from);
     for (unsigned cols = __shfl_sync(0xffffffffu, again, from); cols; cols &= cols - 1) {
