@@ -15,8 +15,11 @@
 // Measured against f32 multiply-adds on the CUDA cores: 1000 x 4096 x 1024 198 -> 66 us, error against 64 bits 5.7e-7 -> 1.1e-7;
 // 2048 x 4096 x 4096 1443 -> 439 us, 1.2e-6 -> 1.7e-7; 300 x 700 x 2000 45 -> 17 us; 512^3 14.1 -> 9.8 us.
 //
-// Infinities and NaNs split into NaNs, numbers near the largest one may round to infinity in the first term, and below 2^-110 or so
-// the third term runs out of exponent: results that are not finite or are smaller than 2^-100 are computed again, with f32 multiply-adds.
+// bf16 has the exponents of f32 but only eight bits, so the terms of a small number would run out of exponent: the third below 2^-110, all
+// three below 2^-134.  Both operands are therefore taken times 2^24, with which every term of every f32 number, the smallest subnormal
+// included, is a normal bf16 number or zero, and the sums leave tensor memory times 2^-48.  What that costs is at the other end: from
+// 2^104 on an operand, and from 2^80 on a sum, may overflow, infinities and NaNs split into NaNs, and results that are not finite
+// are computed again, with f32 multiply-adds.
 #include <atomic>
 
 #include "common.cuh"
@@ -29,7 +32,7 @@ namespace {
 constexpr int kBM = 128, kBK = 64;
 constexpr int kSplitWarps = 8, kSumWarps = 8;
 constexpr int kThreads = 32 * (kSplitWarps + kSumWarps);  // 16 warps: 128 registers each, the most with two warps of either kind per scheduler
-constexpr float kTiny = 7.8886090522101181e-31f, kLargest = 3.4028234663852886e38f;  // 2^-100, FLT_MAX
+constexpr float kUp = 0x1p24f, kDown = 0x1p-48f;  // of the operands, of the sums
 constexpr int kTileA = kBM * 128;  // one bf16 term of 64 k of A: 128 bytes per row
 template <int BN> struct Cfg {
   static constexpr int kTileB = BN * 128;
@@ -52,11 +55,12 @@ struct F32Args {
   int* err;
 };
 
-// two numbers -> their three bf16 terms, packed
+// two numbers -> the three bf16 terms of kUp times them, packed
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const f32x2 minus = pack2(-1.0f, -1.0f);
-  hi = pack_bf16x2(x, y);
-  const f32x2 r = fma2(pack2(bf16_lo(hi), bf16_hi(hi)), minus, pack2(x, y));
+  const f32x2 minus = pack2(-1.0f, -1.0f), v = mul2(pack2(x, y), pack2(kUp, kUp));
+  const float2 u = unpack2(v);
+  hi = pack_bf16x2(u.x, u.y);
+  const f32x2 r = fma2(pack2(bf16_lo(hi), bf16_hi(hi)), minus, v);
   const float2 f = unpack2(r);
   mid = pack_bf16x2(f.x, f.y);
   const float2 q = unpack2(fma2(pack2(bf16_lo(mid), bf16_hi(mid)), minus, r));
@@ -91,7 +95,7 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t local, uint32_t rank) {
   return v;
 }
 
-// Results (m, n .. n + 3) of every lane of a warp; what left the range of the split is computed again.
+// Results (m, n .. n + 3) of every lane of a warp; what is not finite is computed again.
 template <bool KN>
 __device__ __forceinline__ void store4(const F32Args& g, int m, int n, float4 v, int lane) {
   const float x[4] = {v.x, v.y, v.z, v.w};
@@ -100,8 +104,7 @@ __device__ __forceinline__ void store4(const F32Args& g, int m, int n, float4 v,
     float y[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float size = fabsf(x[q]);
-      if (!(size >= kTiny && size <= kLargest) && x[q] != 0.0f && n + q < g.N) again |= 1u << q;
+      if (!isfinite(x[q]) && n + q < g.N) again |= 1u << q;
       y[q] = x[q] + (g.bias && n + q < g.N ? __ldg(g.bias + n + q) : 0.0f);
     }
     float* out = g.c + m * g.scm + n * g.scn;
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
       umma_commit(acc_full(s));
       return true;
     };
-    const f32x2 one = pack2(1.0f, 1.0f);
+    const f32x2 down = pack2(kDown, kDown);
     const bool issuer = w == 0 && lane == 0;
     if (issuer && total > 0) issue(0);
     __syncwarp();
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
             if constexpr (kStep == 32) tmem_ld_32x32(addr + p * BN + c, r); else tmem_ld_32x16(addr + p * BN + c, r);
             tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < kStep; e += 2) acc[(c + e) / 2] = fma2(pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), one, acc[(c + e) / 2]);
+            for (int e = 0; e < kStep; e += 2) acc[(c + e) / 2] = fma2(pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), down, acc[(c + e) / 2]);
           }
         }
         tc_fence_before();

@@ -63,3 +63,29 @@ def test_numbers_at_the_limits(ops, M, N, K, kn):
     b = (48 + K // 64 + 12) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
     assert bool(((y.double() - e).abs() <= b)[ok].all())
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(2048, 2304, 64), (600, 1500, 320), (200, 1500, 1600), (512, 512, 512)])
+@pytest.mark.parametrize("kn", [False, True])
+@pytest.mark.parametrize("lo,hi,wlo,whi", [(-149, -126, 60, 127), (-134, -110, 20, 120), (-126, -90, -10, 90), (-100, -60, -48, -20), (90, 127, -149, -100), (100, 127, -90, -20),
+                                           (70, 110, -30, 17)])
+def test_single_products_over_all_exponents(ops, M, N, K, kn, lo, hi, wlo, whi):
+    """One product per result, down to the subnormals on one side and up to the largest numbers on the other: no sum hides what the split of
+    an operand loses."""
+    g = torch.Generator(device="cuda").manual_seed(K + lo)
+
+    def numbers(shape, lo, hi):
+        e = torch.randint(lo, hi + 1, shape, generator=g, device="cuda").double()
+        m = 1.0 + torch.randint(0, 1 << 23, shape, generator=g, device="cuda").double() * 2.0 ** -23
+        return (m * torch.where(torch.rand(shape, generator=g, device="cuda") < 0.5, -1.0, 1.0).double() * torch.exp2(e)).float()
+
+    x, w = torch.zeros(M, K, device="cuda"), numbers((N, K), wlo, whi)
+    at = torch.randint(0, K, (M,), generator=g, device="cuda")
+    x[torch.arange(M, device="cuda"), at] = numbers((M,), lo, hi)
+    y = ops.matmul_forward(x, w.T.contiguous()) if kn else ops.linear_forward(x, w, None)
+    e = x[torch.arange(M, device="cuda"), at].double()[:, None] * w[:, at].T.double()
+    # three products of 2^-24 each left out, five roundings of 2^-24, a half subnormal step
+    b = 8 * 2.0 ** -24 * e.abs() + 2.0 ** -149
+    over = e.abs() >= 2.0 ** 128 * (1 - 2.0 ** -25)
+    assert bool(torch.isinf(y)[over].all()) and bool(((y.double() - e).abs() <= b)[~over].all())
+    assert ops.device_error() == 0
