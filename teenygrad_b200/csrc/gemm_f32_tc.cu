@@ -6,20 +6,22 @@
 // 1e-6.  So the sum stays in it for 64 k only (smallest products first) and is then added to f32 registers, rounded.
 //
 // Bound: shared memory.  For 64 k of a 128 x 128 tile its 128 bytes a clock carry the f32 numbers in and out of L1 (1000 clocks), the
-// stores of the terms (770) and the reads of 24 MMAs (1540), 3300 in all against 770 of the tensor pipe; 3100 were measured.  A pass
+// stores of the terms (770) and the reads of 24 MMAs (1540), 3300 in all against 770 of the tensor pipe; 3100 were measured (by the counters L1 is 57 % busy and
+// the tensor pipe 47 %: the stages' hand-overs keep it from the rest).  A pass
 // that splits the operands beforehand would bring 6 bytes per number through L2 for every tile instead of 4.  So the split runs
 // beside the products: warps 0-7 load f32 rows, split them and store the three terms of each operand as swizzled tiles (two stages
 // of 96 KB), warps 8-15 move finished 64-k sums from tensor memory (two accumulators) into registers; a lane of warp 8 issues
 // the MMAs of a chunk before it turns to the sums of the chunk before.  (16 splitting warps with the registers divided anew: no
 // faster, 427 against 418 us for 2048 x 4096 x 4096.)
-// Measured against f32 multiply-adds on the CUDA cores: 1000 x 4096 x 1024 198 -> 66 us, error against 64 bits 5.7e-7 -> 1.1e-7;
-// 2048 x 4096 x 4096 1443 -> 439 us, 1.2e-6 -> 1.7e-7; 300 x 700 x 2000 45 -> 17 us; 512^3 14.1 -> 9.8 us.
+// Measured against f32 multiply-adds on the CUDA cores: 1000 x 4096 x 1024 198 -> 69 us, error against 64 bits 5.7e-7 -> 1.1e-7;
+// 2048 x 4096 x 4096 1447 -> 478 us, 1.2e-6 -> 1.7e-7; 300 x 700 x 2000 46 -> 17 us; 512^3 14.1 -> 9.6 us.
 //
 // bf16 has the exponents of f32 but only eight bits, so the terms of a small number would run out of exponent: the third below 2^-110, all
 // three below 2^-134.  Both operands are therefore taken times 2^24, with which every term of every f32 number, the smallest subnormal
 // included, is a normal bf16 number or zero, and the sums leave tensor memory times 2^-48.  What that costs is at the other end: from
-// 2^104 on an operand, and from 2^80 on a sum, may overflow, infinities and NaNs split into NaNs, and results that are not finite
-// are computed again, with f32 multiply-adds.
+// 2^104 on an operand, and from 2^80 on a sum, may overflow, infinities and NaNs split into NaNs, and the sums of a tile with results that
+// are not finite are made again for these, with f32 multiply-adds (every result infinite: 2048 x 4096 x 4096 2.9 ms, 512^3 34 us).  The scale costs
+// up to 8 % with B as [N][K] (2048 x 4096 x 4096: 439 us without) and nothing with [K][N].
 #include <atomic>
 
 #include "common.cuh"
@@ -67,27 +69,6 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
   lo = pack_bf16x2(q.x, q.y);
 }
 
-// Element (m, n) in f32 multiply-adds by a whole warp; a NaN once there stays.
-template <bool KN>
-__device__ __noinline__ float plain_dot(const F32Args& g, int m, int n, int lane) {
-  const float* a = g.a + m * g.lda;
-  const float* b = KN ? g.b + n : g.b + n * g.ldb;
-  float s = 0.0f;
-  for (int k0 = 0; k0 < g.K; k0 += 256) {
-    float x[8], y[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int k = k0 + i * 32 + lane;
-      x[i] = k < g.K ? a[k] : 0.0f;
-      y[i] = k < g.K ? b[KN ? k * g.ldb : k] : 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s = fmaf(x[i], y[i], s);
-    if (__any_sync(0xffffffffu, s != s)) break;
-  }
-  return warp_sum(s);
-}
-
 __device__ __forceinline__ float4 ld_cluster4(uint32_t local, uint32_t rank) {
   float4 v;
   asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
@@ -95,37 +76,108 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t local, uint32_t rank) {
   return v;
 }
 
-// Results (m, n .. n + 3) of every lane of a warp; what is not finite is computed again.
-template <bool KN>
-__device__ __forceinline__ void store4(const F32Args& g, int m, int n, float4 v, int lane) {
+// Results (m, n .. n + 3); whether one of them is not finite.
+__device__ __forceinline__ bool store4(const F32Args& g, int m, int n, float4 v) {
+  if (m >= g.M) return false;
   const float x[4] = {v.x, v.y, v.z, v.w};
-  unsigned again = 0;
-  if (m < g.M) {
-    float y[4];
+  float y[4];
+  bool again = false;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (!isfinite(x[q]) && n + q < g.N) again |= 1u << q;
-      y[q] = x[q] + (g.bias && n + q < g.N ? __ldg(g.bias + n + q) : 0.0f);
+  for (int q = 0; q < 4; ++q) {
+    again |= !isfinite(x[q]) && n + q < g.N;
+    y[q] = x[q] + (g.bias && n + q < g.N ? __ldg(g.bias + n + q) : 0.0f);
+  }
+  float* out = g.c + m * g.scm + n * g.scn;
+  if (g.scn == 1 && n + 4 <= g.N && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (n + q < g.N) out[q * g.scn] = y[q];
+  }
+  return again;
+}
+
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool there) {  // zeros where nothing is
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+// The results of rows m0 .. m0 + 16 TM - 1 and columns n0 .. n0 + BN - 1 that are not finite, in f32 multiply-adds in the order of k, by all
+// threads of the CTA: a warp has TM rows, a lane BN / 32 columns.  32 k at a time in two buffers; the next are on their way while one is
+// multiplied.  The whole tile is summed whatever the number of such results, at about the rate of the CUDA-core kernel, and the finite
+// ones keep what the tensor cores gave.
+template <int BN, bool KN, int TM>
+__device__ __noinline__ void sum_again(const F32Args& g, float* sm, int m0, int n0) {
+  constexpr int kK = 32, kLd = kK + 4, kRows = 16 * TM, kA = kRows * kLd, kBuffer = kA + (KN ? kK * BN : BN * kLd), TN = BN / 32;
+  static_assert(2 * kBuffer * 4 <= 2 * Cfg<BN>::kStage, "in the place of the terms");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t base = smem_u32(sm);
+  auto request = [&](int k0, int buf) {
+    const uint32_t d = base + buf * kBuffer * 4;
+    for (int i = tid; i < kRows * (kK / 4); i += kThreads) {
+      const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4;
+      const bool there = m0 + r < g.M && k < g.K;
+      copy16(d + (r * kLd + i % (kK / 4) * 4) * 4, there ? g.a + (m0 + r) * g.lda + k : g.a, there);
     }
-    float* out = g.c + m * g.scm + n * g.scn;
-    if (g.scn == 1 && n + 4 <= g.N && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-      *reinterpret_cast<float4*>(out) = make_float4(y[0], y[1], y[2], y[3]);
-    } else {
+    for (int i = tid; i < BN * (kK / 4); i += kThreads) {
+      if constexpr (KN) {
+        const int r = i / (BN / 4), n = i % (BN / 4) * 4;
+        const bool there = k0 + r < g.K && n0 + n < g.N;
+        copy16(d + (kA + r * BN + n) * 4, there ? g.b + (k0 + r) * g.ldb + n0 + n : g.b, there);
+      } else {
+        const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4;
+        const bool there = n0 + r < g.N && k < g.K;
+        copy16(d + (kA + r * kLd + i % (kK / 4) * 4) * 4, there ? g.b + (n0 + r) * g.ldb + k : g.b, there);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[TM][TN];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (n + q < g.N) out[q * g.scn] = y[q];
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+  __syncthreads();  // the buffers are free
+  request(0, 0);
+  for (int k0 = 0, buf = 0; k0 < g.K; k0 += kK, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (k0 + kK < g.K) request(k0 + kK, buf ^ 1);
+    const float* as = sm + buf * kBuffer + warp * TM * kLd;
+    const float* bs = sm + buf * kBuffer + kA;
+#pragma unroll 2
+    for (int k = 0; k < kK; k += 4) {
+      float b[TN][4];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        if constexpr (KN) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) b[j][e] = bs[(k + e) * BN + j * 32 + lane];
+        } else {
+          const float4 v = *reinterpret_cast<const float4*>(bs + (j * 32 + lane) * kLd + k);
+          b[j][0] = v.x; b[j][1] = v.y; b[j][2] = v.z; b[j][3] = v.w;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(as + i * kLd + k);
+        const float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[e], b[j][e], acc[i][j]);
+      }
     }
   }
-  __syncwarp();  // what follows stores to the same places
-  for (unsigned lanes = __ballot_sync(0xffffffffu, again != 0); lanes; lanes &= lanes - 1) {
-    const int from = __ffs(lanes) - 1, mm = __shfl_sync(0xffffffffu, m, from), nn = __shfl_sync(0xffffffffu, n, from);
-    for (unsigned cols = __shfl_sync(0xffffffffu, again, from); cols; cols &= cols - 1) {
-      const int c = nn + __ffs(cols) - 1;
-      const float s = plain_dot<KN>(g, mm, c, lane);
-      if (lane == 0) g.c[mm * g.scm + c * g.scn] = s + (g.bias ? g.bias[c] : 0.0f);
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int m = m0 + warp * TM + i, n = n0 + j * 32 + lane;
+      if (m >= g.M || n >= g.N) continue;
+      float* out = g.c + m * g.scm + n * g.scn;
+      if (!isfinite(*out)) *out = acc[i][j] + (g.bias ? g.bias[n] : 0.0f);
     }
-  }
-  __syncwarp();
 }
 
 template <int BN, bool KN>
@@ -140,9 +192,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
   auto acc_full = [&](int s) { return bars + 32u + 8u * s; };
   auto acc_empty = [&](int s) { return bars + 48u + 8u * s; };
   const uint32_t tmem_slot = bars + 64u;
+  // bit i: a result of this CTA's tile number i (modulo the bits) is not finite and its sums are made again
+  __shared__ unsigned again[32], gave_up;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x % g.split, chunk0 = rank * g.per, chunks = min(g.per, (g.K + kBK - 1) / kBK - chunk0);
   const int tile0 = blockIdx.x / g.split, tile_step = gridDim.x / g.split;
+  if (tid < 32) again[tid] = 0;
   if (tid == 0) {
     for (int s = 0; s < 2; ++s) {
       mbar_init(full(s), kSplitWarps);
@@ -246,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
     // Products of chunk number n of this CTA, the largest last: what is cut off is relative to the sum so far.  Narrow tiles are bound by
     // the number of MMAs (one in 90 clocks at best into the same accumulator), so there the terms of B, which lie side by side, are
     // taken two at a time: mid x (hi, mid), lo x hi, hi x lo, hi x (hi, mid) are 16 MMAs instead of 24, into two parts that are
-    // added in the registers (64 x 4096 x 4096: 85 -> 72 us; 128 wide the second part costs more than it saves, 418 -> 449 us
+    // added in the registers (64 x 4096 x 4096, K not split: 85 -> 72 us; 128 wide the second part costs more than it saves, 418 -> 449 us
     // for 2048 x 4096 x 4096).
     const int total = (g.tiles - tile0 + tile_step - 1) / tile_step * chunks;
     auto issue = [&](int n) -> bool {
@@ -276,9 +331,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
     const bool issuer = w == 0 && lane == 0;
     if (issuer && total > 0) issue(0);
     __syncwarp();
-    int it = 0;
+    int it = 0, number = 0;
     bool ok = true;
-    for (int t = tile0; ok && t < g.tiles; t += tile_step) {
+    for (int t = tile0; ok && t < g.tiles; t += tile_step, ++number) {
       f32x2 acc[kCols / 2];
 #pragma unroll
       for (int e = 0; e < kCols / 2; ++e) acc[e] = pack2(0.0f, 0.0f);
@@ -315,11 +370,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
         continue;
       }
       const int tn = t / g.tiles_m, m = (t - tn * g.tiles_m) * kBM + quarter * 32 + lane, n0 = tn * BN + col0;
+      bool bad = false;
 #pragma unroll
       for (int e = 0; e < kCols; e += 4) {
         const float2 x = unpack2(acc[e / 2]), y = unpack2(acc[e / 2 + 1]);
-        store4<KN>(g, m, n0 + e, make_float4(x.x, x.y, y.x, y.y), lane);
+        bad |= store4(g, m, n0 + e, make_float4(x.x, x.y, y.x, y.y));
       }
+      if (bad) atomicOr(&again[(number >> 5) & 31], 1u << (number & 31));
     }
   }
   if (g.split > 1) {
@@ -338,22 +395,36 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tc_kernel(const __grid_c
 #pragma unroll
       for (int q = 1; q < 8; ++q)
         if (q < g.split) x = make_float4(x.x + v[q].x, x.y + v[q].y, x.z + v[q].z, x.w + v[q].w);
-      store4<KN>(g, m0 + r, tn * BN + n, x, lane);
+      if (store4(g, m0 + r, tn * BN + n, x)) atomicOr(&again[0], 1u);
     }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
   __syncwarp();
+  if (tid == 0) gave_up = *reinterpret_cast<volatile int*>(g.err) != 0;
   tc_fence_before();
   __syncthreads();
   if (warp == kSplitWarps) {
-    if (*reinterpret_cast<volatile int*>(g.err) != 0) {
+    if (gave_up) {
       // a wait gave up: let MMAs that are still in flight drain before the memory is released
       const uint64_t t0 = global_timer_ns();
       while (global_timer_ns() - t0 < 2000000ull) __nanosleep(1000);
     }
     tc_fence_after();
     tmem_dealloc(tmem, C::kCols);
+  }
+  if (gave_up) return;
+  // (the barrier above: every result is stored, every MMA and every CTA of the cluster is done with this shared memory)
+  for (int t = tile0, number = 0; t < g.tiles; t += tile_step, ++number) {
+    if (!((again[(number >> 5) & 31] >> (number & 31)) & 1u)) continue;
+    const int tn = t / g.tiles_m, m0 = (t - tn * g.tiles_m) * kBM + rank * (kBM / g.split), n0 = tn * BN;
+    float* sm = reinterpret_cast<float*>(gen);
+    switch (g.split) {
+      case 1: sum_again<BN, KN, 8>(g, sm, m0, n0); break;
+      case 2: sum_again<BN, KN, 4>(g, sm, m0, n0); break;
+      case 4: sum_again<BN, KN, 2>(g, sm, m0, n0); break;
+      default: sum_again<BN, KN, 1>(g, sm, m0, n0); break;
+    }
   }
 }
 

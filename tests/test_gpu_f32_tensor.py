@@ -89,3 +89,53 @@ def test_single_products_over_all_exponents(ops, M, N, K, kn, lo, hi, wlo, whi):
     over = e.abs() >= 2.0 ** 128 * (1 - 2.0 ** -25)
     assert bool(torch.isinf(y)[over].all()) and bool(((y.double() - e).abs() <= b)[~over].all())
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1000, 2048, 2048), (512, 512, 512), (64, 4096, 2048), (40, 300, 4000)])
+@pytest.mark.parametrize("kn", [False, True])
+def test_numbers_out_of_range_cost_a_second_pass_at_most(ops, M, N, K, kn):
+    """Results that overflow, operands full of infinities, sums beyond what tensor memory holds at the split's scale and tiny results: right,
+    and in the time of a few finite products."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    run = (lambda a, b: ops.matmul_forward(a, b)) if kn else (lambda a, b: ops.linear_forward(a, b, None))
+
+    def passes(a, b):
+        b = b.T.contiguous() if kn else b
+        for _ in range(3):
+            y = run(a, b)
+        t = []
+        for _ in range(5):
+            t0, t1 = torch.cuda.Event(True), torch.cuda.Event(True)
+            t0.record()
+            for _ in range(10):
+                run(a, b)
+            t1.record()
+            torch.cuda.synchronize()
+            t.append(t0.elapsed_time(t1))
+        return y, min(t)
+
+    usual = passes(x, w)[1]
+    for a, b in ((x * 1e30, w * 1e6), (x * 1e-30, w * 1e-3), (x * 1e18, w * 1e17)):
+        y, t = passes(a, b)
+        e = a.double() @ b.double().T
+        bound = (48 + K // 64 + 12) * 2.0 ** -24 * (a.double().abs() @ b.double().abs().T) + K * 2.0 ** -149
+        if float(e.abs().max()) > 1e30:  # these are sums of K multiply-adds, any order
+            bound = bound + K * 2.0 ** -24 * (a.double().abs() @ b.double().abs().T)
+        fits = e.abs() < 3e38
+        assert bool(((y.double() - e).abs() <= bound)[fits].all())
+        assert t < 8 * usual + 0.3, (t, usual)
+    a = x.clone()
+    a[:, 5] = float("inf")
+    y, t = passes(a, w)
+    assert bool((y == torch.where(w[:, 5] > 0, float("inf"), -float("inf"))).all())
+    assert t < 8 * usual + 0.3, (t, usual)
+    a[:, 7] = float("nan")
+    assert bool(torch.isnan(passes(a, w)[0]).all())
+    # one bad row leaves the others what they are without it
+    a = x.clone()
+    a[M // 2, 3] = float("inf")
+    y, clean = passes(a, w)[0], passes(x, w)[0]
+    rows = torch.arange(M, device="cuda") != M // 2
+    assert torch.equal(y[rows], clean[rows]) and bool(torch.isinf(y[M // 2]).all())
+    assert ops.device_error() == 0
