@@ -468,8 +468,9 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t
   return v;
 }
 
-// grid (S, tiles, token tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile, blockIdx.z = BN tokens.
-template <int BN, bool W8 = false, bool F8 = false>
+// grid (S, tiles, token tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile, blockIdx.z = BN tokens (TOKEN_TILES;
+// compiled apart, since every decode GEMM would pay for the offsets: 32 x 4096 x 4096 12.2 us with them, 12.05 without).
+template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
 __global__ void __launch_bounds__((SkinnyCfg<BN, W8, F8>::kThreads), 2)
 gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const GemmArgs args) {
@@ -495,7 +496,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   int* err = args.err;
   const uint32_t S = cluster_size(), rank = cluster_rank();
   const int tile = blockIdx.y;
-  const int m0 = blockIdx.z * BN, rows = args.M - m0;  // this CTA's tokens
+  const int m0 = TOKEN_TILES ? blockIdx.z * BN : 0, rows = args.M - m0;  // this CTA's tokens
   bf16* const y = args.y + static_cast<size_t>(m0) * args.ldy;
   const int kb0 = static_cast<int>(rank) * args.kb_per_split;
   const int kb1 = min(args.k_blocks, kb0 + args.kb_per_split);
@@ -539,7 +540,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       // while the previous kernel may still be running; the activation tiles follow once it has finished.  Weights that
       // the kernel in front may be writing (an operator's, a prefill's converted copy) are only asked into L2, where its
       // stores arrive, too.
-      const int ring = min(kb1 - kb0, Cfg::kStages), pre = args.w_early ? ring : 0;
+      const int ring = min(kb1 - kb0, Cfg::kStages), pre = !TOKEN_TILES && args.w_early ? ring : 0;
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), Cfg::kStageBytes);
         tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, full_bar(i), (kb0 + i) * Cfg::kKB, tile * kBM);
@@ -884,13 +885,13 @@ int prepare_variant() {
   return 0;
 }
 
-template <int BN, bool W8 = false, bool F8 = false>
+template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
 int prepare_skinny() {
   static std::atomic<unsigned long long> done{0};  // one bit per device; threads may race to set it
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && (done.load(std::memory_order_acquire) >> dev) & 1ull) return 0;
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_skinny_kernel<BN, W8, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_skinny_kernel<BN, W8, F8, TOKEN_TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        SkinnyCfg<BN, W8, F8>::kSmemBytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
@@ -905,12 +906,12 @@ int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, const GemmArgs&
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int BN, bool W8 = false, bool F8 = false>
+template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
 int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int split, int tiles,
                   cudaStream_t st, int token_tiles = 1) {
-  const int rc = prepare_skinny<BN, W8, F8>();
+  const int rc = prepare_skinny<BN, W8, F8, TOKEN_TILES>();
   if (rc) return rc;
-  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8>, dim3(split, tiles, token_tiles),
+  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8, TOKEN_TILES>, dim3(split, tiles, token_tiles),
                        dim3(SkinnyCfg<BN, W8, F8>::kThreads, 1, 1), SkinnyCfg<BN, W8, F8>::kSmemBytes, st,
                        static_cast<unsigned>(split), tw, tx, a);
 }
@@ -984,7 +985,8 @@ int gemm_bf16_prepare() {
   if ((rc = prepare_skinny<16, true, true>())) return rc;
   if ((rc = prepare_skinny<32, true, true>())) return rc;
   if ((rc = prepare_skinny<64, true, true>())) return rc;
-  return prepare_skinny<128, true, true>();
+  if ((rc = prepare_skinny<128, true, true>())) return rc;
+  return prepare_skinny<128, false, false, true>();
 }
 
 bool gemm_bf16_uses_2cta(int M, int N) {
@@ -1083,8 +1085,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
       // when all its CTAs are resident at once (two per SM) and share HBM evenly -- about 0.85 of the slots -- and a
       // wider cluster than that only adds barrier and reduction cost; with at least as many tiles as SMs no split.
       const int split = large.split ? large.split : skinny_split(tiles, a.k_blocks, sms);
-      const int token_tiles = ceil_div(M, bn);
-      a.w_early = w_early && !large.split;
+      a.w_early = w_early;
       if (large.split) a.l2_ahead = -1;
       a.kb_per_split = ceil_div(a.k_blocks, split);
       {  // what the CTAs ask into L2 ahead of time must stay well inside it (126 MB): at most 48 MB over the grid
@@ -1095,7 +1096,9 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
         case 16: return launch_skinny<16>(tmw, tmx, a, split, tiles, stream);
         case 32: return launch_skinny<32>(tmw, tmx, a, split, tiles, stream);
         case 64: return launch_skinny<64>(tmw, tmx, a, split, tiles, stream);
-        default: return launch_skinny<128>(tmw, tmx, a, split, tiles, stream, token_tiles);
+        default:
+          if (large.split) return launch_skinny<128, false, false, true>(tmw, tmx, a, split, tiles, stream, ceil_div(M, bn));
+          return launch_skinny<128>(tmw, tmx, a, split, tiles, stream);
       }
     }
     a.tiles_p = tiles;
