@@ -1007,7 +1007,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (ldx & 7) || (ldw & 7))
     return TEENY_ERR_ALIGNMENT;
 
-  if (!w_is_kn && !push && gemm_rows_takes(M, N, K, ldw, false, kRowsNormNone)) {
+  if (!w_is_kn && !push && (M <= kRowsStepM || !w_early) && gemm_rows_takes(M, N, K, ldw, false, kRowsNormNone)) {
     RowsGemm g{};
     g.x = x; g.ldx = ldx;
     g.w = w; g.ldw = ldw;

@@ -1,4 +1,4 @@
-// Linear layers of a decode step with few sequences on a small model: y[M, N] = f(x)[M, K] W[N, K]^T, M <= 16.
+// Linear layers of a decode step with few sequences on a small model: y[M, N] = f(x)[M, K] W[N, K]^T, M <= 8 (16 as an operator).
 //
 // What bounds these calls is the way from one kernel to the next, not the bytes: at M = 1 a layer of a 1024-wide model has 31 MB of
 // weights, 5 us at HBM rate, and its seven kernels took 33 us.  So the kernel is built for a short chain:
@@ -10,8 +10,8 @@
 //   * little code: a short rolled loop of mma.m16n8k16 with the tokens as the 16-row A operand and 8 weight rows as B; no tensor
 //     memory, no tensor maps, no cluster reduction.
 // Measured (graph of back-to-back calls, weights from HBM, M = 1, against the 128-row kernel with its cluster reduction): 1024 x 1024
-// 5.0 -> 2.5 us, 1024 x 3072 6.0 -> 3.3, 4096 x 1024 6.3 -> 4.2, 6144 x 1024 7.1 -> 5.0; at M = 16 5.3 -> 4.2, 6.2 -> 6.2, 6.5 -> 5.7,
-// 7.6 -> 6.8.  Decode step of a 28-layer, 1024-wide model at batch 1: 944 -> 663 us; of a 24-layer recurrent hybrid at batch 4 1010 ->
+// 5.5 -> 3.0 us, 1024 x 3072 6.5 -> 4.0, 4096 x 1024 6.5 -> 4.3, 6144 x 1024 7.5 -> 5.2; weights read behind the wait, as an operator
+// does it, 3.0, 4.0, 4.7, 5.5, and at M = 16 5.6 -> 4.6, 6.7 -> 6.7, 6.6 -> 6.5, 7.8 -> 7.3.  Decode step of a 28-layer, 1024-wide model at batch 1: 944 -> 663 us; of a 24-layer recurrent hybrid at batch 4 1010 ->
 // 805.  A first version that kept the weights in registers (16 loads of a thread in flight, loops unrolled to match) took 822 us:
 // its code was five times as long, and every launch fetches it anew.
 // The eight warps of a CTA share the K range (64 k each in turn) and add their sums through shared memory.  Unit = 8 weight rows
@@ -308,7 +308,7 @@ int rows_upc(int N) {
 }  // namespace
 
 bool gemm_rows_takes(int M, int N, int K, int ldw, bool w8, int norm) {
-  if (M < 1 || M > kRowsMaxM || N < 1 || K < 8 || K % (w8 ? 16 : 8) || ldw % (w8 ? 16 : 8)) return false;
+  if (M < 1 || M > (w8 ? kRowsStepM : kRowsMaxM) || N < 1 || K < 8 || K % (w8 ? 16 : 8) || ldw % (w8 ? 16 : 8)) return false;
   // All weights at once in the shared memory of the GPU, half of it left for the kernel behind: about 14 MB.  Beyond that a call
   // lasts long enough for HBM to bound it, and the 128-row kernel's ring streams better (24576 x 4096 at M = 1: 35.9 us there, 46.1 in
   // a variant of this kernel with several passes).
@@ -321,8 +321,7 @@ int gemm_rows_prepare() {
   int rc = 0;
   if ((rc = prepare_rows<1, false, false>()) || (rc = prepare_rows<2, false, false>()) || (rc = prepare_rows<4, false, false>()) ||
       (rc = prepare_rows<1, true, false>()) || (rc = prepare_rows<2, true, false>()) || (rc = prepare_rows<4, true, false>()) ||
-      (rc = prepare_rows<1, false, true>()) || (rc = prepare_rows<2, false, true>()) || (rc = prepare_rows<4, false, true>()) ||
-      (rc = prepare_rows<1, true, true>()) || (rc = prepare_rows<2, true, true>()) || (rc = prepare_rows<4, true, true>()))
+      (rc = prepare_rows<1, false, true>()) || (rc = prepare_rows<2, false, true>()) || (rc = prepare_rows<4, false, true>()))
     return rc;
   return 0;
 }
@@ -338,7 +337,7 @@ int gemm_rows(const RowsGemm& in, cudaStream_t st) {
   int* err = device_error_word();
   if (!err) return TEENY_ERR_DRIVER;
   const int units = (g.N + 7) / 8, upc = rows_upc(g.N);
-  if (two) return w8 ? launch_rows_upc<true, true>(g, upc, units, err, st) : launch_rows_upc<true, false>(g, upc, units, err, st);
+  if (two) return launch_rows_upc<true, false>(g, upc, units, err, st);
   return w8 ? launch_rows_upc<false, true>(g, upc, units, err, st) : launch_rows_upc<false, false>(g, upc, units, err, st);
 }
 

@@ -594,7 +594,7 @@ int norm(teeny_hybrid* m, const float* w, int T, cudaStream_t st) {
 int normed_linear(teeny_hybrid* m, const float* norm_w, const void* w, void* y, int ldy, int T, int N, int glu, const void* bias, cudaStream_t st) {
   const Plan& p = m->p;
   const int d = m->cfg.width;
-  if (!m->cfg.f32 && !m->pending_delta && d % 8 == 0 && !(reinterpret_cast<uintptr_t>(norm_w) & 15) &&
+  if (T <= kRowsStepM && !m->cfg.f32 && !m->pending_delta && d % 8 == 0 && !(reinterpret_cast<uintptr_t>(norm_w) & 15) &&
       gemm_rows_takes(T, N, d, p.width_ld, false, kRowsNormF32)) {
     RowsGemm g = rows_call(m->at<float>(p.x), d, w, p.width_ld, T, N, d, glu, bias);
     g.norm = kRowsNormF32; g.norm_w = norm_w; g.eps = m->cfg.eps;
@@ -610,7 +610,7 @@ int normed_linear(teeny_hybrid* m, const float* norm_w, const void* w, void* y, 
 int sublayer_out(teeny_hybrid* m, const void* x, const void* w, int K, const float* post, bool last, int T, cudaStream_t st) {
   const Plan& p = m->p;
   const int d = m->cfg.width;
-  if (!m->cfg.f32 && !post && !last && gemm_rows_takes(T, d, K, K, false, kRowsNormNone)) {
+  if (T <= kRowsStepM && !m->cfg.f32 && !post && !last && gemm_rows_takes(T, d, K, K, false, kRowsNormNone)) {
     RowsGemm g = rows_call(x, K, w, K, T, d, K, 0, nullptr);
     g.add32 = m->at<float>(p.x); g.ldy = d;
     m->pending_delta = false;

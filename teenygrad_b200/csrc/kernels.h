@@ -95,7 +95,10 @@ int linear_w8a16(const bf16* x, int ldx, const uint8_t* wq, int ldw, const float
 //   out  y [M, N] (+ bias); glu (kGluSilu, kGluGelu; weight rows interleaved in blocks of 64): y [M, N / 2]; add16 / add32: the
 //        rounded product is added into the residual rows there instead (row stride ldy)
 // w: bf16 [N, K], or with w_scale FP8 E4M3 bytes (scale kind 0 or 1, see above; no NaN bytes).
-constexpr int kRowsMaxM = 16;
+// Rows: 8 in a runner's step, and with FP8 weights; 16 as an operator of its own.  Beyond 8 a CTA needs up to 105 KB, so the neighbouring kernels
+// of a step find no place beside it: decode step of a 28-layer, 1024-wide model at 9 and 16 sequences 1167 and 1039 us, through the
+// 128-row kernel 886 and 909 (recurrent hybrid of that width: 977 and 836 at 9; 850 and 872 at 16); 16 x 1024 x 1024 by itself 4.6, there 5.6.
+constexpr int kRowsMaxM = 16, kRowsStepM = 8;
 constexpr int kRowsNormNone = 0, kRowsNormBf16 = 1, kRowsNormF32 = 2;
 struct RowsGemm {
   const void* x;

@@ -490,7 +490,7 @@ bool qkv_fuse_enabled() {
 // Whether a decode step's projection of T rows runs in the kernel for few rows (gemm_rows.cu), with `norm` in front of it.
 // FP8 weights: per-tensor and per-channel scales.
 bool rows_take(const teeny_qwen3* m, const Weight& w, int T, int N, int K, int norm = kRowsNormNone) {
-  return !m->tp && T <= kRowsMaxM && (!w.q || w.kind <= 1) && gemm_rows_takes(T, N, K, K, w.q != nullptr, norm);
+  return !m->tp && T <= kRowsStepM && (!w.q || w.kind <= 1) && gemm_rows_takes(T, N, K, K, w.q != nullptr, norm);
 }
 RowsGemm rows_call(const Weight& w, const void* x, int ldx, int T, int N, int K) {
   RowsGemm g{};
