@@ -53,11 +53,13 @@ unsigned long long teeny_launch_count(int reset);
  * GEMM
  * ------------------------------------------------------------------------------------------------------------- */
 /* C[M,N] = A[M,K] @ B[K,N], all row-major.  Replaces matmul_forward, kernels/teeny-kernels/src/math/gemm.rs:44-108
- * (arguments a_ptr, b_ptr, c_ptr, M, N, K, :52-59).  bf16: f32 accumulate.  f32: f32 accuracy either way -- with
- * global_scratch of at least teeny_matmul_f32_scratch_bytes(M, N, K) bytes (and K, N multiples of 8, 16-byte aligned
- * pointers) on the tensor cores, every operand split into two bf16 terms and three products accumulated in f32 (the
+ * (arguments a_ptr, b_ptr, c_ptr, M, N, K, :52-59).  bf16: f32 accumulate.  f32: with global_scratch NULL the accuracy of f32 FMAs, from
+ * the CUDA cores or, where that is faster (K, N multiples of 4, 16-byte aligned pointers), from the tensor cores with every operand
+ * split into three bf16 terms.  With global_scratch of at least teeny_matmul_f32_scratch_bytes(M, N, K) bytes (and K, N multiples
+ * of 8) large products may also take two bf16 terms per operand and three products accumulated in f32, a few 1e-6 (the
  * split the reference's DSL calls TF32x3, kernels/teeny-triton/src/triton/mod.rs:76-83; its kernel uses one TF32 pass,
- * math/gemm.rs:95, which the 1e-4 bar rules out); with global_scratch NULL by f32 FMAs on the CUDA cores. */
+ * math/gemm.rs:95, which the 1e-4 bar rules out).
+ * Operands of all operators of this header may have been written by the call just before, weights included. */
 int matmul_forward_entry_point_f32(const float* a, const float* b, float* c, int M, int N, int K,
                                    void* global_scratch, size_t global_scratch_bytes, teeny_stream_t stream);
 int matmul_forward_entry_point_bf16(const teeny_bf16* a, const teeny_bf16* b, teeny_bf16* c, int M, int N, int K,

@@ -202,7 +202,8 @@ constexpr Choice kChoices[] = {{128, 128, 1, 92.0, 3500.0}, {64, 64, 2, 75.0, 20
 
 // The tile that is estimated to end first: rounds of tiles over the SMs at the tile's rate, or the chain of slices if that is longer.
 // 1000 x 4096 x 1024: 128 x 128 at 199 us (64 x 64: 210); 512^3: 32 x 64 at 16.5 us (64 x 64: 23, 16 x 32: 23).  The one 64 x 64 tile
-// with 4 x 4 sums per thread that served every size before took 308 us and 50 us.
+// with 4 x 4 sums per thread that served every size before took 308 us and 50 us.  (Call by call, as in the table above; back to back in a
+// graph a call takes 2.4 us less: 14.1 for 512^3.)
 int choose(long long M, long long N, long long K, int sms, double& least) {
   int best = 0;
   least = 0.0;
@@ -262,7 +263,8 @@ double gemm_f32_clocks(const float* a, long long sam, long long sak, const float
 int gemm_f32(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn,
              const float* bias, float* c, long long scm, long long scn, int M, int N, int K, cudaStream_t stream) {
   // On the tensor cores where that is estimated to end first, and always with a smaller error: from about 1 M multiply-adds per
-  // SM on.  64 x 512 x 512: 6.8 us here, 7.7 there; 17 x 1000 x 1000: 10.9, 10.2; 512^3: 14.1, 9.8; 64 x 4096 x 4096: 93, 36.
+  // SM on.  Back to back, [N][K]: 64 x 512 x 512 6.8 us here, 8.0 there; 17 x 1000 x 1000 11.1, 12.0; 512^3 14.1, 9.6; 64 x 4096 x 4096 93,
+  // 39.6; 300 x 700 x 2000 45.7, 17.0; 1000 x 2048 x 2048 236, 66.6.
   if (a && b && c && gemm_f32_tc_takes(a, sam, sak, b, sbk, sbn, M, N, K)) {
     double here;
     choose(M, N, K, sm_count(), here);

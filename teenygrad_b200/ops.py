@@ -50,8 +50,8 @@ def gemm_scratch(M, N, K, device="cuda"):
 
 
 def matmul_f32_scratch(M, N, K, device="cuda"):
-    """Scratch that sends the f32 matmul to the tensor cores (operands split into bf16 terms); without it the f32
-    entry point runs on the CUDA cores."""
+    """Scratch with which large f32 matmuls may take two bf16 terms per operand on the tensor cores (a few 1e-6); without it
+    every f32 product has the accuracy of f32 multiply-adds."""
     return torch.empty(lib.teeny_matmul_f32_scratch_bytes(M, N, K), dtype=torch.uint8, device=device)
 
 
