@@ -286,7 +286,7 @@ int rms_norm_forward_entry_point_f32(const float* x, float* y, const float* w, f
 }
 int rms_norm_forward_entry_point_bf16(const teeny_bf16* x, teeny_bf16* y, const teeny_bf16* w, float* rrms, int M,
                                       int N, float eps, teeny_stream_t stream) {
-  return rms_norm_bf16(B(x), N, B(y), N, B(w), rrms, M, N, eps, S(stream));
+  return rms_norm_bf16(B(x), N, B(y), N, B(w), rrms, M, N, eps, S(stream), nullptr, 0, nullptr, /*w_early=*/false);
 }
 int silu_forward_entry_point_f32(const float* x, float* y, int n, teeny_stream_t s) { return silu_f32(x, y, n, S(s)); }
 int silu_forward_entry_point_bf16(const teeny_bf16* x, teeny_bf16* y, int n, teeny_stream_t s) { return silu_bf16(B(x), B(y), n, S(s)); }
@@ -299,7 +299,7 @@ int softmax_forward_entry_point_bf16(const teeny_bf16* x, teeny_bf16* y, int r, 
 
 int teeny_add_rms_norm_bf16(const teeny_bf16* x, teeny_bf16* residual, teeny_bf16* y, const teeny_bf16* w, int M, int N,
                             float eps, teeny_stream_t s) {
-  return add_rms_norm_bf16(B(x), N, B(residual), N, B(y), N, B(w), M, N, eps, S(s));
+  return add_rms_norm_bf16(B(x), N, B(residual), N, B(y), N, B(w), M, N, eps, S(s), nullptr, 0, nullptr, /*w_early=*/false);
 }
 int teeny_silu_mul_bf16(const teeny_bf16* gate_up, long long ld, teeny_bf16* out, int T, int inter, teeny_stream_t s) {
   return silu_mul_bf16(B(gate_up), ld, B(out), T, inter, S(s));
@@ -351,7 +351,7 @@ int teeny_qk_norm_rope_kv_bf16(teeny_bf16* qkv, long long ld, const teeny_bf16* 
                                int Hq, int Hkv, int D, int max_len, int pos0, const int* pos0_dev, float eps,
                                teeny_stream_t s) {
   return qk_norm_rope_kv_bf16(B(qkv), ld, B(qw), B(kw), B(c), B(sn), B(kc), B(vc), T, Sx, Hq, Hkv, D, max_len, pos0,
-                              pos0_dev, eps, S(s));
+                              pos0_dev, eps, S(s), /*w_early=*/false);
 }
 int teeny_embedding_bf16(const int* ids, const teeny_bf16* table, teeny_bf16* out, int T, int hidden, int vocab,
                          teeny_stream_t s) {

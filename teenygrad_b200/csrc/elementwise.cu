@@ -143,8 +143,9 @@ template <int VPT, bool ADD>
 __global__ void rms_norm_bf16_kernel(const bf16* __restrict__ x, long long ldx, bf16* __restrict__ res,
                                      long long ldr, bf16* __restrict__ y, long long ldy, const bf16* __restrict__ w,
                                      float* __restrict__ rrms, int N, float eps, uint8_t* __restrict__ y8 = nullptr,
-                                     long long ld8 = 0, float* __restrict__ y8_scale = nullptr) {
-  // the norm weights are written by no kernel: fetch them while the producer of x is still running, and let the
+                                     long long ld8 = 0, float* __restrict__ y8_scale = nullptr, bool w_early = true) {
+  if (!w_early) pdl_wait();
+  // a model's norm weights are written by no kernel of its steps: fetch them while the producer of x is still running, and let the
   // consumer of y become resident (and fetch its own weights) as soon as this kernel's input is complete
   const int nv = N >> 3;
   const uint4* wr = reinterpret_cast<const uint4*>(w);
@@ -276,7 +277,7 @@ __global__ void rms_norm_bf16_scalar_kernel(const bf16* __restrict__ x, long lon
 
 template <bool ADD>
 int launch_rms_bf16(const bf16* x, long long ldx, bf16* res, long long ldr, bf16* y, long long ldy, const bf16* w, float* rrms,
-                    int M, int N, float eps, cudaStream_t st, uint8_t* y8 = nullptr, long long ld8 = 0, float* y8_scale = nullptr) {
+                    int M, int N, float eps, cudaStream_t st, uint8_t* y8, long long ld8, float* y8_scale, bool w_early) {
   if (!x || !y || !w || (ADD && !res) || M < 0 || N <= 0) return TEENY_ERR_BAD_ARG;
   if (y8 && (!y8_scale || (ld8 & 7) || ld8 < N || (reinterpret_cast<uintptr_t>(y8) & 7))) return TEENY_ERR_BAD_ARG;
   if (M == 0) return TEENY_OK;
@@ -293,7 +294,7 @@ int launch_rms_bf16(const bf16* x, long long ldx, bf16* res, long long ldr, bf16
     const int vpt = (nv + threads - 1) / threads;
 #define TEENY_RMS_CASE(V)                                                                                    \
   launch_kernel(rms_norm_bf16_kernel<V, ADD>, dim3(M), dim3(threads), 0, st, 1, x, ldx, res, ldr, y, ldy, w, rrms, N, eps, y8, \
-                ld8, y8_scale)
+                ld8, y8_scale, w_early)
     if (vpt <= 1) TEENY_RMS_CASE(1);
     else if (vpt <= 2) TEENY_RMS_CASE(2);
     else if (vpt <= 4) TEENY_RMS_CASE(4);
@@ -662,13 +663,14 @@ __global__ void qk_norm_rope_kv_kernel(bf16* __restrict__ qkv, long long ld, con
                                        const bf16* __restrict__ k_w, const bf16* __restrict__ cos_t,
                                        const bf16* __restrict__ sin_t, bf16* __restrict__ k_cache,
                                        bf16* __restrict__ v_cache, int T, int S, int Hq, int Hkv, int max_len,
-                                       int pos0, const int* __restrict__ pos0_dev, float eps) {
+                                       int pos0, const int* __restrict__ pos0_dev, float eps, bool w_early) {
   constexpr int D = 128;
   const int heads = Hq + 2 * Hkv;
   const long long total = static_cast<long long>(T) * heads;
   const long long unit0 = ((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4) * kRopeUnits;
   const int sub = threadIdx.x & 15;
-  // head-norm weights are constants: fetched ahead of the wait for the projection
+  // a model's head-norm weights are fetched ahead of the wait for the projection
+  if (!w_early) pdl_wait();
   const uint4 wq = __ldg(reinterpret_cast<const uint4*>(q_w + sub * 8));
   const uint4 wk = __ldg(reinterpret_cast<const uint4*>(k_w + sub * 8));
   pdl_wait();
@@ -1004,12 +1006,12 @@ int rms_norm_f32(const float* x, float* y, const float* w, float* rrms, int M, i
   return static_cast<int>(cudaGetLastError());
 }
 int rms_norm_bf16(const bf16* x, long long ldx, bf16* y, long long ldy, const bf16* w, float* rrms, int M, int N,
-                  float eps, cudaStream_t st, uint8_t* y8, long long ld8, float* y8_scale) {
-  return launch_rms_bf16<false>(x, ldx, nullptr, 0, y, ldy, w, rrms, M, N, eps, st, y8, ld8, y8_scale);
+                  float eps, cudaStream_t st, uint8_t* y8, long long ld8, float* y8_scale, bool w_early) {
+  return launch_rms_bf16<false>(x, ldx, nullptr, 0, y, ldy, w, rrms, M, N, eps, st, y8, ld8, y8_scale, w_early);
 }
 int add_rms_norm_bf16(const bf16* x, long long ldx, bf16* residual, long long ldr, bf16* y, long long ldy,
-                      const bf16* w, int M, int N, float eps, cudaStream_t st, uint8_t* y8, long long ld8, float* y8_scale) {
-  return launch_rms_bf16<true>(x, ldx, residual, ldr, y, ldy, w, nullptr, M, N, eps, st, y8, ld8, y8_scale);
+                      const bf16* w, int M, int N, float eps, cudaStream_t st, uint8_t* y8, long long ld8, float* y8_scale, bool w_early) {
+  return launch_rms_bf16<true>(x, ldx, residual, ldr, y, ldy, w, nullptr, M, N, eps, st, y8, ld8, y8_scale, w_early);
 }
 int gather_add_rms_norm_bf16(const uint2* recv, size_t slot_elems, int world, const unsigned* epoch, unsigned round,
                              bf16* residual, long long ldr, bf16* y, long long ldy, const bf16* w, int M, int N,
@@ -1101,7 +1103,7 @@ int rope_table_bf16(const float* inv_freq, bf16* cos_t, bf16* sin_t, int max_pos
 
 int qk_norm_rope_kv_bf16(bf16* qkv, long long ld, const bf16* q_w, const bf16* k_w, const bf16* cos_t,
                          const bf16* sin_t, bf16* k_cache, bf16* v_cache, int T, int S, int Hq, int Hkv, int D,
-                         int max_len, int pos0, const int* pos0_dev, float eps, cudaStream_t st) {
+                         int max_len, int pos0, const int* pos0_dev, float eps, cudaStream_t st, bool w_early) {
   if (!qkv || !q_w || !k_w || !cos_t || !sin_t || !k_cache || !v_cache || T < 0 || S <= 0 || Hq <= 0 || Hkv <= 0 ||
       max_len <= 0)
     return TEENY_ERR_BAD_ARG;
@@ -1115,7 +1117,7 @@ int qk_norm_rope_kv_bf16(bf16* qkv, long long ld, const bf16* q_w, const bf16* k
   const long long blocks = (units + 16 * kRopeUnits - 1) / (16 * kRopeUnits);
   if (blocks > 0x7fffffffLL) return TEENY_ERR_BAD_ARG;
   launch_kernel(qk_norm_rope_kv_kernel, dim3(static_cast<int>(blocks)), dim3(256), 0, st, 1, qkv, ld, q_w, k_w, cos_t, sin_t, k_cache, v_cache,
-                                                                   T, S, Hq, Hkv, max_len, pos0, pos0_dev, eps);
+                                                                   T, S, Hq, Hkv, max_len, pos0, pos0_dev, eps, w_early);
   return static_cast<int>(cudaGetLastError());
 }
 

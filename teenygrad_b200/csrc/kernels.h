@@ -240,11 +240,12 @@ int rms_norm_f32(const float* x, float* y, const float* w, float* rrms, int M, i
 // y8 != null: y is also written as two-term FP8 activations (hi rows, then M lo rows; row stride ld8 bytes;
 // y8_scale[M]), as split_e4m3 would split it.
 int rms_norm_bf16(const bf16* x, long long ldx, bf16* y, long long ldy, const bf16* w, float* rrms, int M, int N,
-                  float eps, cudaStream_t st, uint8_t* y8 = nullptr, long long ld8 = 0, float* y8_scale = nullptr);
+                  float eps, cudaStream_t st, uint8_t* y8 = nullptr, long long ld8 = 0, float* y8_scale = nullptr, bool w_early = true);
+// (w_early here and below: see gemm_bf16, of the norms' weights; the public operators pass false)
 // residual <- bf16(residual + x); y <- rms_norm(residual) (same rounding as rms_norm_bf16).
 int add_rms_norm_bf16(const bf16* x, long long ldx, bf16* residual, long long ldr, bf16* y, long long ldy,
                       const bf16* w, int M, int N, float eps, cudaStream_t st, uint8_t* y8 = nullptr, long long ld8 = 0,
-                      float* y8_scale = nullptr);
+                      float* y8_scale = nullptr, bool w_early = true);
 int silu_f32(const float* x, float* y, long long n, cudaStream_t st);
 int silu_bf16(const bf16* x, bf16* y, long long n, cudaStream_t st);
 int mul_f32(const float* a, const float* b, float* o, long long n, cudaStream_t st);
@@ -264,7 +265,7 @@ int rope_table_bf16(const float* inv_freq, bf16* cos_t, bf16* sin_t, int max_pos
 //   to the caches laid out [B, Hkv, max_len, D].
 int qk_norm_rope_kv_bf16(bf16* qkv, long long ld, const bf16* q_w, const bf16* k_w, const bf16* cos_t,
                          const bf16* sin_t, bf16* k_cache, bf16* v_cache, int T, int S, int Hq, int Hkv, int D,
-                         int max_len, int pos0, const int* pos0_dev, float eps, cudaStream_t st);
+                         int max_len, int pos0, const int* pos0_dev, float eps, cudaStream_t st, bool w_early = true);
 // Row argmax with lowest index on ties; writes value (f32) and index + idx_offset.
 int argmax_bf16(const bf16* logits, long long ld, float* best_val, int* best_idx, int rows, int cols, int idx_offset,
                 cudaStream_t st);

@@ -219,3 +219,32 @@ def test_cached_rows_written_just_before(cached, cap):
         ops.rope_cache(qs, *src[i % 3], kc, vc, freq, D, whole, cached)
     _chain(write, lambda: ops.cached_attention(q, kc, vc, D ** -0.5, last, out=y, scratch=scratch), torch.equal)
     assert ops.device_error() == 0
+
+
+def test_bf16_norm_weights_just_before():
+    """The weights of the bf16 norms and of the head norms, from a norm in front whose rows they are."""
+    from teenygrad_b200 import ops
+    rows, n, H, G = 600, 2048, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(9)
+    src = [torch.randn(rows, n, generator=g, device="cuda").bfloat16() for _ in range(3)]
+    x = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    w, zero, one = (torch.zeros(rows, n, device="cuda").bfloat16() for _ in range(3))
+    one += 1
+    qkv0 = torch.randn(8, (H + 2 * G) * 128, generator=g, device="cuda").bfloat16()
+    cos, sin = ops.rope_table(1.0 / 1e4 ** (torch.arange(64, device="cuda").float() / 64), 16)
+    kc, vc = (torch.zeros(1, G, 16, 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    qkv, res = qkv0.clone(), zero.clone()
+
+    def write(i):
+        w.copy_(src[i % 3])
+        qkv.copy_(qkv0)
+        res.copy_(zero)
+        ops.add_rms_norm(zero, w, one[0], 1e-6)  # w <- w + 0, by the kernel that lets the next one in before it stores
+
+    def heads():
+        ops.qk_norm_rope_kv(qkv, w[rows - 1, :128], w[rows - 1, 128:256], cos, sin, kc, vc, 8, H, G, 0, 1e-6)
+        return torch.cat([qkv[:, :H * 128].flatten(), kc.flatten()])
+    _chain(write, lambda: ops.rms_norm_forward(x, w[rows - 1], 1e-6), torch.equal)
+    _chain(write, lambda: ops.add_rms_norm(x, res, w[rows - 1], 1e-6), torch.equal)
+    _chain(write, heads, torch.equal)
+    assert ops.device_error() == 0
