@@ -940,24 +940,34 @@ int swap_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128))
 //   800 x 4096 x 4096 40.0 / 30.9 / 28.6 / 41.6     300 x 12288 x 1024 16.3 / 16.6 / 22.1 / 24.6     512 x 1024 x 3072 17.4 / 21.0 / 21.4 / 11.7
 //   200 x 4096 x 12288 54.5 / 75.3 / 62.7 / 32.5    4500 x 1024 x 3072 33.3 / 24.5 / 24.3 / -        200 x 520 x 8192 39.3 / 46.4 / 46.8 / 12.5
 // (By tile counts alone, wide tiles only with one for every SM and no K split, these took 40.7, 22.0, 17.4, 54.4, 33.1 and 41.7.)
+// An estimate is good to a few per cent: what the tile counts alone would take stays unless another kernel is estimated to be 3.5 % faster (700 x
+// 1024 x 1024: narrow 9.2 us, K over three CTAs 10.5, estimated 9.5 and 9.2; 1500 x 4096 x 1024: pairs 18.4, narrow 19.4, estimated 18.5 and
+// 18.4).  Of 541 sizes with 129 to 4500 tokens none is then more than 3 % slower than by tile counts; 5 % would do as well, at 7 % fifteen lose.
 enum { kLargeNone, kLargeNarrow, kLargeWide, kLargePair, kLargeSplit };
 struct LargeChoice { int kind, split; };
 LargeChoice choose_large(int M, int N, int k_blocks, int sms) {
   auto rounds = [](long long tiles, long long slots) { return static_cast<double>((tiles + slots - 1) / slots); };
-  const long long m128 = ceil_div(M, 128), n128 = ceil_div(N, 128), n256 = ceil_div(N, 256);
-  LargeChoice best{kLargeNarrow, 0};
-  double least = 5.0 + rounds(m128 * n128, sms) * k_blocks * 0.28;
+  const long long m128 = ceil_div(M, 128), n128 = ceil_div(N, 128), n256 = ceil_div(N, 256), pairs = static_cast<long long>(ceil_div(M, 256)) * n256;
+  const double narrow = 5.0 + rounds(m128 * n128, sms) * k_blocks * 0.28;
   const double wide = 8.0 + rounds(m128 * n256, sms) * k_blocks * 0.385;
-  if (N > 128 && wide < least) { best.kind = kLargeWide; least = wide; }
-  const double pair = 7.5 + rounds(static_cast<long long>(ceil_div(M, 256)) * n256, sms / 2) * k_blocks * 0.345;
-  if (pair < least) { best.kind = kLargePair; least = pair; }
+  const double pair = 7.5 + rounds(pairs, sms / 2) * k_blocks * 0.345;
+  LargeChoice best{kLargeNarrow, 0};
+  double least = narrow;
+  if (pairs >= sms / 2) { best.kind = kLargePair; least = pair; }
+  else if (N > 128 && m128 * n256 >= sms) { best.kind = kLargeWide; least = wide; }
+  least *= 0.965;
+  auto consider = [&](int kind, int split, double t) {
+    if (t < least) { best = LargeChoice{kind, split}; least = t; }
+  };
+  consider(kLargeNarrow, 0, narrow);
+  if (N > 128) consider(kLargeWide, 0, wide);
+  consider(kLargePair, 0, pair);
   for (int split = 2; split <= 8; ++split) {
     const int per = ceil_div(k_blocks, split);
     // all of them resident, two on an SM; clusters do not find place on every SM (300 x 4096 x 4096 in 288 CTAs: 30.5 us, in 192: 22.7)
     const long long ctas = m128 * n128 * split;
     if (ctas * 100 > 2LL * sms * 87 || per < 4 || per * (split - 1) >= k_blocks || n128 > 65535) continue;
-    const double t = ctas <= sms ? 6.5 + per * 0.45 : 9.0 + per * 0.47;
-    if (t < least) { best = LargeChoice{kLargeSplit, split}; least = t; }
+    consider(kLargeSplit, split, ctas <= sms ? 6.5 + per * 0.45 : 9.0 + per * 0.47);
   }
   return best;
 }
