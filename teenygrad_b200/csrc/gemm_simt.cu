@@ -204,16 +204,18 @@ constexpr Choice kChoices[] = {{128, 128, 1, 92.0, 3500.0}, {64, 64, 2, 75.0, 20
 // 1000 x 4096 x 1024: 128 x 128 at 199 us (64 x 64: 210); 512^3: 32 x 64 at 16.5 us (64 x 64: 23, 16 x 32: 23).  The one 64 x 64 tile
 // with 4 x 4 sums per thread that served every size before took 308 us and 50 us.  (Call by call, as in the table above; back to back in a
 // graph a call takes 2.4 us less: 14.1 for 512^3.)
-int choose(long long M, long long N, long long K, int sms, double& least) {
-  int best = 0;
+// bf16 takes the three smaller ones (`first` = 1): its operands come two bytes at a time where they are not aligned, which 256 threads an SM that
+// hold 128 sums each do not keep up with (1000 x 4096 x 1024, odd rows: 368 us with 128 x 128, 281 with 64 x 64; f32 216 and 242).
+int choose(long long M, long long N, long long K, int sms, double& least, int first = 0) {
+  int best = first;
   least = 0.0;
-  for (int i = 0; i < 4; ++i) {
+  for (int i = first; i < 4; ++i) {
     const Choice& x = kChoices[i];
     const long long tiles = ((M + x.bm - 1) / x.bm) * ((N + x.bn - 1) / x.bn);
     const double pipe = static_cast<double>((tiles + sms - 1) / sms) * x.bm * x.bn * K / x.rate;
     const double chain = static_cast<double>((K + kTK * x.kg - 1) / (kTK * x.kg)) * x.slice;
     const double t = pipe > chain ? pipe : chain;
-    if (i == 0 || t < least) { least = t; best = i; }
+    if (i == first || t < least) { least = t; best = i; }
   }
   return best;
 }
@@ -234,14 +236,16 @@ int launch(const T* a, long long sam, long long sak, const T* b, long long sbk, 
   if ((static_cast<long long>(M) + 63) / 64 > 65535) return TEENY_ERR_BAD_ARG;
   const Operand<T> oa = operand(a, sam, sak, M, K), ob = operand(b, sbn, sbk, N, K);
   double clocks;
-  const Choice x = kChoices[choose(M, N, K, sm_count(), clocks)];
+  const Choice x = kChoices[choose(M, N, K, sm_count(), clocks, sizeof(T) == 2 ? 1 : 0)];
   const long long tiles_n = (static_cast<long long>(N) + x.bn - 1) / x.bn, tiles = (static_cast<long long>(M) + x.bm - 1) / x.bm * tiles_n;
   if (tiles > 0x7fffffffLL) return TEENY_ERR_BAD_ARG;
 #define TEENY_SIMT(BM, BN, TM, TN, KG)                                                                                              \
   launch_kernel(gemm_simt_kernel<T, BM, BN, TM, TN, KG>, dim3(static_cast<unsigned>(tiles)), dim3(Tile<BM, BN, TM, TN, KG>::kThreads), \
                 0, st, 1, oa, ob, bias, c, scm, scn, K, static_cast<int>(tiles_n))
   switch (x.bm) {
-    case 128: TEENY_SIMT(128, 128, 16, 8, 1); break;
+    case 128:
+      if constexpr (sizeof(T) == 4) TEENY_SIMT(128, 128, 16, 8, 1);
+      break;
     case 64: TEENY_SIMT(64, 64, 8, 4, 2); break;
     case 32: TEENY_SIMT(32, 64, 4, 4, 3); break;
     default: TEENY_SIMT(16, 32, 2, 4, 6); break;
