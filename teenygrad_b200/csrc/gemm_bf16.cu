@@ -942,7 +942,7 @@ int swap_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128))
 // (By tile counts alone, wide tiles only with one for every SM and no K split, these took 40.7, 22.0, 17.4, 54.4, 33.1 and 41.7.)
 // An estimate is good to a few per cent: what the tile counts alone would take stays unless another kernel is estimated to be 3.5 % faster (700 x
 // 1024 x 1024: narrow 9.2 us, K over three CTAs 10.5, estimated 9.5 and 9.2; 1500 x 4096 x 1024: pairs 18.4, narrow 19.4, estimated 18.5 and
-// 18.4).  Of 541 sizes with 129 to 4500 tokens none is then more than 3 % slower than by tile counts; 5 % would do as well, at 7 % fifteen lose.
+// 18.4).  Of 541 sizes with 129 to 4500 tokens two are then 3 and 6 % slower than by tile counts, instead of nine by 4 to 18 %.
 enum { kLargeNone, kLargeNarrow, kLargeWide, kLargePair, kLargeSplit };
 struct LargeChoice { int kind, split; };
 LargeChoice choose_large(int M, int N, int k_blocks, int sms) {
