@@ -233,6 +233,13 @@ int attention_decode_bf16_static(const bf16* q, const bf16* k, const bf16* v, bf
                                  const int* kv_len_dev, cudaStream_t stream);
 template <typename T>
 int attention_generic(const T* q, const T* k, const T* v, T* o, float* lse, const AttnShape& s, cudaStream_t stream);
+// The same on the tensor cores (attention_f32_tc.cu), for operands that attention_f32_tc_takes.
+template <typename T>
+bool attention_f32_tc_takes(const T* q, const T* k, const T* v, const AttnShape& s);
+double attention_f32_tc_us(bool f32, const AttnShape& s);  // estimated time
+inline double attention_mean_keys(const AttnShape& s) { return s.causal ? s.Skv - 0.5 * (s.Sq - 1) : s.Skv; }  // of a query
+template <typename T>
+int attention_f32_tc(const T* q, const T* k, const T* v, T* o, float* lse, const AttnShape& s, cudaStream_t stream);
 
 // ---- normalisation / elementwise ----------------------------------------------------------------
 int rms_norm_f32(const float* x, float* y, const float* w, float* rrms, int M, int N, float eps, cudaStream_t st);
