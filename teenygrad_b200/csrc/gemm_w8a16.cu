@@ -65,6 +65,44 @@ dequant_e4m3_bf16_kernel(const uint8_t* __restrict__ wq, long long ldw, const fl
   }
 }
 
+// The same for rows of whole 8-byte pieces, one scale a piece (kind 2: groups of a multiple of 8).  Bound: HBM, 3 bytes per weight.  A thread
+// converts one 8-byte piece of each of four rows, with the four loads in flight together, and stores 16 bytes of each: neighbouring lanes
+// read and write neighbouring pieces, and no piece number is divided.  24576 x 4096: 142 us with the kernel above (two 64-bit divisions and
+// 16 shift-and-mask conversions per 16 bytes), 49 us here (6.2 TB/s).
+constexpr int kDequantRows = 4;
+__global__ void __launch_bounds__(256)
+dequant_e4m3_bf16_vec_kernel(const uint8_t* __restrict__ wq, long long ldw, const float* __restrict__ scale, int kind, int group,
+                             bf16* __restrict__ out, long long ldo, int N, int K) {
+  pdl_wait();
+  pdl_trigger();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, k0 = c * 8;
+  if (k0 >= K) return;
+  const int groups_per_row = kind == 2 ? (K + group - 1) / group : 0, g = kind == 2 ? k0 / group : 0;
+  for (int n0 = blockIdx.y * kDequantRows; n0 < N; n0 += gridDim.y * kDequantRows) {
+    uint2 w[kDequantRows];
+    float s[kDequantRows];
+#pragma unroll
+    for (int i = 0; i < kDequantRows; ++i) {
+      const int n = min(n0 + i, N - 1);
+      w[i] = __ldg(reinterpret_cast<const uint2*>(wq + n * ldw + k0));
+      s[i] = __ldg(scale + (kind == 0 ? 0 : (kind == 1 ? static_cast<size_t>(n) : static_cast<size_t>(n) * groups_per_row + g)));
+    }
+#pragma unroll
+    for (int i = 0; i < kDequantRows; ++i) {
+      if (n0 + i >= N) break;
+      const uint32_t words[2] = {w[i].x, w[i].y};
+      uint32_t o[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(words[q >> 1] >> (16 * (q & 1))), __NV_E4M3);
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h));
+        o[q] = pack_bf16x2(v.x * s[i], v.y * s[i]);
+      }
+      *reinterpret_cast<uint4*>(out + (n0 + i) * ldo + k0) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
 // Integer schemes (utilities/teeny-quant/src/quant/affine.rs:151-161): value = (q - zero point) * scale, q an int8 or a
 // sign-extended nibble (two per byte over the flattened tensor, the first in the low nibble, pack4.rs:31-40).  One
 // thread per 8 consecutive k of a row.
@@ -196,6 +234,11 @@ int dequant_e4m3_bf16(const uint8_t* wq, long long ldw, const float* scale, int 
   if (!wq || !scale || !out || N <= 0 || K <= 0 || kind < 0 || kind > 2 || (kind == 2 && group <= 0)) return TEENY_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(wq) & 15) || (ldw & 15) || (reinterpret_cast<uintptr_t>(out) & 15) || (ldo & 7))
     return TEENY_ERR_ALIGNMENT;
+  if (K % 8 == 0 && (kind != 2 || group % 8 == 0)) {
+    const int rows = (N + kDequantRows - 1) / kDequantRows;
+    return launch_kernel(dequant_e4m3_bf16_vec_kernel, dim3((K / 8 + 255) / 256, rows < 65535 ? rows : 65535), dim3(256), 0, st, 1, wq, ldw, scale, kind,
+                         group, out, ldo, N, K);
+  }
   const long long total = static_cast<long long>(N) * ((K + 15) / 16);
   const long long want = (total + 255) / 256;
   const int grid = static_cast<int>(want < 148 * 16 ? want : 148 * 16);

@@ -311,3 +311,19 @@ def test_linear_w8a8x2_swiglu_and_bias(ops):
     b = (torch.arange(I).float() * 0.01).bfloat16()
     yb = ops.linear_w8a8x2(x8, xs, torch.from_numpy(qg).cuda(), torch.from_numpy(sg).cuda(), "channel", bias=b.cuda())
     assert rel(yb, oq.linear_w8a16(x.float().numpy(), qg, sg, "channel", axis=0, bias=b.float().numpy())) < BF16_TOL
+
+
+@pytest.mark.parametrize("N,K", [(1, 8), (3, 2040), (4, 2048), (5, 2056), (9, 520), (1030, 64), (2, 20)])
+@pytest.mark.parametrize("strategy,group_size", [("tensor", 0), ("channel", 0), ("group", 8), ("group", 40), ("group", 12)])
+def test_dequant_rows_and_pieces(ops, N, K, strategy, group_size):
+    """Row counts around the four rows of a thread, rows around a block's 2048 bytes and not of whole pieces, groups of whole pieces and others."""
+    g = torch.Generator().manual_seed(N + K)
+    wide = torch.randint(0, 256, (N, (K + 31) // 16 * 16), generator=g, dtype=torch.uint8)
+    wide[(wide & 0x7f) == 0x7f] = 0x7e
+    groups = -(-K // group_size) if group_size else 1
+    s = torch.rand((N, groups) if group_size else ((N,) if strategy == "channel" else (1,)), generator=g) + 0.1
+    value = wide[:, :K].view(torch.float8_e4m3fn).float()
+    scale = s.repeat_interleave(group_size, 1)[:, :K] if group_size else (s[:, None] if strategy == "channel" else s)
+    out = torch.full((N, (K + 15) // 8 * 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.dequant_fp8(wide.cuda()[:, :K], s.flatten().cuda(), strategy, group_size, out=out[:, :K])
+    assert torch.equal(out[:, :K].cpu(), (value * scale).bfloat16()) and bool((out[:, K:] == 7.0).all())
