@@ -14,12 +14,18 @@ from ._lib import lib, check, AttnShape
 _BF16, _F32 = torch.bfloat16, torch.float32
 
 
+# An operator on small tensors is bound by its host side: of 13.4 us a call, the objects behind torch.cuda.current_stream() and ctypes'
+# pointer wrappers were 4.  The raw handle and plain integers say the same.
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of torch's current stream on the current device."""
+    return _raw_stream(_current_device())
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _req(t, dtype=None, name="tensor"):
@@ -36,6 +42,19 @@ def _sfx(t):
     if t.dtype == _BF16:
         return "bf16"
     raise ValueError(f"unsupported dtype {t.dtype}")
+
+
+def _entry(name):
+    """``t -> C entry point of t's type``."""
+    of = {d: getattr(lib, f"{name}_forward_entry_point_{n}") for d, n in ((_F32, "f32"), (_BF16, "bf16"))}
+
+    def get(t):
+        fn = of.get(t.dtype)
+        return fn if fn is not None else _sfx(t)  # (which raises)
+    return get
+
+
+_matmul, _linear, _attention2 = _entry("matmul"), _entry("linear"), _entry("flash_attention2")
 
 
 def device_error(clear=True):
@@ -62,7 +81,7 @@ def matmul_forward(a, b, out=None, scratch=None):
     M, K = a.shape
     N = b.shape[1]
     out = torch.empty(M, N, dtype=a.dtype, device=a.device) if out is None else out
-    fn = getattr(lib, f"matmul_forward_entry_point_{_sfx(a)}")
+    fn = _matmul(a)
     check(fn(_ptr(a), _ptr(b), _ptr(out), M, N, K, _ptr(scratch), scratch.numel() if scratch is not None else 0,
              _stream()), "matmul_forward")
     return out
@@ -74,7 +93,7 @@ def linear_forward(x, w, bias=None, out=None, scratch=None):
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty(M, N, dtype=x.dtype, device=x.device) if out is None else out
-    fn = getattr(lib, f"linear_forward_entry_point_{_sfx(x)}")
+    fn = _linear(x)
     check(fn(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), M, N, K, x.stride(0), x.stride(1), w.stride(0), w.stride(1),
              out.stride(0), out.stride(1), _ptr(scratch), scratch.numel() if scratch is not None else 0, _stream()),
           "linear_forward")
@@ -89,7 +108,7 @@ def flash_attention2_forward(q, k, v, softmax_scale, want_lse=True):
     nk = k.shape[1]
     o = torch.empty_like(q)
     l = torch.empty(BH, nq, dtype=_F32, device=q.device) if want_lse else None
-    fn = getattr(lib, f"flash_attention2_forward_entry_point_{_sfx(q)}")
+    fn = _attention2(q)
     check(fn(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(l), nq, nk, float(softmax_scale), float("-inf"), BH, D,
              _stream()), "flash_attention2_forward")
     return o, l
