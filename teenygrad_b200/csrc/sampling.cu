@@ -17,8 +17,14 @@
 // goes into a list per CTA; the first CTA sorts their union, which also orders the ties at the threshold (a row with
 // thousands of them, such as a masked one, is collected in index order instead).  One thread does the running sums,
 // so that the result does not depend on a reduction tree; the cut and the pick are searches over them.
-// Measured on B200: 32 x 151936, top-k 50: 18.8 us, 8 rows, top-k 1000: 29 us; with one CTA per row, 2-byte loads and an ordered pass of
-// four barriers per 1024 columns the former took 154 us.
+//
+// Mostly no histogram is needed: logits share a handful of exponents, so that a warp's 32 increments of the high byte's bins mostly hit the
+// same one or two.  Instead each thread takes the largest of its columns' keys (packed pairs), and each of the row's P CTAs finds the
+// ceil(K / P)-th largest of its 1024, a bit at a time by barriers that count.  The smallest of these P bounds is reached by at least K
+// entries of the row, so every one of the top K is among the entries not below it, of which there are little more than K: only the threads whose
+// largest reaches it look at their columns again.  Where they do not fit the list (ties), or the threads are too few, the histograms decide.
+// Measured on B200, before (histograms, bitonic sort) and now: 32 x 151936, top-k 50 17.0 -> 11.8 us, top-k 1000 36.4 -> 19.8; 8 x 151936 16.4 -> 11.5;
+// 64 x 151936 22.8 -> 13.9; 64 x 32768 13.0 -> 8.7; 5 x 1000 8.4 -> 6.7.
 #include <atomic>
 
 #include "common.cuh"
@@ -77,14 +83,18 @@ __device__ __forceinline__ void pick_from_sorted(const unsigned long long* cand,
   __syncthreads();
   if (tid == 0) {
     float c = 0.0f;
+    float4 x = *reinterpret_cast<const float4*>(sh.e), y = *reinterpret_cast<const float4*>(sh.e + 4);
     for (unsigned i = 0; i < K; i += 8) {  // the sums behind K are not read
-      const float4 x = *reinterpret_cast<const float4*>(sh.e + i), y = *reinterpret_cast<const float4*>(sh.e + i + 4);
+      const unsigned next = min(i + 8, static_cast<unsigned>(kMaxTopK) - 8u);  // on its way while these are added
+      const float4 xn = *reinterpret_cast<const float4*>(sh.e + next), yn = *reinterpret_cast<const float4*>(sh.e + next + 4);
       float4 r, t;
       r.x = c + x.x; r.y = r.x + x.y; r.z = r.y + x.z; r.w = r.z + x.w;
       t.x = r.w + y.x; t.y = t.x + y.y; t.z = t.y + y.z; t.w = t.z + y.w;
       c = t.w;
       *reinterpret_cast<float4*>(sh.c + i) = r;
       *reinterpret_cast<float4*>(sh.c + i + 4) = t;
+      x = xn;
+      y = yn;
     }
   }
   __syncthreads();
@@ -165,13 +175,88 @@ __device__ __forceinline__ void sort_descending(unsigned long long* cand, unsign
   }
 }
 
+// Keys of two bf16 numbers at once.
+__device__ __forceinline__ unsigned sort_keys2(unsigned w) { return w ^ (((w >> 15) & 0x00010001u) * 0xffffu | 0x80008000u); }
+
+// Sorts the first n <= 128 slots of `from` descending into `to` by counting, for each, the larger ones (the slots differ): 1024 / (n rounded
+// up) threads per slot.
+__device__ __forceinline__ void sort_by_rank(const unsigned long long* from, unsigned long long* to, unsigned n) {
+  unsigned lg = 5;  // threads of a slot
+  while ((static_cast<unsigned>(kSampleThreads) >> lg) < n) --lg;
+  const unsigned at = threadIdx.x >> lg, sub = threadIdx.x & ((1u << lg) - 1u);
+  const unsigned long long mine = at < n ? from[at] : 0ull;
+  unsigned larger = 0;
+  for (unsigned i = sub; i < n; i += 1u << lg) larger += from[i] > mine ? 1u : 0u;
+  for (unsigned o = 1u << lg >> 1; o > 0; o >>= 1) larger += __shfl_xor_sync(0xffffffffu, larger, o);
+  if (at < n && sub == 0) to[larger] = mine;
+  __syncthreads();
+}
+
+// Sorts the first n <= 2048 slots of `from`, whose keys are not below `lowest`, descending into `from` again: into bins, one per key, in the
+// order of the keys (`other` has them then), and each by counting within its bin.  Returns false, with `from` as it was, where the keys are too far apart (1024:
+// 8 octaves) or a bin too full.  1100 slots: about 1 us, the bitonic sort 8.
+__device__ __forceinline__ bool sort_by_key(unsigned long long* from, unsigned long long* other, unsigned n, unsigned lowest, unsigned* count,
+                                            unsigned* base, unsigned* warp_tot) {
+  constexpr unsigned kBins = kSampleThreads, kMost = 128;
+  const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned long long x[2];
+  unsigned bin[2], place[2];
+  bool far = false;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const unsigned i = tid + kSampleThreads * j;
+    x[j] = i < n ? from[i] : 0ull;
+    bin[j] = static_cast<unsigned>(x[j] >> 32) - lowest;
+    far |= i < n && bin[j] >= kBins;
+  }
+  count[tid] = 0;
+  if (__syncthreads_or(far)) return false;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (tid + kSampleThreads * j < n) place[j] = atomicAdd(count + bin[j], 1u);
+  __syncthreads();
+  // slots in the bins above: thread t has bin 1023 - t
+  const unsigned mine = count[kBins - 1 - tid];
+  unsigned upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
+  }
+  if (lane == 31) warp_tot[warp] = upto;
+  if (__syncthreads_or(mine > kMost)) return false;
+  unsigned before = warp_tot[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned t = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += t;
+  }
+  before = __shfl_sync(0xffffffffu, before, (warp + 31) & 31);
+  base[kBins - 1 - tid] = upto - mine + (warp ? before : 0u);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (tid + kSampleThreads * j < n) other[base[bin[j]] + place[j]] = x[j];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    if (tid + kSampleThreads * j >= n) continue;
+    const unsigned b = base[bin[j]], end = b + count[bin[j]];
+    unsigned at = b;
+    for (unsigned i = b; i < end; ++i) at += other[i] > x[j] ? 1u : 0u;
+    from[at] = x[j];
+  }
+  __syncthreads();
+  return true;
+}
+
 struct SampleShared {
   unsigned hist[2][256];                       // this CTA's histograms
   unsigned sum[256];                           // the row's
   unsigned long long list[kSampleList];        // this CTA's candidates
   unsigned long long cand[kSampleList];        // the row's (first CTA)
   PickShared pick;
-  unsigned bin, above, count, eq_base, warp_tot[32];
+  unsigned bin, above, count, eq_base, bound, warp_tot[32];
 };
 
 // cand_out != null: stop after step 1 and write the K sorted candidates of the row, indices shifted by idx_offset, to
@@ -181,7 +266,7 @@ __global__ void __launch_bounds__(kSampleThreads, 1)
 sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int cols, float inv_temperature, int top_k,
                           float top_p, const float* __restrict__ u, int* __restrict__ out_idx,
                           float* __restrict__ out_prob, unsigned long long* __restrict__ cand_out, int cand_stride,
-                          int idx_offset, int parts) {
+                          int idx_offset, int parts, int by_bound) {
   __shared__ __align__(16) SampleShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned rank = parts > 1 ? cluster_rank() : 0u;
@@ -216,88 +301,182 @@ sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int col
   if (tid == 0) sh.count = 0;
   __syncthreads();
   pdl_wait();
-  // ---- pass 1: histogram of the key's high byte ----
-  for_keys(row, begin, end, [&](int, unsigned k) { atomicAdd(&sh.hist[0][k >> 8], 1u); });
-  decide(0, K);
-  const unsigned hi_bin = sh.bin, above_hi = sh.above;
-  // ---- pass 2: histogram of the low byte inside that bin ----
-  for_keys(row, begin, end, [&](int, unsigned k) { if ((k >> 8) == hi_bin) atomicAdd(&sh.hist[1][k & 255u], 1u); });
-  decide(1, K - above_hi);
-  const unsigned thresh = (hi_bin << 8) | sh.bin;        // the K-th largest key
-  const unsigned above = above_hi + sh.above;            // entries above it
-  const unsigned total = above + sh.sum[sh.bin];         // and with all of its ties
-  // ---- pass 3 ----
-  unsigned sorted;  // slots of cand[] in use, a power of two
-  if (total <= kSampleList) {
-    for_keys(row, begin, end, [&](int i, unsigned k) {
-      if (k >= thresh) sh.list[atomicAdd(&sh.count, 1u)] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(i));
-    });
-    sync_row();
-    for (sorted = 32; sorted < total; sorted <<= 1) {}
-    if (rank == 0) {
-      unsigned at = 0;
-      for (int p = 0; p < parts; ++p) {
-        const unsigned n = parts > 1 ? ld_peer_u32(peer_smem(&sh.count, p)) : sh.count;
-        for (unsigned i = tid; i < n; i += kSampleThreads) sh.cand[at + i] = parts > 1 ? ld_peer_u64(peer_smem(&sh.list[i], p)) : sh.list[i];
-        at += n;
-      }
-      for (unsigned i = at + tid; i < sorted; i += kSampleThreads) sh.cand[i] = 0ull;
+  unsigned entries = 0, lowest = 0;  // in cand[], unsorted; no key is below
+  bool found = false;
+  if (by_bound) {
+    // The row as 16-byte vectors behind `head` columns; the first and last columns that fill none are a few threads' of the first CTA.
+    const int head = min(cols, static_cast<int>((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) >> 1), vecs = (cols - head) >> 3;
+    const int per = (vecs + parts - 1) / parts, v0 = min(vecs, static_cast<int>(rank) * per), v1 = min(vecs, v0 + per);
+    const int tail0 = head + 8 * vecs, odd = rank == 0 ? (tid < head ? tid : (tid - head < cols - tail0 ? tail0 + tid - head : -1)) : -1;
+    const uint4* vec = reinterpret_cast<const uint4*>(row + head);
+    unsigned top2 = 0;
+#pragma unroll 4
+    for (int i = v0 + tid; i < v1; i += kSampleThreads) {
+      const uint4 v = vec[i];
+      top2 = __vmaxu2(top2, __vmaxu2(__vmaxu2(sort_keys2(v.x), sort_keys2(v.y)), __vmaxu2(sort_keys2(v.z), sort_keys2(v.w))));
     }
-    if (parts > 1) cluster_sync();  // nobody leaves while its list is being read
-    if (rank != 0) return;
-  } else {
-    if (parts > 1) cluster_sync();  // nor while its histogram is
-    if (rank != 0) return;
-    // in index order: everything above the threshold, and the first need_eq entries equal to it
-    const unsigned need_eq = K - above;
-    sorted = kMaxTopK;
-    if (tid == 0) sh.eq_base = 0;
-    for (int i = tid; i < kMaxTopK; i += kSampleThreads) sh.cand[i] = 0ull;
-    __syncthreads();
-    for (int base = 0; base < cols; base += kSampleThreads) {
-      const int i = base + tid;
-      const unsigned k = i < cols ? sort_key(row[i]) : 0u;
-      const bool gt = i < cols && k > thresh, eq = i < cols && k == thresh;
-      // rank of this thread's tie among the ties of the tile (block-wide exclusive count in index order)
-      const unsigned eq_mask = __ballot_sync(0xffffffffu, eq);
-      if (lane == 0) sh.warp_tot[warp] = __popc(eq_mask);
-      __syncthreads();
-      unsigned before = sh.eq_base;
-      for (int w = 0; w < warp; ++w) before += sh.warp_tot[w];
-      before += __popc(eq_mask & ((1u << lane) - 1u));
-      if (gt || (eq && before < need_eq)) {
-        const unsigned slot = atomicAdd(&sh.count, 1u);
-        if (slot < static_cast<unsigned>(kMaxTopK))
-          sh.cand[slot] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(i));
+    unsigned top = max(top2 & 0xffffu, top2 >> 16);
+    if (odd >= 0) top = max(top, sort_key(row[odd]));
+    unsigned bound = 0;
+    const int want = static_cast<int>((K + parts - 1) / parts);
+    for (unsigned bit = 0x8000u; bit; bit >>= 1)
+      if (__syncthreads_count(top >= (bound | bit)) >= want) bound |= bit;
+    if (parts > 1) {
+      if (tid == 0) sh.bound = bound;
+      cluster_sync();
+      unsigned v[8];
+#pragma unroll
+      for (int p = 0; p < 8; ++p) v[p] = p < parts ? ld_peer_u32(peer_smem(&sh.bound, p)) : bound;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) bound = min(bound, v[p]);
+    }
+    if (top >= bound) {
+      auto list = [&](int i, unsigned k) {
+        if (k < bound) return;
+        const unsigned at = atomicAdd(&sh.count, 1u);
+        if (at < kSampleList) sh.list[at] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(i));
+      };
+      if (odd >= 0) list(odd, sort_key(row[odd]));
+#pragma unroll 4
+      for (int i = v0 + tid; i < v1; i += kSampleThreads) {
+        const uint4 v = vec[i];
+        const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          list(head + 8 * i + 2 * j, sort_key(static_cast<unsigned short>(w[j] & 0xffffu)));
+          list(head + 8 * i + 2 * j + 1, sort_key(static_cast<unsigned short>(w[j] >> 16)));
+        }
       }
-      __syncthreads();
-      if (tid == 0) {
-        unsigned t = 0;
-        for (int w = 0; w < 32; ++w) t += sh.warp_tot[w];
-        sh.eq_base += t;
+    }
+    sync_row();
+    unsigned n[8], total = 0;  // (a list that ran over has a count beyond it)
+#pragma unroll
+    for (int p = 0; p < 8; ++p) n[p] = p < parts ? (parts > 1 ? ld_peer_u32(peer_smem(&sh.count, p)) : sh.count) : 0u;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) total += n[p];
+    found = total <= kSampleList;
+    if (found) {
+      if (rank == 0) {
+        unsigned at = 0;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+          if (p >= parts) break;
+          for (unsigned i = tid; i < n[p]; i += kSampleThreads) sh.cand[at + i] = parts > 1 ? ld_peer_u64(peer_smem(&sh.list[i], p)) : sh.list[i];
+          at += n[p];
+        }
       }
-      __syncthreads();
+      if (parts > 1) cluster_sync(); else __syncthreads();  // nobody leaves while its list is being read
+      if (rank != 0) return;
+      entries = total;
+      lowest = bound;
+    } else {
+      sync_row();  // the counts are read
+      if (tid == 0) sh.count = 0;
     }
   }
-  __syncthreads();
-  sort_descending(sh.cand, sorted);  // empty slots are zero and end up last
+  if (!found) {
+    // ---- pass 1: histogram of the key's high byte ----
+    for_keys(row, begin, end, [&](int, unsigned k) { atomicAdd(&sh.hist[0][k >> 8], 1u); });
+    decide(0, K);
+    const unsigned hi_bin = sh.bin, above_hi = sh.above;
+    // ---- pass 2: histogram of the low byte inside that bin ----
+    for_keys(row, begin, end, [&](int, unsigned k) { if ((k >> 8) == hi_bin) atomicAdd(&sh.hist[1][k & 255u], 1u); });
+    decide(1, K - above_hi);
+    const unsigned thresh = (hi_bin << 8) | sh.bin;        // the K-th largest key
+    const unsigned above = above_hi + sh.above;            // entries above it
+    const unsigned total = above + sh.sum[sh.bin];         // and with all of its ties
+    // ---- pass 3 ----
+    lowest = thresh;
+    if (total <= kSampleList) {
+      for_keys(row, begin, end, [&](int i, unsigned k) {
+        if (k >= thresh) sh.list[atomicAdd(&sh.count, 1u)] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(i));
+      });
+      sync_row();
+      if (rank == 0) {
+        unsigned at = 0;
+        for (int p = 0; p < parts; ++p) {
+          const unsigned n = parts > 1 ? ld_peer_u32(peer_smem(&sh.count, p)) : sh.count;
+          for (unsigned i = tid; i < n; i += kSampleThreads) sh.cand[at + i] = parts > 1 ? ld_peer_u64(peer_smem(&sh.list[i], p)) : sh.list[i];
+          at += n;
+        }
+      }
+      entries = total;
+      if (parts > 1) cluster_sync();  // nobody leaves while its list is being read
+      if (rank != 0) return;
+    } else {
+      if (parts > 1) cluster_sync();  // nor while its histogram is
+      if (rank != 0) return;
+      // in index order: everything above the threshold, and the first need_eq entries equal to it
+      const unsigned need_eq = K - above;
+      entries = K;
+      if (tid == 0) sh.eq_base = 0;
+      __syncthreads();
+      for (int base = 0; base < cols; base += kSampleThreads) {
+        const int i = base + tid;
+        const unsigned k = i < cols ? sort_key(row[i]) : 0u;
+        const bool gt = i < cols && k > thresh, eq = i < cols && k == thresh;
+        // rank of this thread's tie among the ties of the tile (block-wide exclusive count in index order)
+        const unsigned eq_mask = __ballot_sync(0xffffffffu, eq);
+        if (lane == 0) sh.warp_tot[warp] = __popc(eq_mask);
+        __syncthreads();
+        unsigned before = sh.eq_base;
+        for (int w = 0; w < warp; ++w) before += sh.warp_tot[w];
+        before += __popc(eq_mask & ((1u << lane) - 1u));
+        if (gt || (eq && before < need_eq)) {
+          const unsigned slot = atomicAdd(&sh.count, 1u);
+          if (slot < static_cast<unsigned>(kMaxTopK))
+            sh.cand[slot] = (static_cast<unsigned long long>(k) << 32) | (0xFFFFFFFFu - static_cast<unsigned>(i));
+        }
+        __syncthreads();
+        if (tid == 0) {
+          unsigned t = 0;
+          for (int w = 0; w < 32; ++w) t += sh.warp_tot[w];
+          sh.eq_base += t;
+        }
+        __syncthreads();
+      }
+    }
+    __syncthreads();
+  }
+  const unsigned long long* sorted_list = sh.cand;
+  if (entries <= 128) {
+    sort_by_rank(sh.cand, sh.list, entries);
+    sorted_list = sh.list;
+  } else if (!sort_by_key(sh.cand, sh.list, entries, lowest, reinterpret_cast<unsigned*>(sh.pick.e), reinterpret_cast<unsigned*>(sh.pick.c), sh.warp_tot)) {
+    unsigned slots = 256;
+    while (slots < entries) slots <<= 1;
+    for (unsigned i = entries + tid; i < slots; i += kSampleThreads) sh.cand[i] = 0ull;  // these end up last
+    __syncthreads();
+    sort_descending(sh.cand, slots);
+  }
   if (cand_out) {
     // entries past K are zero (smaller than any real candidate); the shift keeps (value desc, index asc) order
     if (tid < cand_stride) {
-      const unsigned long long c = static_cast<unsigned>(tid) < K ? sh.cand[tid] : 0ull;
+      const unsigned long long c = static_cast<unsigned>(tid) < K ? sorted_list[tid] : 0ull;
       cand_out[static_cast<size_t>(r) * cand_stride + tid] =
           static_cast<unsigned>(tid) < K ? ((c & 0xFFFFFFFF00000000ull) | ((c & 0xFFFFFFFFull) - static_cast<unsigned>(idx_offset))) : 0ull;
     }
     return;
   }
-  pick_from_sorted(sh.cand, sh.pick, K, inv_temperature, top_p, u[r], out_idx + r, out_prob ? out_prob + r : nullptr);
+  pick_from_sorted(sorted_list, sh.pick, K, inv_temperature, top_p, u[r], out_idx + r, out_prob ? out_prob + r : nullptr);
 }
 
-// CTAs per row: as many as keep the grid within one CTA per SM (what its 1024 threads allow), and a slice at least half a round of
-// 16-byte loads.
-int sample_parts(int rows, int cols) {
-  int parts = 1;
-  while (parts < 8 && 2LL * rows * parts <= sm_count() && cols >= 2 * parts * kSampleThreads * 4) parts *= 2;
+// Whether the threads' largest keys bound the candidates well: a bound that k of g largest keys reach is reached by about -g ln(1 - k / g)
+// entries, 1.6 g at k = 0.8 g.
+bool sample_by_bound(int cols, int top_k, int parts) {
+  const int k = ((top_k < cols ? top_k : cols) + parts - 1) / parts, groups = (cols / 8 + parts - 1) / parts;
+  return 10 * k <= 8 * (groups < kSampleThreads ? groups : kSampleThreads);
+}
+
+// CTAs per row: up to four, while all clusters are resident at once (one CTA per SM by its 1024 threads; the GPU's SMs hold 33 clusters of four of these)
+// and slices are no less than what the meetings of the cluster cost, or as many as the bounds take.  Top-k 50, one, two, four, eight CTAs a row:
+// 1 x 151936 17.5, 13.3, 11.2, 12.2 us; 32 x 151936 18.4, 14.5, 12.4; 36 rows 18.6, 14.5, 20.4; 37 x 70001 12.2, 11.5; 16 x 32768 9.1, 9.7, 9.8, 19.2 (16 clusters
+// of eight do not find place).
+int sample_parts(int rows, int cols, int top_k) {
+  const int sms = sm_count();
+  const bool two = 2LL * rows <= sms, four = 9LL * rows <= 2 * sms;
+  int parts = !two || cols < 65536 ? 1 : (four && cols >= 98304 ? 4 : 2);
+  while ((parts == 1 ? two : parts == 2 && four) && !sample_by_bound(cols, top_k, parts) && sample_by_bound(cols, top_k, 2 * parts)) parts *= 2;
   return parts;
 }
 
@@ -377,9 +556,10 @@ int sample_top_k_top_p_bf16(const bf16* logits, long long ld, int rows, int cols
   if (!logits || !u || !out_idx || rows < 0 || cols <= 0 || ld < cols) return TEENY_ERR_BAD_ARG;
   if (!(temperature > 0.0f) || top_k < 1 || top_k > kMaxTopK || !(top_p > 0.0f) || top_p > 1.0f) return TEENY_ERR_BAD_ARG;
   if (rows == 0) return TEENY_OK;
-  const int parts = sample_parts(rows, cols);
+  const int parts = sample_parts(rows, cols, top_k);
   launch_kernel(sample_top_k_top_p_kernel, dim3(rows * parts), dim3(kSampleThreads), 0, st, static_cast<unsigned>(parts), logits, ld, cols,
-                1.0f / temperature, top_k, top_p, u, out_idx, out_prob, static_cast<unsigned long long*>(nullptr), 0, 0, parts);
+                1.0f / temperature, top_k, top_p, u, out_idx, out_prob, static_cast<unsigned long long*>(nullptr), 0, 0, parts,
+                static_cast<int>(sample_by_bound(cols, top_k, parts)));
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -388,10 +568,10 @@ int sample_candidates_bf16(const bf16* logits, long long ld, int rows, int cols,
   if (!logits || !cand_out || rows < 0 || cols <= 0 || ld < cols || top_k < 1 || top_k > kMaxTopK || idx_offset < 0)
     return TEENY_ERR_BAD_ARG;
   if (rows == 0) return TEENY_OK;
-  const int parts = sample_parts(rows, cols);
+  const int parts = sample_parts(rows, cols, top_k);
   launch_kernel(sample_top_k_top_p_kernel, dim3(rows * parts), dim3(kSampleThreads), 0, st, static_cast<unsigned>(parts), logits, ld, cols,
                 1.0f, top_k, 1.0f, static_cast<const float*>(nullptr), static_cast<int*>(nullptr), static_cast<float*>(nullptr), cand_out,
-                top_k, idx_offset, parts);
+                top_k, idx_offset, parts, static_cast<int>(sample_by_bound(cols, top_k, parts)));
   return static_cast<int>(cudaGetLastError());
 }
 

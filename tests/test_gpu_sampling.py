@@ -54,3 +54,26 @@ def test_picks_follow_the_definition(ops, kind, rows, cols, top_k):
             masses = [c[m] for m in range(len(c)) if abs(c[m] - 0.9 * c[-1]) <= tol] + [c[n - 1]]
             assert any((c[i - 1] if i else 0.0) - tol <= float(u[r]) * m <= c[i] + tol for m in masses)
     assert ops.device_error() == 0
+
+
+def test_candidates_at_the_edges_of_the_bounds(ops):
+    """Top-k around what the threads' largest keys bound (a CTA's 1024 threads, one to four CTAs a row), ordered rows, rows whose largest entries share a
+    thread, keys far apart, and candidate counts around the two ways of sorting them: the picks of u near 0 and 1 and of the whole nucleus."""
+    from oracle import sampling as osamp
+    g = torch.Generator().manual_seed(3)
+    for rows, cols, top_k in [(3, 33001, 819), (2, 70008, 820), (1, 151936, 1000), (40, 99999, 128), (2, 8200, 129), (2, 1029, 103), (2, 1031, 1024), (80, 16384, 300)]:
+        x = torch.randn(rows, cols, generator=g) * 3
+        x[0] = x[0].sort().values          # the largest side by side
+        x[-1, ::997] *= 2.0 ** 40          # keys far apart
+        x = x.bfloat16()
+        for u in (0.0, 0.5, 0.999):
+            got, prob = ops.sample_top_k_top_p(x.cuda(), 0.9, top_k, 1.0, torch.full((rows,), u).cuda(), want_prob=True)
+            for r in {0, rows - 1, rows // 2}:
+                want, wprob, c, n, cand = osamp.sample_row(x[r].float().numpy(), 0.9, top_k, 1.0, u)
+                if int(got[r]) != want:  # the neighbour across a boundary of the running sums
+                    i = list(cand).index(int(got[r]))
+                    tol = 1e-5 * c[-1]
+                    assert (c[i - 1] if i else 0.0) - tol <= u * c[-1] <= c[i] + tol
+                else:
+                    assert abs(float(prob[r]) - wprob) <= 1e-4
+    assert ops.device_error() == 0
