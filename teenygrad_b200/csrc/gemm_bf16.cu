@@ -199,19 +199,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
 
   const int num_work = args.tiles_p * args.tiles_q;
 
+  // The producer's and the issuer's whole warps walk their loops and one lane issues, so that addresses and descriptors stay in uniform
+  // registers: by one lane alone a 64-k block took 470 clocks to issue whatever the tile, now 255 (128 x 128 tiles 290).
+  const bool one = elect_one();
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
-        int tp, tq;
-        tile_coords(w, args.tiles_p, args.tiles_q, args.group, tp, tq);
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1, err, DEVERR_GEMM_PRODUCER)) { ok = false; break; }
-          const uint32_t sp = smem_base + stage * Cfg::kStageBytes;
-          const uint32_t sq = sp + Cfg::kStageP;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
+      int tp, tq;
+      tile_coords(w, args.tiles_p, args.tiles_q, args.group, tp, tq);
+      for (int kb = 0; kb < args.k_blocks; ++kb) {
+        if (!mbar_wait(empty_bar(stage), phase ^ 1, err, DEVERR_GEMM_PRODUCER)) { ok = false; break; }
+        const uint32_t sp = smem_base + stage * Cfg::kStageBytes;
+        const uint32_t sq = sp + Cfg::kStageP;
+        if (one) {
           mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
           tma_load_2d(sp, &tmap_p, full_bar(stage), kb * kBK, tp * kBM);
           if constexpr (Q_MN_MAJOR) {
@@ -222,33 +225,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
           } else {
             tma_load_2d(sq, &tmap_q, full_bar(stage), kb * kBK, tq * BN);
           }
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int local = 0;
-      for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x, ++local) {
-        const int buf = local & 1;
-        const uint32_t acc_phase = (local >> 1) & 1;
-        if (!mbar_wait(acc_empty_bar(buf), acc_phase ^ 1, err, DEVERR_GEMM_MMA)) { ok = false; break; }
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int local = 0;
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, Q_MN_MAJOR);
+    const uint64_t pdesc = make_smem_desc_sw128(smem_base, 16, 1024);
+    const uint64_t qdesc = make_smem_desc_sw128(smem_base + Cfg::kStageP, Q_MN_MAJOR ? kBK * 128 : 16, 1024);
+    uint32_t off = 0;  // of the stage, in the descriptors' 16 bytes
+    for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x, ++local) {
+      const int buf = local & 1;
+      const uint32_t acc_phase = (local >> 1) & 1;
+      if (!mbar_wait(acc_empty_bar(buf), acc_phase ^ 1, err, DEVERR_GEMM_MMA)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * BN;
+      bool ready = mbar_try_wait(full_bar(stage), phase);  // asked a block ahead
+      for (int kb = 0; kb < args.k_blocks; ++kb) {
+        if (!ready && !mbar_wait(full_bar(stage), phase, err, DEVERR_GEMM_MMA)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, err, DEVERR_GEMM_MMA)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sp = smem_base + stage * Cfg::kStageBytes;
-          issue_kblock<BN, Q_MN_MAJOR>(d_tmem, sp, sp + Cfg::kStageP, kb == 0);
+        if (one) {
+          umma_bf16_ss_x4<2, Q_MN_MAJOR ? 128 : 2>(d_tmem, pdesc + off, qdesc + off, idesc, kb ? 1u : 0u);
           umma_commit(empty_bar(stage));  // stage reusable once these MMAs have read it
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit(acc_full_bar(buf));
+        off += Cfg::kStageBytes / 16;
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; off = 0; }
+        ready = kb + 1 < args.k_blocks && mbar_try_wait(full_bar(stage), phase);
       }
+      if (ok && one) umma_commit(acc_full_bar(buf));
     }
   } else {
     // ---------------- epilogue (warps 2..5; TMEM lane quarter = warp % 4) ----------------
@@ -468,9 +477,8 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t
   return v;
 }
 
-// grid (S, tiles, token tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile, blockIdx.z = BN tokens (TOKEN_TILES;
-// compiled apart, since every decode GEMM would pay for the offsets: 32 x 4096 x 4096 12.2 us with them, 12.05 without).
-template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
+// grid (S, tiles): blockIdx.x = cluster rank = k-split, blockIdx.y = 128-row weight tile
+template <int BN, bool W8 = false, bool F8 = false>
 __global__ void __launch_bounds__((SkinnyCfg<BN, W8, F8>::kThreads), 2)
 gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const GemmArgs args) {
@@ -496,8 +504,8 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   int* err = args.err;
   const uint32_t S = cluster_size(), rank = cluster_rank();
   const int tile = blockIdx.y;
-  const int m0 = TOKEN_TILES ? blockIdx.z * BN : 0, rows = args.M - m0;  // this CTA's tokens
-  bf16* const y = args.y + static_cast<size_t>(m0) * args.ldy;
+  const int rows = args.M;
+  bf16* const y = args.y;
   const int kb0 = static_cast<int>(rank) * args.kb_per_split;
   const int kb1 = min(args.k_blocks, kb0 + args.kb_per_split);
   // W8: what the accumulator of weight row n is multiplied by on the way out (per-group scales are already in the
@@ -540,7 +548,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       // while the previous kernel may still be running; the activation tiles follow once it has finished.  Weights that
       // the kernel in front may be writing (an operator's, a prefill's converted copy) are only asked into L2, where its
       // stores arrive, too.
-      const int ring = min(kb1 - kb0, Cfg::kStages), pre = !TOKEN_TILES && args.w_early ? ring : 0;
+      const int ring = min(kb1 - kb0, Cfg::kStages), pre = args.w_early ? ring : 0;
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), Cfg::kStageBytes);
         tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, full_bar(i), (kb0 + i) * Cfg::kKB, tile * kBM);
@@ -551,9 +559,9 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
       pdl_wait();
       auto load_x = [&](uint32_t sq, uint32_t bar, int kb) {  // the activation tile(s) of one stage: 64 k each
-        tma_load_2d(sq, &tmap_x, bar, kb * Cfg::kKB, m0);
-        if constexpr (F8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB, args.x_lo_row + m0);  // the lo terms
-        else if constexpr (W8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB + kBK, m0);
+        tma_load_2d(sq, &tmap_x, bar, kb * Cfg::kKB, 0);
+        if constexpr (F8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB, args.x_lo_row);  // the lo terms
+        else if constexpr (W8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB + kBK, 0);
       };
       for (int i = 0; i < pre; ++i) load_x(smem_base + i * Cfg::kStageBytes + Cfg::kStageP, full_bar(i), kb0 + i);
       int stage = pre == Cfg::kStages ? 0 : pre;
@@ -710,7 +718,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
           for (int e = 0; e < kChunk; ++e) {
             if constexpr (F8) {
-              const float xs = (c0 + e < rows) ? __ldg(args.x_scale + m0 + c0 + e) : 0.0f;
+              const float xs = (c0 + e < rows) ? __ldg(args.x_scale + c0 + e) : 0.0f;
               r[e] = __float_as_uint(fmaf(__uint_as_float(r1[e]), 0.0625f, __uint_as_float(r[e])) * xs);
             } else {
               r[e] = __float_as_uint(__uint_as_float(r[e]) + __uint_as_float(r1[e]));
@@ -885,13 +893,13 @@ int prepare_variant() {
   return 0;
 }
 
-template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
+template <int BN, bool W8 = false, bool F8 = false>
 int prepare_skinny() {
   static std::atomic<unsigned long long> done{0};  // one bit per device; threads may race to set it
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && (done.load(std::memory_order_acquire) >> dev) & 1ull) return 0;
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_skinny_kernel<BN, W8, F8, TOKEN_TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_skinny_kernel<BN, W8, F8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        SkinnyCfg<BN, W8, F8>::kSmemBytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
@@ -906,12 +914,11 @@ int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, const GemmArgs&
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int BN, bool W8 = false, bool F8 = false, bool TOKEN_TILES = false>
-int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int split, int tiles,
-                  cudaStream_t st, int token_tiles = 1) {
-  const int rc = prepare_skinny<BN, W8, F8, TOKEN_TILES>();
+template <int BN, bool W8 = false, bool F8 = false>
+int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int split, int tiles, cudaStream_t st) {
+  const int rc = prepare_skinny<BN, W8, F8>();
   if (rc) return rc;
-  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8, TOKEN_TILES>, dim3(split, tiles, token_tiles),
+  return launch_kernel(gemm_bf16_skinny_kernel<BN, W8, F8>, dim3(split, tiles, 1),
                        dim3(SkinnyCfg<BN, W8, F8>::kThreads, 1, 1), SkinnyCfg<BN, W8, F8>::kSmemBytes, st,
                        static_cast<unsigned>(split), tw, tx, a);
 }
@@ -936,39 +943,29 @@ int swap_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128))
 
 // More than kSwapMaxM tokens: the kernel that is estimated to end first.  Microseconds: a start, and the rounds of tiles over the SMs
 // times the 64-k blocks of a tile times what a block takes.  Fitted to calls with 129 to 4500 tokens (M x N x K; narrow 128 x 128
-// tiles / wide 128 x 256 / CTA pairs with 256 x 256 / K of 128 x 128 tiles over clusters):
-//   800 x 4096 x 4096 40.0 / 30.9 / 28.6 / 41.6     300 x 12288 x 1024 16.3 / 16.6 / 22.1 / 24.6     512 x 1024 x 3072 17.4 / 21.0 / 21.4 / 11.7
-//   200 x 4096 x 12288 54.5 / 75.3 / 62.7 / 32.5    4500 x 1024 x 3072 33.3 / 24.5 / 24.3 / -        200 x 520 x 8192 39.3 / 46.4 / 46.8 / 12.5
-// (By tile counts alone, wide tiles only with one for every SM and no K split, these took 40.7, 22.0, 17.4, 54.4, 33.1 and 41.7.)
-// An estimate is good to a few per cent: what the tile counts alone would take stays unless another kernel is estimated to be 3.5 % faster (700 x
-// 1024 x 1024: narrow 9.2 us, K over three CTAs 10.5, estimated 9.5 and 9.2; 1500 x 4096 x 1024: pairs 18.4, narrow 19.4, estimated 18.5 and
-// 18.4).  Of 541 sizes with 129 to 4500 tokens two are then 3 and 6 % slower than by tile counts, instead of nine by 4 to 18 %.
-enum { kLargeNone, kLargeNarrow, kLargeWide, kLargePair, kLargeSplit };
-struct LargeChoice { int kind, split; };
+// tiles / wide 128 x 256 / CTA pairs with 256 x 256):
+//   800 x 4096 x 4096 40.0 / 30.9 / 28.6     300 x 12288 x 1024 16.3 / 16.6 / 22.1     512 x 1024 x 3072 17.4 / 21.0 / 21.4
+//   4500 x 1024 x 3072 33.3 / 24.5 / 24.3
+// An estimate is good to a few per cent: what the tile counts alone would take stays unless another kernel is estimated to be 3.5 % faster.
+// Beside them stand tiles that are all resident at once, also with K over clusters (gemm_bf16_split.cu).
+enum { kLargeNarrow, kLargeWide, kLargePair };
+struct LargeChoice { int kind; double us; };
 LargeChoice choose_large(int M, int N, int k_blocks, int sms) {
   auto rounds = [](long long tiles, long long slots) { return static_cast<double>((tiles + slots - 1) / slots); };
   const long long m128 = ceil_div(M, 128), n128 = ceil_div(N, 128), n256 = ceil_div(N, 256), pairs = static_cast<long long>(ceil_div(M, 256)) * n256;
   const double narrow = 5.0 + rounds(m128 * n128, sms) * k_blocks * 0.28;
   const double wide = 8.0 + rounds(m128 * n256, sms) * k_blocks * 0.385;
   const double pair = 7.5 + rounds(pairs, sms / 2) * k_blocks * 0.345;
-  LargeChoice best{kLargeNarrow, 0};
-  double least = narrow;
-  if (pairs >= sms / 2) { best.kind = kLargePair; least = pair; }
-  else if (N > 128 && m128 * n256 >= sms) { best.kind = kLargeWide; least = wide; }
-  least *= 0.965;
-  auto consider = [&](int kind, int split, double t) {
-    if (t < least) { best = LargeChoice{kind, split}; least = t; }
+  LargeChoice best{kLargeNarrow, narrow};
+  if (pairs >= sms / 2) best = LargeChoice{kLargePair, pair};
+  else if (N > 128 && m128 * n256 >= sms) best = LargeChoice{kLargeWide, wide};
+  best.us *= 0.965;
+  auto consider = [&](int kind, double t) {
+    if (t < best.us) best = LargeChoice{kind, t};
   };
-  consider(kLargeNarrow, 0, narrow);
-  if (N > 128) consider(kLargeWide, 0, wide);
-  consider(kLargePair, 0, pair);
-  for (int split = 2; split <= 8; ++split) {
-    const int per = ceil_div(k_blocks, split);
-    // all of them resident, two on an SM; clusters do not find place on every SM (300 x 4096 x 4096 in 288 CTAs: 30.5 us, in 192: 22.7)
-    const long long ctas = m128 * n128 * split;
-    if (ctas * 100 > 2LL * sms * 87 || per < 4 || per * (split - 1) >= k_blocks || n128 > 65535) continue;
-    consider(kLargeSplit, split, ctas <= sms ? 6.5 + per * 0.45 : 9.0 + per * 0.47);
-  }
+  consider(kLargeNarrow, narrow);
+  if (N > 128) consider(kLargeWide, wide);
+  consider(kLargePair, pair);
   return best;
 }
 
@@ -996,7 +993,7 @@ int gemm_bf16_prepare() {
   if ((rc = prepare_skinny<32, true, true>())) return rc;
   if ((rc = prepare_skinny<64, true, true>())) return rc;
   if ((rc = prepare_skinny<128, true, true>())) return rc;
-  return prepare_skinny<128, false, false, true>();
+  return gemm_bf16_split_prepare();
 }
 
 bool gemm_bf16_uses_2cta(int M, int N) {
@@ -1029,6 +1026,13 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
     return gemm_rows(g, stream);
   }
 
+  const int sms = sm_count();
+  LargeChoice large{};
+  if (!w_is_kn && !push && (M > kSwapMaxM || !w_early)) {
+    const SplitChoice split = gemm_bf16_split_choose(M, N, K, sms);
+    if (M > kSwapMaxM) large = choose_large(M, N, ceil_div(K, kBK), sms);
+    if (split.bn && (M <= kSwapMaxM || split.us < large.us)) return gemm_bf16_split(x, ldx, w, ldw, bias, y, ldy, M, N, K, split.bn, split.split, swiglu, stream);
+  }
   GemmArgs a{};
   a.M = M; a.N = N; a.K = K; a.ldy = ldy; a.y = y; a.y32 = y32; a.bias = bias;
   a.k_blocks = ceil_div(K, kBK);
@@ -1050,13 +1054,11 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
   }
   a.err = device_error_word();
   if (!a.err) return TEENY_ERR_DRIVER;  // kernels report expired waits through this word: no launch without it
-  const int sms = sm_count();
 
   CUtensorMap tmx, tmw;
-  const LargeChoice large = (w_is_kn || M <= kSwapMaxM) ? LargeChoice{} : choose_large(M, N, a.k_blocks, sms);
   // Enough 256 x 256 tiles for the SM pairs: the CTA-pair kernel.
   if (large.kind == kLargePair) return gemm_bf16_2cta(x, ldx, w, ldw, bias, y, ldy, M, N, K, stream, swiglu);
-  const bool swap = !w_is_kn && (M <= kSwapMaxM || large.kind == kLargeSplit);
+  const bool swap = !w_is_kn && M <= kSwapMaxM;
   int bn;
   if (swap) {
     bn = swap_bn(M);
@@ -1090,13 +1092,12 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
 
   if (swap) {
     const int tiles = ceil_div(N, kBM);
-    if ((tiles < 4 * sms || swiglu || push || large.split) && tiles <= 65535) {
+    if ((tiles < 4 * sms || swiglu || push) && tiles <= 65535) {
       // Few weight tiles: cluster split-K.  Measured on B200 (batch 32, K = 4096 / 12288): the kernel is fastest
       // when all its CTAs are resident at once (two per SM) and share HBM evenly -- about 0.85 of the slots -- and a
       // wider cluster than that only adds barrier and reduction cost; with at least as many tiles as SMs no split.
-      const int split = large.split ? large.split : skinny_split(tiles, a.k_blocks, sms);
+      const int split = skinny_split(tiles, a.k_blocks, sms);
       a.w_early = w_early;
-      if (large.split) a.l2_ahead = -1;
       a.kb_per_split = ceil_div(a.k_blocks, split);
       {  // what the CTAs ask into L2 ahead of time must stay well inside it (126 MB): at most 48 MB over the grid
         const long long per_cta = (48ll << 20) / (static_cast<long long>(kBM * kBK * 2) * split * tiles);
@@ -1106,9 +1107,7 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
         case 16: return launch_skinny<16>(tmw, tmx, a, split, tiles, stream);
         case 32: return launch_skinny<32>(tmw, tmx, a, split, tiles, stream);
         case 64: return launch_skinny<64>(tmw, tmx, a, split, tiles, stream);
-        default:
-          if (large.split) return launch_skinny<128, false, false, true>(tmw, tmx, a, split, tiles, stream, ceil_div(M, bn));
-          return launch_skinny<128>(tmw, tmx, a, split, tiles, stream);
+        default: return launch_skinny<128>(tmw, tmx, a, split, tiles, stream);
       }
     }
     a.tiles_p = tiles;

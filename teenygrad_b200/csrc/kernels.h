@@ -142,6 +142,13 @@ struct QkvEpilogue {
 int gemm_bf16_2cta_prepare();
 int gemm_bf16_2cta(const bf16* x, int ldx, const bf16* w, int ldw, const bf16* bias, bf16* y, int ldy, int M, int N,
                    int K, cudaStream_t stream, int swiglu = 0, const QkvEpilogue* qkv = nullptr);
+// Few tiles, K of a tile of 128 weight rows x bn (32, 64, 128, 192, 256) tokens over a cluster of `split` CTAs (gemm_bf16_split.cu); for operators
+// and prefills.  The choice: bn 0 where no split leaves all CTAs resident at once; us is estimated.
+struct SplitChoice { int bn, split; double us; };
+SplitChoice gemm_bf16_split_choose(int M, int N, int K, int sms);
+int gemm_bf16_split_prepare();
+int gemm_bf16_split(const bf16* x, int ldx, const bf16* w, int ldw, const bf16* bias, bf16* y, int ldy, int M, int N, int K, int bn, int split,
+                    int glu, cudaStream_t st);
 // Whether gemm_bf16 hands an [M, N] problem to the CTA-pair kernel (enough 256 x 256 tiles for every SM pair).
 bool gemm_bf16_uses_2cta(int M, int N);
 // C[M, N] = A[M, K] B[K, N], all f32 row-major and contiguous, on the tensor cores at f32 accuracy: each operand is

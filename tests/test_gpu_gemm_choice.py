@@ -34,3 +34,24 @@ def test_swiglu_any_kernel(M, C, K):
     # the projections, silu and the product are bf16 tensors: four roundings
     assert float(((y.double() - ref).abs() / (ref.abs() * 2 ** -6 + 2e-2 * ref.pow(2).mean().sqrt())).max()) <= 1.0
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 136, 520), (33, 8, 4096), (64, 1000, 72), (65, 129, 8200), (128, 520, 8200), (100, 4096, 1000), (31, 12288, 512), (127, 700, 136),
+                                   (16, 640, 11160), (190, 2000, 1032), (257, 3000, 4104), (385, 6144, 1024), (193, 8200, 512)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_resident_tiles_and_their_clusters(M, N, K, pad):
+    """K of few tiles over clusters of one to eight CTAs, 32 to 256 tokens wide: ragged tokens, weight rows and k, rows of Y that take 8-byte stores and
+    rows that do not."""
+    from teenygrad_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g, device="cuda").bfloat16()
+    out = torch.full((M, N + pad), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.linear_forward(x, w, b, out=out[:, :N])
+    ref = x.double() @ w.double().t() + b.double()
+    assert float(((out[:, :N].double() - ref).abs() / (ref.abs() * 2 ** -8 + 1e-3 * ref.pow(2).mean().sqrt())).max()) <= 1.0
+    assert bool((out[:, N:] == 7.0).all()) and ops.device_error() == 0
+    again = torch.empty_like(out)
+    ops.linear_forward(x, w, b, out=again[:, :N])
+    assert torch.equal(out[:, :N], again[:, :N])
