@@ -26,7 +26,7 @@ namespace teeny {
 namespace {
 
 constexpr int kBM = 128, kBK = 64, kEpiWarps = 8, kThreads = 32 * (2 + kEpiWarps), kEpi = 32 * kEpiWarps;
-constexpr int kMaxStages = 8, kSmem = 226 << 10;
+constexpr int kMaxStages = 8, kSmem = 226 << 10, kSmemTwo = 112 << 10;
 
 template <int BN> struct Cfg {
   static constexpr int kP = kBM * kBK * 2, kQ = BN * kBK * 2, kStage = kP + kQ;
@@ -310,11 +310,14 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, SplitArgs g, int split,
   const int rc = prepare<BN>();
   if (rc) return rc;
   g.cw = (BN + split - 1) / split;
-  const int sent = (split - 1) * g.cw * (kBM * 4), room = (kSmem - 1024 - sent) / C::kStage;
+  const int sent = (split - 1) * g.cw * (kBM * 4);
+  // more tiles than SMs: two CTAs on an SM
+  const long long ctas = static_cast<long long>((g.N + kBM - 1) / kBM) * ((g.M + BN - 1) / BN) * split;
+  const int most = split == 1 && ctas > sm_count() ? kSmemTwo : kSmem, room = (most - 1024 - sent) / C::kStage;
   g.stages = g.per < kMaxStages ? g.per : kMaxStages;
   if (g.stages > room) g.stages = room;
   g.ring = g.stages * C::kStage > C::kPart ? g.stages * C::kStage : C::kPart;
-  if (g.stages < 1 || 1024 + g.ring + sent > kSmem) return TEENY_ERR_BAD_ARG;
+  if (g.stages < 1 || 1024 + g.ring + sent > most) return TEENY_ERR_BAD_ARG;
   return launch_kernel(gemm_bf16_split_kernel<BN>, dim3(split, (g.N + kBM - 1) / kBM, (g.M + BN - 1) / BN), dim3(kThreads), 1024 + g.ring + sent, st,
                        static_cast<unsigned>(split), tw, tx, g);
 }
@@ -323,29 +326,29 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, SplitArgs g, int split,
 
 // Microseconds of K over `split` CTAs of 128 x bn tiles, which are all resident at once (0: they would not be): a start and an end, and the blocks of a
 // CTA, each what its MMAs take to issue, its bytes at the rate of one SM, or all CTAs' bytes at the rate of L2 -- which are lower where rows do not start on
-// 128 bytes: a row of a tile is then two lines.  Fitted to 796 calls with 16 to 2000 tokens (11 % off in the mean; the best of a size's choices is missed by 1.2 %).
-double gemm_bf16_split_us(int M, int N, int K, int bn, int split, int sms) {
-  // clusters of 1 to 8 CTAs, one on an SM, that a B200 holds at once (cudaOccupancyMaxActiveClusters)
-  constexpr int kResident[8] = {148, 74, 45, 33, 26, 22, 15, 15};
+// 128 bytes (`lines`): a row of a tile is then two lines.  Fitted to calls with 16 to 2000 tokens (12 % off in the mean; what is taken is 1.8 % slower than the best of
+// a size's choices).
+double gemm_bf16_split_us(int M, int N, int K, bool lines, int bn, int split, int sms) {
+  // clusters of 1 to 8 CTAs, one on an SM, that a B200 holds at once (cudaOccupancyMaxActiveClusters); single CTAs also two on an SM
+  constexpr int kResident[8] = {296, 74, 45, 33, 26, 22, 15, 15};
   const int blocks = (K + kBK - 1) / kBK, per = (blocks + split - 1) / split;
   const long long tiles = static_cast<long long>((N + kBM - 1) / kBM) * ((M + bn - 1) / bn);
   if (tiles * 148 > static_cast<long long>(kResident[split - 1]) * sms || per * (split - 1) >= blocks || (split > 1 && per < 2)) return 0.0;
-  const double kb = kBK * 2.0 * (kBM + bn), narrow = bn / 128.0;  // bytes of a block
-  const bool lines = K % 64 == 0;
-  const double issue = bn <= 128 ? 0.128 : (bn == 192 ? 0.236 : 0.367), sm = kb / (lines ? 181e3 : 106e3), all = kb * tiles * split / (lines ? 16.4e6 : 10.6e6);
+  if (bn == 256 && (split > 2 || tiles * split > sms)) return 0.0;  // (shared memory for less than three blocks)
+  const double kb = kBK * 2.0 * (kBM + bn), narrow = bn / 128.0, ctas = static_cast<double>(tiles) * split, per_sm = ctas > sms ? ctas / sms : 1.0;
+  const double issue = bn <= 128 ? 0.09 : (bn == 192 ? 0.21 : 0.32), sm = kb * per_sm / (lines ? 196e3 : 97e3), all = kb * ctas / (lines ? 17.0e6 : 11.1e6);
   const double block = std::pow(std::pow(issue, 6) + std::pow(sm, 6) + std::pow(all, 6), 1.0 / 6);
-  const double end = 2.2 + 0.83 * narrow + (split > 1 ? 2.7 * narrow * (split - 1) / split : 0.0);
-  const double hbm = 2.0 * (static_cast<double>(N) * K + static_cast<double>(M) * K + static_cast<double>(M) * N) / 6.0e6;
-  return 0.9 + end + (per * block > hbm ? per * block : hbm);
+  const double ends = 2.26 + 0.75 * narrow + (split > 1 ? 2.58 * narrow * (split - 1) / split : 0.0);
+  const double hbm = 2.0 * (static_cast<double>(N) * K + static_cast<double>(M) * K + static_cast<double>(M) * N) / 7.8e6;
+  return 0.9 + ends * (per_sm > 1.0 ? (bn > 128 ? 1.8 : 1.43) : 1.0) + std::cbrt(std::pow(per * block, 3) + std::pow(hbm, 3));
 }
 
-SplitChoice gemm_bf16_split_choose(int M, int N, int K, int sms) {
+SplitChoice gemm_bf16_split_choose(int M, int N, int K, bool lines, int sms) {
   SplitChoice best{};
   for (int bn : {32, 64, 128, 192, 256}) {
     if (bn >= 192 && M <= 128) break;
     for (int split = 1; split <= (bn >= 192 ? 4 : 8); ++split) {
-      if (bn == 256 && split > 3) break;  // (shared memory)
-      const double us = gemm_bf16_split_us(M, N, K, bn, split, sms);
+      const double us = gemm_bf16_split_us(M, N, K, lines, bn, split, sms);
       if (us > 0.0 && (!best.bn || us < best.us)) best = SplitChoice{bn, split, us};
     }
   }

@@ -145,7 +145,7 @@ int gemm_bf16_2cta(const bf16* x, int ldx, const bf16* w, int ldw, const bf16* b
 // Few tiles, K of a tile of 128 weight rows x bn (32, 64, 128, 192, 256) tokens over a cluster of `split` CTAs (gemm_bf16_split.cu); for operators
 // and prefills.  The choice: bn 0 where no split leaves all CTAs resident at once; us is estimated.
 struct SplitChoice { int bn, split; double us; };
-SplitChoice gemm_bf16_split_choose(int M, int N, int K, int sms);
+SplitChoice gemm_bf16_split_choose(int M, int N, int K, bool lines, int sms);  // lines: rows of X and W start on 128 bytes
 int gemm_bf16_split_prepare();
 int gemm_bf16_split(const bf16* x, int ldx, const bf16* w, int ldw, const bf16* bias, bf16* y, int ldy, int M, int N, int K, int bn, int split,
                     int glu, cudaStream_t st);
