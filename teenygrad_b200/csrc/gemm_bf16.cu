@@ -25,6 +25,7 @@
 // bit-reproducible.  No global scratch, no atomics.
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -141,15 +142,6 @@ __device__ __forceinline__ void umma_bf16_ts_x4(uint32_t d_tmem, uint32_t a_tmem
       "add.u32 a, %1, 24;\n\t add.u64 b, %2, %7;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "n"(B_STEP), "n"(2 * B_STEP), "n"(3 * B_STEP)
       : "memory");
-}
-
-// One k-block of MMAs: four K=16 steps over the 64-wide stage.
-template <int BN, bool Q_MN_MAJOR>
-__device__ __forceinline__ void issue_kblock(uint32_t d_tmem, uint32_t sp, uint32_t sq, bool first) {
-  constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, Q_MN_MAJOR);
-  const uint64_t pdesc = make_smem_desc_sw128(sp, 16, 1024);
-  const uint64_t qdesc = Q_MN_MAJOR ? make_smem_desc_sw128(sq, kBK * 128, 1024) : make_smem_desc_sw128(sq, 16, 1024);
-  umma_bf16_ss_x4<2, Q_MN_MAJOR ? 128 : 2>(d_tmem, pdesc, qdesc, idesc, first ? 0u : 1u);
 }
 
 template <int BN, bool SWAP, bool Q_MN_MAJOR>
@@ -426,8 +418,11 @@ struct SkinnyCfg {
   static constexpr int kStageBytes = kStageP + kStageQ;
   // As many stages as let two CTAs share an SM (about 100 KB each): what streams the weights fast is the number of
   // bytes in flight per SM, and two short-lived CTAs overlap each other's set-up and reduction.
+  // Up to 32 tokens the partial sums are sent into a place behind the ring (kReceive); wider tiles leave no room for it.
+  static constexpr bool kSend = BN <= 32;
+  static constexpr int kReceive = BN == 16 ? 9216 : (BN == 32 ? 15360 : 0);  // (S - 1) ceil(BN / S) columns of 512 bytes, the most of S = 2 .. 8
   static constexpr int kStages = W8 ? (BN <= 16 ? 5 : (BN <= 32 ? 4 : (BN <= 64 ? 3 : 2)))
-                                    : ((BN <= 32) ? 5 : (BN <= 64 ? 4 : 3));
+                                    : (BN <= 16 ? 5 : (BN <= 64 ? 4 : 3));
   static constexpr int kPartialBytes = BN * kBM * 4;  // f32 partial tile, column-major [BN][128]; reuses the ring
   static_assert(kPartialBytes <= kStages * kStageBytes, "partial tile must fit in the stage ring");
   // W8: 64 k of 128 weight rows as bf16 pairs are 32 columns of tensor memory; four such tiles behind the accumulator
@@ -449,8 +444,9 @@ struct SkinnyCfg {
   static_assert(F8 || (kTmemA + kABufs * 32 <= 256 && kAccCols <= kTmemA && (kIssuers == 1 || kAcc1 + kAccCols <= kTmemA)),
                 "accumulators and weight tiles share the allocation");
   static_assert(!F8 || kAcc1 + kAccCols <= kTmemCols, "two accumulators share the allocation");
-  static constexpr int kBarOffset = kStages * kStageBytes;
+  static constexpr int kBarOffset = kStages * kStageBytes + kReceive;
   static constexpr int kSmemBytes = kBarOffset + 1024 + 256;
+  static_assert(!kSend || 2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs on an SM");
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -465,6 +461,20 @@ __device__ __forceinline__ uint32_t cluster_size() {
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// An arrival that orders nothing (a releasing one waits for what the thread has under way, 1000 clocks): for barriers whose initialisation has
+// its own fence, and for bulk copies that a barrier has counted.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+// shared memory -> another CTA's (dst and bar are its addresses); its barrier counts the bytes
+__device__ __forceinline__ void send_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
 }
 // 16 bytes of CTA `rank`'s shared memory at this CTA's address `local_addr`.  Volatile (so it stays behind the cluster
 // barrier, itself a volatile asm) but without a memory clobber: consecutive loads are all in flight together.
@@ -495,6 +505,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const uint32_t tmem_slot = acc_full_bar + 8;
   auto wfull_bar = [&](int b) { return acc_full_bar + 16u + 8u * b; };   // W8: weight tile b is in tensor memory
   auto wempty_bar = [&](int b) { return acc_full_bar + 48u + 8u * b; };  // W8: the MMAs that read tile b are done
+  const uint32_t received_bar = acc_full_bar + 80u;                      // kSend: the other CTAs' sums of this one's columns are here
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   float* part_gen = reinterpret_cast<float*>(smem_gen);
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(
@@ -525,6 +536,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       mbar_init(empty_bar(s), Cfg::kIssuers + Cfg::kConvWarps);
     }
     mbar_init(acc_full_bar, Cfg::kIssuers);
+    if constexpr (Cfg::kSend) mbar_init(received_bar, 1);
     if constexpr (W8 && !F8) {
       for (int b = 0; b < Cfg::kABufs; ++b) {
         mbar_init(wfull_bar(b), Cfg::kConvWarps / 2);  // a tile is written by one group of four warps
@@ -537,99 +549,105 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
+  // CTA q of the cluster finishes the token columns [q cw, (q + 1) cw)
+  const int cw = (BN + static_cast<int>(S) - 1) / static_cast<int>(S);
+  auto first_column = [&](int q) { return min(BN, q * cw); };
+  const int c_begin = first_column(static_cast<int>(rank)), ncols = first_column(static_cast<int>(rank) + 1) - c_begin;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  if constexpr (Cfg::kSend) {
+    if (S > 1) {
+      if (threadIdx.x == 0) mbar_expect_tx(received_bar, (S - 1) * ncols * (kBM * 4));
+      __syncwarp();
+      cluster_arrive_relaxed();  // this CTA's barriers exist
+    }
+  }
 
+  // The loops that issue are walked by whole warps and one lane issues (see gemm_bf16_kernel).
+  const bool one = elect_one();
   if (warp == 0) {
-    if (lane == 0) {
+    {
       // A model's weights are not written by any kernel of its steps (w_early), so the first ring of weight tiles is requested
       // while the previous kernel may still be running; the activation tiles follow once it has finished.  Weights that
       // the kernel in front may be writing (an operator's, a prefill's converted copy) are only asked into L2, where its
       // stores arrive, too.
       const int ring = min(kb1 - kb0, Cfg::kStages), pre = args.w_early ? ring : 0;
       for (int i = 0; i < pre; ++i) {
+        if (!one) continue;
         mbar_expect_tx(full_bar(i), Cfg::kStageBytes);
         tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, full_bar(i), (kb0 + i) * Cfg::kKB, tile * kBM);
       }
       // ... and the weight tiles behind them are asked into L2, so that HBM keeps streaming this kernel's weights for
       // as long as the predecessor's tail lasts, not just until the ring is full
       for (int kb = kb0 + pre; kb < min(kb1, kb0 + (args.l2_ahead < 0 ? 0 : ring + args.l2_ahead)); ++kb)
-        tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
+        if (one) tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
       pdl_wait();
       auto load_x = [&](uint32_t sq, uint32_t bar, int kb) {  // the activation tile(s) of one stage: 64 k each
         tma_load_2d(sq, &tmap_x, bar, kb * Cfg::kKB, 0);
         if constexpr (F8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB, args.x_lo_row);  // the lo terms
         else if constexpr (W8) tma_load_2d(sq + BN * kBK * 2, &tmap_x, bar, kb * Cfg::kKB + kBK, 0);
       };
-      for (int i = 0; i < pre; ++i) load_x(smem_base + i * Cfg::kStageBytes + Cfg::kStageP, full_bar(i), kb0 + i);
+      for (int i = 0; i < pre; ++i)
+        if (one) load_x(smem_base + i * Cfg::kStageBytes + Cfg::kStageP, full_bar(i), kb0 + i);
       int stage = pre == Cfg::kStages ? 0 : pre;
       uint32_t phase = pre == Cfg::kStages ? 1 : 0;
       for (int kb = kb0 + pre; kb < kb1; ++kb) {
         if (!mbar_wait(empty_bar(stage), phase ^ 1, err, DEVERR_GEMM_PRODUCER)) break;
         const uint32_t sp = smem_base + stage * Cfg::kStageBytes;
-        mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
-        tma_load_2d(sp, &tmap_w, full_bar(stage), kb * Cfg::kKB, tile * kBM);
-        load_x(sp + Cfg::kStageP, full_bar(stage), kb);
+        if (one) {
+          mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
+          tma_load_2d(sp, &tmap_w, full_bar(stage), kb * Cfg::kKB, tile * kBM);
+          load_x(sp + Cfg::kStageP, full_bar(stage), kb);
+        }
         if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
-    } else {
-      pdl_wait();
     }
   } else if (warp == 1 || (Cfg::kIssuers == 2 && warp == 2 + Cfg::kConvWarps)) {
     pdl_wait();
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      TRACE_ONLY(long long m_full = 0, m_wfull = 0, m_issue = 0, c0; const long long m_begin = clock64();)
-      // W8 with two issuers: warp 1 takes half 0 of every stage into the first accumulator, the other MMA warp half 1
-      // into the second
-      const int h_first = (W8 && warp != 1) ? 1 : 0, h_step = Cfg::kIssuers;
-      const uint32_t acc = tmem_base + ((W8 && warp != 1) ? Cfg::kAcc1 : 0);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        TRACE_ONLY(c0 = clock64();)
-        if (!mbar_wait(full_bar(stage), phase, err, DEVERR_GEMM_MMA)) { ok = false; break; }
-        TRACE_ONLY(m_full += clock64() - c0;)
-        const uint32_t sp = smem_base + stage * Cfg::kStageBytes;
-        if constexpr (F8) {
-          tc_fence_after();
-          constexpr uint32_t idesc = make_idesc_e4m3(kBM, BN);
-          const uint64_t wdesc = make_smem_desc_sw128(sp, 16, 1024);
-          const uint64_t hdesc = make_smem_desc_sw128(sp + Cfg::kStageP, 16, 1024);
-          const uint64_t ldesc = make_smem_desc_sw128(sp + Cfg::kStageP + BN * kBK * 2, 16, 1024);
-          // 128 k of the stage = four K = 32 steps of 32 bytes (+2 in both address fields); hi products, then lo
-          umma_f8_ss_x4(tmem_base, wdesc, hdesc, idesc, kb == kb0 ? 0u : 1u);
-          umma_f8_ss_x4(tmem_base + Cfg::kAcc1, wdesc, ldesc, idesc, kb == kb0 ? 0u : 1u);
-        } else if constexpr (W8) {
-          for (int h = h_first; h < 2; h += h_step) {
-            const int q = 2 * (kb - kb0) + h, j = q & 3;  // the q-th 64-k block goes through weight tile q % 4
-            TRACE_ONLY(c0 = clock64();)
-            if (!mbar_wait(wfull_bar(j), (q >> 2) & 1, err, DEVERR_GEMM_MMA)) { ok = false; break; }
-            TRACE_ONLY(m_wfull += clock64() - c0; c0 = clock64();)
-            tc_fence_after();
-            constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, false);
-            const uint64_t xdesc = make_smem_desc_sw128(sp + Cfg::kStageP + h * BN * kBK * 2, 16, 1024);
-            const uint32_t a_tmem = tmem_base + Cfg::kTmemA + j * 32;
-            umma_bf16_ts_x4<2>(acc, a_tmem, xdesc, idesc, q >= h_step ? 1u : 0u);  // an issuer's first block overwrites
-            umma_commit(wempty_bar(j));
-            TRACE_ONLY(m_issue += clock64() - c0;)
-          }
-          if (!ok) break;
-        } else {
-          tc_fence_after();
-          issue_kblock<BN, false>(tmem_base, sp, sp + Cfg::kStageP, kb == kb0);
+    int stage = 0;
+    uint32_t phase = 0, off = 0;  // off: of the stage, in the descriptors' 16 bytes
+    bool ok = true;
+    // W8 with two issuers: warp 1 takes half 0 of every stage into the first accumulator, the other MMA warp half 1
+    // into the second
+    const int h_first = (W8 && warp != 1) ? 1 : 0, h_step = Cfg::kIssuers;
+    const uint32_t acc = tmem_base + ((W8 && warp != 1) ? Cfg::kAcc1 : 0);
+    const uint64_t wdesc = make_smem_desc_sw128(smem_base, 16, 1024), xdesc = make_smem_desc_sw128(smem_base + Cfg::kStageP, 16, 1024);
+    constexpr uint64_t kHalf = BN * kBK * 2 / 16;  // W8: from a stage's first activation tile to its second
+    bool ready = kb0 < kb1 && mbar_try_wait(full_bar(0), 0);  // asked a block ahead
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!ready && !mbar_wait(full_bar(stage), phase, err, DEVERR_GEMM_MMA)) { ok = false; break; }
+      if constexpr (F8) {
+        tc_fence_after();
+        constexpr uint32_t idesc = make_idesc_e4m3(kBM, BN);
+        // 128 k of the stage = four K = 32 steps of 32 bytes (+2 in both address fields); hi products, then lo
+        if (one) {
+          umma_f8_ss_x4(tmem_base, wdesc + off, xdesc + off, idesc, kb == kb0 ? 0u : 1u);
+          umma_f8_ss_x4(tmem_base + Cfg::kAcc1, wdesc + off, xdesc + off + kHalf, idesc, kb == kb0 ? 0u : 1u);
         }
-        umma_commit(empty_bar(stage));
-        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+      } else if constexpr (W8) {
+        for (int h = h_first; h < 2; h += h_step) {
+          const int q = 2 * (kb - kb0) + h, j = q & 3;  // the q-th 64-k block goes through weight tile q % 4
+          if (!mbar_wait(wfull_bar(j), (q >> 2) & 1, err, DEVERR_GEMM_MMA)) { ok = false; break; }
+          tc_fence_after();
+          constexpr uint32_t idesc = make_idesc_bf16(kBM, BN, false, false);
+          if (one) {
+            umma_bf16_ts_x4<2>(acc, tmem_base + Cfg::kTmemA + j * 32, xdesc + off + h * kHalf, idesc, q >= h_step ? 1u : 0u);  // an issuer's first block overwrites
+            umma_commit(wempty_bar(j));
+          }
+        }
+        if (!ok) break;
+      } else {
+        tc_fence_after();
+        if (one) umma_bf16_ss_x4<2, 2>(tmem_base, wdesc + off, xdesc + off, make_idesc_bf16(kBM, BN, false, false), kb == kb0 ? 0u : 1u);
       }
-      if (ok) umma_commit(acc_full_bar);
-      TRACE_VALUE(0, W8 && blockIdx.y == 0 && warp == 1, clock64() - m_begin);
-      TRACE_VALUE(1, W8 && blockIdx.y == 0 && warp == 1, m_full);
-      TRACE_VALUE(2, W8 && blockIdx.y == 0 && warp == 1, m_wfull);
-      TRACE_VALUE(3, W8 && blockIdx.y == 0 && warp == 1, m_issue);
+      if (one) umma_commit(empty_bar(stage));
+      off += Cfg::kStageBytes / 16;
+      if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; off = 0; }
+      ready = kb + 1 < kb1 && mbar_try_wait(full_bar(stage), phase);
     }
+    if (ok && one) umma_commit(acc_full_bar);
   } else {
     pdl_wait();
     if constexpr (W8 && !F8) {
@@ -754,6 +772,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         }
       }
       tc_fence_before();
+      if constexpr (Cfg::kSend) fence_proxy_async_smem();  // (the tile is sent by bulk copies)
     }
   }
 
@@ -761,31 +780,59 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   pdl_trigger();  // main loop done: the next kernel's set-up (and weight prefetch) overlaps the reduction below
   const bool reduce = (S > 1) || args.swiglu;
   // every partial tile of the cluster is in place
-  if (S > 1) cluster_sync_all(); else if (reduce) __syncthreads();
+  if constexpr (Cfg::kSend) {
+    if (S > 1) cluster_wait();  // (of the arrival at the start)
+    if (reduce) __syncthreads();
+  } else {
+    if (S > 1) cluster_sync_all(); else if (reduce) __syncthreads();
+  }
   TRACE_MARK(2, threadIdx.x == 64);
 
-  if (warp >= 2 && warp < 6 && reduce) {
-    // CTA `rank` finishes token columns [rank * cw, (rank + 1) * cw): per 16-byte unit (4 weight rows of one token
-    // column) all S partial values are requested at once and summed in rank order
-    const int cw = (BN + static_cast<int>(S) - 1) / static_cast<int>(S);  // columns per rank (last rank may get fewer)
-    const int c_begin = static_cast<int>(rank) * cw;
-    const int ncols = min(BN, c_begin + cw) - c_begin;
+  bool arrived = true;
+  if constexpr (Cfg::kSend) {
+    if (S > 1 && warp >= 2 && warp < 6) {
+      const int q = lane;
+      if (warp == 2 && q < static_cast<int>(S) && q != static_cast<int>(rank) && *reinterpret_cast<volatile int*>(err) == 0) {
+        // each other CTA gets the columns that it finishes, by one bulk copy (remote loads bring 6 to 10 bytes a clock)
+        const int from = first_column(q), bytes = (first_column(q + 1) - from) * (kBM * 4), slot = static_cast<int>(rank) - (static_cast<int>(rank) > q);
+        if (bytes > 0)
+          send_bulk(map_rank(smem_base + Cfg::kStages * Cfg::kStageBytes + slot * bytes, q), part_base + from * (kBM * 4), bytes, map_rank(received_bar, q));
+      }
+      if (ncols > 0) arrived = mbar_wait(received_bar, 0, err, DEVERR_GEMM_EPILOGUE);
+    }
+    __syncwarp();
+    if (S > 1) cluster_arrive_relaxed();  // what was sent here has arrived
+  }
+  // This CTA's token columns: per 16-byte unit (4 weight rows of one token column) all parts are requested at once and summed in rank order.
+  // `width` is the cluster's, a constant where the parts lie in this CTA's shared memory.
+  auto finish = [&](auto width) {
+    const int parts = decltype(width)::value ? decltype(width)::value : static_cast<int>(S);
     const int epi = (warp - 2) * 32 + lane;
+    auto part_of = [&](int q, uint32_t off) -> float4 {  // off: bytes from the first of this CTA's columns
+      if constexpr (Cfg::kSend) {
+        const uint32_t at = q == static_cast<int>(rank) ? c_begin * (kBM * 4)
+                                                        : Cfg::kStages * Cfg::kStageBytes + (q - (q > static_cast<int>(rank))) * ncols * (kBM * 4);
+        return *reinterpret_cast<const float4*>(smem_gen + at + off);
+      } else {
+        return ld_cluster_f32x4(part_base + c_begin * (kBM * 4) + off, q);
+      }
+    };
     if (args.swiglu) {
       // the tile holds 64 gate rows then the 64 up rows of the same channels: a unit = 4 channels of one column
       const bool vec_ok = (args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(y) & 7) == 0);
       for (int u = epi; u < ncols * 16; u += kEpilogueThreads) {
         const int c = c_begin + (u >> 4), j = u & 15;
-        const uint32_t ga = part_base + static_cast<uint32_t>((c * kBM + 4 * j) * 4);
+        const uint32_t ga = static_cast<uint32_t>(((c - c_begin) * kBM + 4 * j) * 4);
         float4 gv[8], uv[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          gv[q] = (static_cast<uint32_t>(q) < S) ? ld_cluster_f32x4(ga, q) : make_float4(0.f, 0.f, 0.f, 0.f);
-          uv[q] = (static_cast<uint32_t>(q) < S) ? ld_cluster_f32x4(ga + 64 * 4, q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          gv[q] = q < parts ? part_of(q, ga) : make_float4(0.f, 0.f, 0.f, 0.f);
+          uv[q] = q < parts ? part_of(q, ga + 64 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         float4 gs = gv[0], us = uv[0];
 #pragma unroll
         for (int q = 1; q < 8; ++q) {
+          if (q >= parts) break;
           gs.x += gv[q].x; gs.y += gv[q].y; gs.z += gv[q].z; gs.w += gv[q].w;
           us.x += uv[q].x; us.y += uv[q].y; us.z += uv[q].z; us.w += uv[q].w;
         }
@@ -813,14 +860,14 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       const unsigned stamp = args.push_recv ? __ldcg(args.push_epoch) * 1024u + args.push_round + 1u : 0u;
       for (int u = epi; u < ncols * 32; u += kEpilogueThreads) {
         const int c = c_begin + (u >> 5), j = u & 31;
-        const uint32_t addr = part_base + static_cast<uint32_t>((c * kBM + 4 * j) * 4);
+        const uint32_t addr = static_cast<uint32_t>(((c - c_begin) * kBM + 4 * j) * 4);
         float4 v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-          v[q] = (static_cast<uint32_t>(q) < S) ? ld_cluster_f32x4(addr, q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[q] = q < parts ? part_of(q, addr) : make_float4(0.f, 0.f, 0.f, 0.f);
         float4 acc = v[0];
 #pragma unroll
-        for (int q = 1; q < 8; ++q) { acc.x += v[q].x; acc.y += v[q].y; acc.z += v[q].z; acc.w += v[q].w; }
+        for (int q = 1; q < 8; ++q) if (q < parts) { acc.x += v[q].x; acc.y += v[q].y; acc.z += v[q].z; acc.w += v[q].w; }
         const int n = tile * kBM + 4 * j;
         if (c < rows && n < args.N) {
           float o[4] = {acc.x, acc.y, acc.z, acc.w};
@@ -859,12 +906,33 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         }
       }
     }
+  };
+  if (warp >= 2 && warp < 6 && reduce && arrived) {
+    if constexpr (Cfg::kSend) {
+      switch (S) {
+        case 1: finish(std::integral_constant<int, 1>{}); break;
+        case 2: finish(std::integral_constant<int, 2>{}); break;
+        case 3: finish(std::integral_constant<int, 3>{}); break;
+        case 4: finish(std::integral_constant<int, 4>{}); break;
+        case 5: finish(std::integral_constant<int, 5>{}); break;
+        case 6: finish(std::integral_constant<int, 6>{}); break;
+        case 7: finish(std::integral_constant<int, 7>{}); break;
+        default: finish(std::integral_constant<int, 8>{}); break;
+      }
+    } else {
+      finish(std::integral_constant<int, 0>{});
+    }
   }
   TRACE_MARK(3, threadIdx.x == 64);
 
-  // nobody leaves (and frees its shared memory) while a peer may still be reading it
+  // nobody leaves (and frees its shared memory) while a peer may still be reading it, or what this CTA sent is on its way
   __syncwarp();
-  if (S > 1) cluster_sync_all(); else __syncthreads();
+  if constexpr (Cfg::kSend) {
+    if (S > 1) cluster_wait();
+    __syncthreads();
+  } else {
+    if (S > 1) cluster_sync_all(); else __syncthreads();
+  }
   if (warp == 2) {
     if (*reinterpret_cast<volatile int*>(err) != 0) {
       const uint64_t t0 = global_timer_ns();
