@@ -790,7 +790,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 
   bool arrived = true;
   if constexpr (Cfg::kSend) {
-    if (S > 1 && warp >= 2 && warp < 6) {
+    if (S > 1) {
       const int q = lane;
       if (warp == 2 && q < static_cast<int>(S) && q != static_cast<int>(rank) && *reinterpret_cast<volatile int*>(err) == 0) {
         // each other CTA gets the columns that it finishes, by one bulk copy (remote loads bring 6 to 10 bytes a clock)
@@ -799,6 +799,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           send_bulk(map_rank(smem_base + Cfg::kStages * Cfg::kStageBytes + slot * bytes, q), part_base + from * (kBM * 4), bytes, map_rank(received_bar, q));
       }
       if (ncols > 0) arrived = mbar_wait(received_bar, 0, err, DEVERR_GEMM_EPILOGUE);
+      TRACE_MARK(4, threadIdx.x == 64);
     }
     __syncwarp();
     if (S > 1) cluster_arrive_relaxed();  // what was sent here has arrived
@@ -807,7 +808,8 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   // `width` is the cluster's, a constant where the parts lie in this CTA's shared memory.
   auto finish = [&](auto width) {
     const int parts = decltype(width)::value ? decltype(width)::value : static_cast<int>(S);
-    const int epi = (warp - 2) * 32 + lane;
+    // kSend: all warps, the others have nothing left to do
+    const int epi = Cfg::kSend ? static_cast<int>(threadIdx.x) : (warp - 2) * 32 + lane, threads = Cfg::kSend ? Cfg::kThreads : kEpilogueThreads;
     auto part_of = [&](int q, uint32_t off) -> float4 {  // off: bytes from the first of this CTA's columns
       if constexpr (Cfg::kSend) {
         const uint32_t at = q == static_cast<int>(rank) ? c_begin * (kBM * 4)
@@ -820,7 +822,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     if (args.swiglu) {
       // the tile holds 64 gate rows then the 64 up rows of the same channels: a unit = 4 channels of one column
       const bool vec_ok = (args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(y) & 7) == 0);
-      for (int u = epi; u < ncols * 16; u += kEpilogueThreads) {
+      for (int u = epi; u < ncols * 16; u += threads) {
         const int c = c_begin + (u >> 4), j = u & 15;
         const uint32_t ga = static_cast<uint32_t>(((c - c_begin) * kBM + 4 * j) * 4);
         float4 gv[8], uv[8];
@@ -858,7 +860,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       const bool vec_ok = args.push_recv ? (args.N % 4 == 0)
                                          : ((args.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(y) & 7) == 0));
       const unsigned stamp = args.push_recv ? __ldcg(args.push_epoch) * 1024u + args.push_round + 1u : 0u;
-      for (int u = epi; u < ncols * 32; u += kEpilogueThreads) {
+      for (int u = epi; u < ncols * 32; u += threads) {
         const int c = c_begin + (u >> 5), j = u & 31;
         const uint32_t addr = static_cast<uint32_t>(((c - c_begin) * kBM + 4 * j) * 4);
         float4 v[8];
@@ -907,7 +909,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
     }
   };
-  if (warp >= 2 && warp < 6 && reduce && arrived) {
+  if ((Cfg::kSend || (warp >= 2 && warp < 6)) && reduce && arrived) {
     if constexpr (Cfg::kSend) {
       switch (S) {
         case 1: finish(std::integral_constant<int, 1>{}); break;
