@@ -178,44 +178,55 @@ split_e4m3_kernel(const bf16* __restrict__ x, long long ldx, uint8_t* __restrict
   }
 }
 
-// The same for rows of whole 16-byte pieces (K % 8 == 0, aligned): eight values per load, the row read twice (the
-// second pass comes out of L1), eight bytes per store.
-__global__ void __launch_bounds__(256)
+// The same for rows of whole 16-byte pieces (K % 8 == 0, aligned), by 1024 threads that hold up to two pieces each
+// between the maximum and the split (longer rows are read again).  Bound: latency, one CTA a row; it stands between two
+// GEMMs of a decode step (4096-wide FP8 model, batch 8: 527 us a step, with 256 threads that read the row twice 532).
+constexpr int kSplitThreads = 1024, kSplitHeld = 2;
+__global__ void __launch_bounds__(kSplitThreads)
 split_e4m3_vec_kernel(const bf16* __restrict__ x, long long ldx, uint8_t* __restrict__ out, long long ldo, float* __restrict__ scale,
                       int M, int K) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[8];
-  const int m = blockIdx.x;
+  __shared__ float red[kSplitThreads / 32];
+  const int m = blockIdx.x, tid = threadIdx.x;
   const uint4* row = reinterpret_cast<const uint4*>(x + m * ldx);
   const int chunks = K >> 3;
+  uint4 held[kSplitHeld];
+#pragma unroll
+  for (int i = 0; i < kSplitHeld; ++i) {
+    const int c = tid + i * kSplitThreads;
+    held[i] = c < chunks ? row[c] : make_uint4(0u, 0u, 0u, 0u);
+  }
   float amax = 0.0f;
-  for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const uint4 v = row[c];
+  auto largest = [&](const uint4 v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fmaxf(fabsf(bf16_lo(w[i])), fabsf(bf16_hi(w[i]))));
-  }
+  };
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  for (int i = 0; i < kSplitHeld; ++i) largest(held[i]);
+  for (int c = tid + kSplitHeld * kSplitThreads; c < chunks; c += kSplitThreads) largest(row[c]);
+  amax = warp_max(amax);
+  if ((tid & 31) == 0) red[tid >> 5] = amax;
   __syncthreads();
-  amax = red[0];
-  for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) amax = fmaxf(amax, red[w]);
+  amax = warp_max(red[tid & 31]);
   const int p = split_scale_exponent(amax);
   const float s = ldexpf(1.0f, p);
-  if (threadIdx.x == 0) scale[m] = ldexpf(1.0f, -p);
+  if (tid == 0) scale[m] = ldexpf(1.0f, -p);
   uint2* hi_row = reinterpret_cast<uint2*>(out + m * ldo);
   uint2* lo_row = reinterpret_cast<uint2*>(out + (static_cast<long long>(M) + m) * ldo);
-  for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-    const uint4 v = row[c];
+  auto store = [&](int c, const uint4 v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     unsigned short h[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) split_e4m3_pair(bf16_lo(w[i]) * s, bf16_hi(w[i]) * s, h[i], l[i]);
     hi_row[c] = make_uint2(h[0] | (static_cast<uint32_t>(h[1]) << 16), h[2] | (static_cast<uint32_t>(h[3]) << 16));
     lo_row[c] = make_uint2(l[0] | (static_cast<uint32_t>(l[1]) << 16), l[2] | (static_cast<uint32_t>(l[3]) << 16));
-  }
+  };
+#pragma unroll
+  for (int i = 0; i < kSplitHeld; ++i)
+    if (tid + i * kSplitThreads < chunks) store(tid + i * kSplitThreads, held[i]);
+  for (int c = tid + kSplitHeld * kSplitThreads; c < chunks; c += kSplitThreads) store(c, row[c]);
 }
 
 __global__ void __launch_bounds__(256) e4m3_count_nan_kernel(const uint8_t* __restrict__ p, size_t n, unsigned* count) {
@@ -260,7 +271,7 @@ int split_e4m3(const bf16* x, long long ldx, uint8_t* out, long long ldo, float*
   if (!x || !out || !scale || M <= 0 || K <= 0 || ldo < K) return TEENY_ERR_BAD_ARG;
   const bool vec = K % 8 == 0 && ldx % 8 == 0 && ldo % 8 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15) &&
                    !(reinterpret_cast<uintptr_t>(out) & 7);
-  if (vec) return launch_kernel(split_e4m3_vec_kernel, dim3(M), dim3(256), 0, st, 1, x, ldx, out, ldo, scale, M, K);
+  if (vec) return launch_kernel(split_e4m3_vec_kernel, dim3(M), dim3(kSplitThreads), 0, st, 1, x, ldx, out, ldo, scale, M, K);
   return launch_kernel(split_e4m3_kernel, dim3(M), dim3(256), 0, st, 1, x, ldx, out, ldo, scale, M, K);
 }
 

@@ -597,8 +597,10 @@ int run_layers(teeny_qwen3* m, int B, int S, int pos0, const int* pos_dev, const
     TEENY_TRY(sublayer_out(attn, w.o, Hq * D, true, false));
     TEENY_TRY(normed(w.post_ln, w.gate_up, mlp_rows, mlp8, act, 2 * I, kGluSilu));
     // (one GPU, FP8 down projection: its input as two-term FP8 costs a small kernel and saves the conversion of 50 M
-    // weight bytes next to the tensor core)
-    const bool down8 = down8_enabled() && wants_x8(m, w.down, T) && m->off.a8 != m->off.a8_scale &&
+    // weight bytes next to the tensor core.  With more than 16 rows the two terms' products take longer than the
+    // conversion: 4096-wide model, us a step with the split and without, batch 8 527, 541; 16 554, 563; 24 624, 618;
+    // 32 624, 607.)
+    const bool down8 = T <= 16 && down8_enabled() && wants_x8(m, w.down, T) && m->off.a8 != m->off.a8_scale &&
                        !(decode && rows_take(m, w.down, T, H, I));
     if (down8) TEENY_TRY(split_e4m3(act, I, m->at<uint8_t>(m->off.a8), I, m->at<float>(m->off.a8_scale), T, I, st));
     TEENY_TRY(sublayer_out(act, w.down, I, l + 1 < c.num_layers, down8));
