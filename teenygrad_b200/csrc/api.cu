@@ -108,6 +108,12 @@ int encode_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const u
                            strides_bytes, box);
 }
 
+int encode_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                          const uint64_t* strides_bytes, const uint32_t* box) {
+  return encode_tensor_map(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, CU_TENSOR_MAP_SWIZZLE_128B, base, rank, dims,
+                           strides_bytes, box);
+}
+
 // Bytes in the same 128-byte swizzle: the FP8 weight tiles that warps convert before the MMA reads them.
 int encode_tensor_map_u8(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                          const uint64_t* strides_bytes, const uint32_t* box) {

@@ -86,26 +86,6 @@ __device__ __forceinline__ void terms3(f32x2 v, uint32_t& hi, uint32_t& mid, uin
   lo = pack_bf16x2(q.x, q.y);
 }
 
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-
-// One MMA with constant offsets from the operands' first addresses (descriptors count 16 bytes), added where they are used: as variables of an
-// unrolled loop they are held in registers that the issuing warps do not have.
-template <int OA, int OB>
-__device__ __forceinline__ void umma_ss_at(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 x, y;\n\tadd.u64 x, %1, %5;\n\tadd.u64 y, %2, %6;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, p;\n\t}"
-               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "n"(OA), "n"(OB) : "memory");
-}
-template <int OA, int OB>
-__device__ __forceinline__ void umma_ts_at(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x;\n\t.reg .b64 y;\n\tadd.u32 x, %1, %5;\n\tadd.u64 y, %2, %6;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [x], y, %3, p;\n\t}"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "n"(OA), "n"(OB) : "memory");
-}
 template <typename F, int... I>
 __device__ __forceinline__ void each(std::integer_sequence<int, I...>, F f) { (f(std::integral_constant<int, I>{}), ...); }
 

@@ -259,20 +259,20 @@ int launch(const T* a, long long sam, long long sak, const T* b, long long sbk, 
 double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K) {
   double here;
   choose(M, N, K, sm_count(), here);
-  if (!gemm_f32_tc_takes(a, sam, sak, b, sbk, sbn, M, N, K)) return here;
-  const double there = gemm_f32_tc_clocks(sbk, M, N, K);
+  if (!gemm_f32_tc_takes(sak, sbk, sbn, M, N, K)) return here;
+  const double there = gemm_f32_tc_clocks(a, sam, b, sbk, sbn, M, N, K);
   return there < here ? there : here;
 }
 
 int gemm_f32(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn,
              const float* bias, float* c, long long scm, long long scn, int M, int N, int K, cudaStream_t stream) {
   // On the tensor cores where that is estimated to end first, and always with a smaller error: from about 1 M multiply-adds per
-  // SM on.  Back to back, [N][K]: 64 x 512 x 512 6.8 us here, 8.0 there; 17 x 1000 x 1000 11.1, 12.0; 512^3 14.1, 9.6; 64 x 4096 x 4096 93,
-  // 39.6; 300 x 700 x 2000 45.7, 17.0; 1000 x 2048 x 2048 236, 66.6.
-  if (a && b && c && gemm_f32_tc_takes(a, sam, sak, b, sbk, sbn, M, N, K)) {
+  // SM on.  Back to back, [N][K]: 64 x 512 x 512 6.8 us here, 8.0 there; 34 x 288 x 536 7.2, 9.0; 512^3 14.1, 8.6; 64 x 4096 x 4096 93,
+  // 33.5; 300 x 700 x 2000 45.7, 14.5; 1000 x 2048 x 2048 236, 54.
+  if (a && b && c && gemm_f32_tc_takes(sak, sbk, sbn, M, N, K)) {
     double here;
     choose(M, N, K, sm_count(), here);
-    if (gemm_f32_tc_clocks(sbk, M, N, K) < here) return gemm_f32_tc(a, sam, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
+    if (gemm_f32_tc_clocks(a, sam, b, sbk, sbn, M, N, K) < here) return gemm_f32_tc(a, sam, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
   }
   return launch<float>(a, sam, sak, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
 }

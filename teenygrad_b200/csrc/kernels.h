@@ -161,9 +161,9 @@ int gemm_f32_split(const float* a, const float* b, float* c, int M, int N, int K
                    cudaStream_t stream);
 // The same accuracy as f32 multiply-adds from the tensor cores (gemm_f32_tc.cu): three bf16 terms per operand.  sam = row stride of A
 // (k contiguous); B with either index contiguous.
-bool gemm_f32_tc_takes(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K);
+bool gemm_f32_tc_takes(long long sak, long long sbk, long long sbn, int M, int N, int K);
 int gemm_f32_tc_prepare();
-double gemm_f32_tc_clocks(long long sbk, int M, int N, int K);  // estimated
+double gemm_f32_tc_clocks(const float* a, long long sam, const float* b, long long sbk, long long sbn, int M, int N, int K);  // estimated
 int gemm_f32_tc(const float* a, long long sam, const float* b, long long sbk, long long sbn, const float* bias, float* c, long long scm,
                 long long scn, int M, int N, int K, cudaStream_t stream);
 // f32 GEMM with true f32 accuracy, on the tensor cores or the CUDA cores, whichever is estimated to end first (gemm_f32_clocks).  b_is_nk: B given as [N, K] (linear layout) instead of [K, N].
