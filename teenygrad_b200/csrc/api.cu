@@ -114,6 +114,13 @@ int encode_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const ui
                            strides_bytes, box);
 }
 
+bool encode_store_map(CUtensorMap* out, const bf16* y, int ldy, int rows, int cols) {
+  if (!y || (reinterpret_cast<uintptr_t>(y) & 15) || (ldy & 7) || ldy < cols) return false;
+  const uint64_t dims[2] = {static_cast<uint64_t>(cols), static_cast<uint64_t>(rows)}, strides[1] = {static_cast<uint64_t>(ldy) * 2};
+  const uint32_t box[2] = {64, 32};
+  return encode_tensor_map_bf16(out, y, 2, dims, strides, box) == TEENY_OK;
+}
+
 // Bytes in the same 128-byte swizzle: the FP8 weight tiles that warps convert before the MMA reads them.
 int encode_tensor_map_u8(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                          const uint64_t* strides_bytes, const uint32_t* box) {

@@ -167,9 +167,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, uint32_t src,
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(src), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// every bulk store of this thread has read its shared memory (immediate for a thread that issued none)
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // The eight K-steps of one 128-deep product for the pair, D[tmem] (+)= A[tmem] * B[smem] (rows 0-127 in the leader,
 // 128-255 in the peer), as one block of straight-line code: A advances eight tensor-memory columns per step, the
 // address field of the B descriptor by the compile-time offsets O1..O7 (16-byte units).  One thread issues a
@@ -538,7 +535,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gri
         const uint32_t ph = (g >> 1) & 1;
         if (OPT > 0 && args.gate && lane == 0) {
           if (leaving) {
-            bulk_wait_read();
+            bulk_wait_read<0>();
             mbar_arrive(bar(O_BOX + quarter));
             leaving = false;
           }
@@ -704,11 +701,11 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gri
       // tensor memory as soon as the last Q K^T of this item is complete) and takes that item's first tile, while the
       // first group is still on this item's last tile and output. ----
       if (OPT > 0 && args.gate && lane == 0 && leaving) {
-        bulk_wait_read();
+        bulk_wait_read<0>();
         mbar_arrive(bar(O_BOX + quarter));
         leaving = false;
       }
-      bulk_wait_read();  // this thread's last output rows have left shared memory: whichever group writes there next has
+      bulk_wait_read<0>();  // this thread's last output rows have left shared memory: whichever group writes there next has
       __syncwarp();      // waited for this point, here or through L_READY
       if (!closer) {
         l_sh[r] = l;
@@ -791,7 +788,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gri
       if (seq & 1) m_seen1 += (n_tiles - j_other + 1) >> 1; else m_seen0 += (n_tiles - j_other + 1) >> 1;
       g0 += n_tiles;
     }
-    bulk_wait_read();  // shared memory must outlive the output stores that read it
+    bulk_wait_read<0>();  // shared memory must outlive the output stores that read it
     TRACE_VALUE(6, threadIdx.x == 128, clock64() - c_begin);
     TRACE_VALUE(7, threadIdx.x == 128, w_s);
     TRACE_VALUE(8, threadIdx.x == 128, t_ld);

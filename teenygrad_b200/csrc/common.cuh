@@ -247,6 +247,18 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* m, 
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
+// A tile from shared memory to the tensor, clipped at its edges; bulk_commit() ends a group, bulk_wait_read<N>() waits until all but the last
+// N groups have read shared memory.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Asks for a tile to be brought into L2 only (no shared memory, no barrier): what a kernel launched early uses to
 // keep HBM streaming its next weight tiles, beyond what its shared-memory ring holds, while its predecessor finishes.
 __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
@@ -579,6 +591,62 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// 32 rows of 64 bf16 results, a lane's row packed in v, on their way to (col, row) of a row-major matrix through a warp's 4 KB buffer (the map's box
+// is 64 x 32, 128-byte swizzle).  Stored by each lane for itself a row is 16-byte pieces in 32 lines.
+__device__ __forceinline__ void store_rows64(const CUtensorMap* map, uint32_t buffer, const uint32_t (&v)[32], int col, int row, int lane) {
+  if (lane == 0) bulk_wait_read<0>();  // the store before has left the buffer
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                 ::"r"(buffer + lane * 128 + ((c ^ (lane & 7)) << 4)), "r"(v[4 * c]), "r"(v[4 * c + 1]), "r"(v[4 * c + 2]), "r"(v[4 * c + 3]) : "memory");
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_2d(map, buffer, col, row);
+    bulk_commit();
+  }
+}
+// 64 f32 sums of a row (two loads from tensor memory), with the bias of columns col .. col + 63 of n, as 32 packed pairs
+__device__ __forceinline__ void pack_row64(uint32_t taddr, const bf16* bias, int col, int n, uint32_t (&v)[32]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + h * 32, r);
+    tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      float x = __uint_as_float(r[2 * e]), y = __uint_as_float(r[2 * e + 1]);
+      if (bias) {
+        const int c = col + h * 32 + 2 * e;
+        x += __bfloat162float(bias[min(c, n - 1)]);
+        y += __bfloat162float(bias[min(c + 1, n - 1)]);
+      }
+      v[h * 16 + e] = pack_bf16x2(x, y);
+    }
+  }
+}
+// The same for a gated unit, of 64 gate columns and the 64 up columns behind them.  KIND at compile time: a test at each element kept them from being
+// worked on side by side (6000 x 6144 x 1024 by four warps: 161 us, 110 without).
+template <int KIND>
+__device__ __forceinline__ void pack_glu_row64(uint32_t taddr, uint32_t (&v)[32]) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    uint32_t gr[16], ur[16];
+    tmem_ld_32x16(taddr + h * 16, gr);
+    tmem_ld_32x16(taddr + 64 + h * 16, ur);
+    tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      v[h * 8 + e] = pack_bf16x2(glu_f(KIND, __uint_as_float(gr[2 * e]), __uint_as_float(ur[2 * e])),
+                                 glu_f(KIND, __uint_as_float(gr[2 * e + 1]), __uint_as_float(ur[2 * e + 1])));
+  }
+}
+__device__ __forceinline__ void pack_glu_row64(uint32_t taddr, int kind, uint32_t (&v)[32]) {
+  if (kind == kGluGelu) pack_glu_row64<kGluGelu>(taddr, v);
+  else pack_glu_row64<kGluSilu>(taddr, v);
+}
+
 // ------------------------------------------------------------------------------------------------
 // host: tensor-map encoding through the driver entry point (no link-time dependency on libcuda)
 // ------------------------------------------------------------------------------------------------
@@ -590,6 +658,9 @@ int encode_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const u
 int encode_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box);
 int encode_tensor_map_u8(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                          const uint64_t* strides_bytes, const uint32_t* box);
+
+// of a [rows, cols] bf16 matrix, for store_rows64; false: it cannot be described (16-byte pieces)
+bool encode_store_map(CUtensorMap* out, const bf16* y, int ldy, int rows, int cols);
 
 // SMs of the current device that this thread's launches size their grids for: the device's count, or less while a
 // limit is set (set_sm_limit(n), n <= 0 clears it) to leave SMs to kernels of another stream.

@@ -40,11 +40,13 @@ constexpr int kBM = 128;  // rows of P per tile (MMA M)
 constexpr int kBK = 64;   // k-block: 64 bf16 = one 128-byte swizzle row
 constexpr int kNumThreads = 192;
 constexpr int kEpilogueThreads = 128;
+constexpr int kTileEpiWarps = 8, kTileThreads = 64 + 32 * kTileEpiWarps;  // persistent kernel
 
 struct GemmArgs {
   int M, N, K;            // Y[M, N] = X[M, K] * W[N, K]^T
   int ldy;                // row stride of Y in elements
   bf16* y;
+  int y_map;              // persistent kernel: Y goes by the tensor map (store_rows64)
   float* y32;             // when set (persistent kernel, unswapped): the f32 accumulators are stored as they are, to y32[M, ldy]
   const bf16* bias;       // [N] or null
   int tiles_p, tiles_q;   // tiles along P rows and along Q rows
@@ -80,7 +82,8 @@ struct GemmCfg {
   static constexpr int kStageBytes = kStageP + kStageQ;
   static constexpr int kStages = (BN >= 256) ? 4 : (BN >= 128 ? 6 : 8);
   static constexpr int kTmemCols = (2 * BN < 32) ? 32 : 2 * BN;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align slack*/ + 256 /*barriers*/;
+  static constexpr int kOut = kTileEpiWarps * 4096;  // the epilogue warps' buffers
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOut + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, int tiles_p, int tiles_q, int kGroup, int& tp, int& tq) {
@@ -145,13 +148,13 @@ __device__ __forceinline__ void umma_bf16_ts_x4(uint32_t d_tmem, uint32_t a_tmem
 }
 
 template <int BN, bool SWAP, bool Q_MN_MAJOR>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_q,
-                 const GemmArgs args) {
+                 const __grid_constant__ CUtensorMap tmap_y, const GemmArgs args) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + Cfg::kStages * Cfg::kStageBytes;
+  const uint32_t bar_base = smem_base + Cfg::kStages * Cfg::kStageBytes + Cfg::kOut;
   // barrier layout (8 B each): full[kStages], empty[kStages], acc_full[2], acc_empty[2], then the TMEM address
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (Cfg::kStages + s); };
@@ -160,7 +163,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
   const uint32_t tmem_slot = bar_base + 8u * (2 * Cfg::kStages + 4);
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr =
-      reinterpret_cast<volatile uint32_t*>(smem_gen + Cfg::kStages * Cfg::kStageBytes + 8 * (2 * Cfg::kStages + 4));
+      reinterpret_cast<volatile uint32_t*>(smem_gen + Cfg::kStages * Cfg::kStageBytes + Cfg::kOut + 8 * (2 * Cfg::kStages + 4));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -175,7 +178,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), kEpilogueThreads / 32);
+      mbar_init(acc_empty_bar(b), kTileEpiWarps);
     }
     mbar_fence_init();
   }
@@ -252,9 +255,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
       if (ok && one) umma_commit(acc_full_bar(buf));
     }
   } else {
-    // ---------------- epilogue (warps 2..5; TMEM lane quarter = warp % 4) ----------------
-    const int quarter = warp & 3;
+    // ---------------- epilogue (warps 2..9; TMEM lane quarter = warp % 4, each four warps half of the columns; of narrow tiles and of a
+    // tile that is one group of a gated unit the first four have all) ----------------
+    const int quarter = warp & 3, side = (warp - 2) >> 2;
+    constexpr bool kHalves = BN >= 64;
+    const int c_first = kHalves ? side * (BN / 2) : 0, c_end = kHalves ? c_first + BN / 2 : (side ? 0 : BN);
+    const int glu_first = BN > 128 ? side * 128 : 0, glu_end = BN > 128 ? glu_first + 128 : (side ? 0 : BN);
     const int row_in_tile = quarter * 32 + lane;
+    const uint32_t buffer = smem_base + Cfg::kStages * Cfg::kStageBytes + (warp - 2) * 4096;
     bool ok = true;
     int local = 0;
     for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x, ++local) {
@@ -267,11 +275,38 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
       const int prow = tp * kBM + row_in_tile;  // index along P rows
       constexpr int kChunk = (BN >= 32) ? 32 : 16;
+      if constexpr (!SWAP) {
+        if (args.y_map) {
+          // Rows through shared memory and TMA (us, stored by each lane for itself -> now: 828 x 9496 x 536 23.5 -> 18.8, 1390 x 6712 x 592
+          // 22.7 -> 18.4, 6000 x 3072 x 1024 34.4 -> 31.9).
+          const int row0 = tp * kBM + quarter * 32;
+          if (row0 < args.M) {
+            uint32_t v[32];
+            if (BN >= 128 && args.swiglu) {
+#pragma unroll 1
+              for (int c0 = glu_first; c0 < glu_end && tq * BN + c0 < args.N; c0 += 128) {
+                pack_glu_row64(t_addr + c0, args.swiglu, v);
+                store_rows64(&tmap_y, buffer, v, (tq * BN + c0) / 2, row0, lane);
+              }
+            } else {
+#pragma unroll 1
+              for (int c0 = BN > 64 ? c_first : side * 64; c0 < (BN > 64 ? c_end : BN) && tq * BN + c0 < args.N; c0 += 64) {
+                pack_row64(t_addr + c0, args.bias, tq * BN + c0, args.N, v);
+                store_rows64(&tmap_y, buffer, v, tq * BN + c0, row0, lane);
+              }
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty_bar(buf));
+          continue;
+        }
+      }
       if constexpr (!SWAP && BN >= 128) {
         if (args.swiglu) {
           // columns come in groups of 128 weight rows = 64 gate + 64 up channels: emit 64 outputs per group
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 128) {
+          for (int c0 = glu_first; c0 < glu_end; c0 += 128) {
 #pragma unroll 1
             for (int sub = 0; sub < 64; sub += 32) {
               uint32_t gr[32], ur[32];
@@ -309,7 +344,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
         }
       }
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += kChunk) {
+      for (int c0 = c_first; c0 < c_end; c0 += kChunk) {
         uint32_t r[kChunk];
         if constexpr (kChunk == 32) tmem_ld_32x32(t_addr + c0, r); else tmem_ld_32x16(t_addr + c0, r);
         tmem_wait_ld();
@@ -373,6 +408,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty_bar(buf));
     }
+    if (lane == 0) bulk_wait_all();
   }
 
   // ---------------- teardown ----------------
@@ -977,10 +1013,12 @@ int prepare_skinny() {
 }
 
 template <int BN, bool SWAP, bool Q_MN>
-int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, const GemmArgs& a, int grid, cudaStream_t st) {
+int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, GemmArgs a, int grid, cudaStream_t st) {
   const int rc = prepare_variant<BN, SWAP, Q_MN>();
   if (rc) return rc;
-  launch_kernel(gemm_bf16_kernel<BN, SWAP, Q_MN>, dim3(grid), dim3(kNumThreads), GemmCfg<BN>::kSmemBytes, st, 1, tp, tq, a);
+  CUtensorMap ty{};
+  if (!SWAP) a.y_map = !a.y32 && encode_store_map(&ty, a.y, a.ldy, a.M, a.swiglu ? a.N / 2 : a.N);
+  launch_kernel(gemm_bf16_kernel<BN, SWAP, Q_MN>, dim3(grid), dim3(kTileThreads), GemmCfg<BN>::kSmemBytes, st, 1, tp, tq, ty, a);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -32,13 +32,16 @@ constexpr int kStages = 6;
 constexpr int kStageA = kBM * kBK * 2;
 constexpr int kStageB = kBNh * kBK * 2;
 constexpr int kStageBytes = kStageA + kStageB;   // 32 KB per CTA
-constexpr int kThreads = 192;
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kOut = kEpiWarps * 4096;  // the epilogue warps' buffers
+constexpr int kSmemBytes = kStages * kStageBytes + kOut + 1024 + 256;
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;   // clears the CTA-rank bit of a shared::cluster address -> leader
 
 struct Args2 {
   int M, N, K, ldy;
   bf16* y;
+  int y_map;              // Y goes by the tensor map (store_rows64)
   const bf16* bias;
   int tiles_m, tiles_n;   // 256 x 256 tiles
   int k_blocks;
@@ -100,10 +103,10 @@ __device__ __forceinline__ void tile_coords2(int tile, int tiles_m, int tiles_n,
 
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                      const Args2 args) {
+                      const __grid_constant__ CUtensorMap tmap_y, const Args2 args) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + kStages * kStageBytes;
+  const uint32_t bar_base = smem_base + kStages * kStageBytes + kOut;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
   auto acc_full_bar = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
@@ -111,7 +114,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   const uint32_t tmem_slot = bar_base + 8u * (2 * kStages + 4);
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr =
-      reinterpret_cast<volatile uint32_t*>(smem_gen + kStages * kStageBytes + 8 * (2 * kStages + 4));
+      reinterpret_cast<volatile uint32_t*>(smem_gen + kStages * kStageBytes + kOut + 8 * (2 * kStages + 4));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank2();
@@ -127,7 +130,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), 8);  // four epilogue warps in each CTA of the pair
+      mbar_init(acc_empty_bar(b), 2 * kEpiWarps);  // of both CTAs of the pair
     }
     mbar_fence_init();
   }
@@ -197,9 +200,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       }
     }
   } else {
-    // ---------------- epilogue (both CTAs; TMEM lane quarter = warp % 4) ----------------
-    const int quarter = warp & 3;
+    // ---------------- epilogue (both CTAs; TMEM lane quarter = warp % 4, each four warps 128 of the columns) ----------------
+    const int quarter = warp & 3, side = (warp - 2) >> 2, c_first = side * 128;
     const int row_in_half = quarter * 32 + lane;
+    const uint32_t buffer = smem_base + kStages * kStageBytes + (warp - 2) * 4096;
     const uint32_t acc_empty_leader0 = map_to_rank(acc_empty_bar(0), 0), acc_empty_leader1 = map_to_rank(acc_empty_bar(1), 0);
     bool ok = true;
     int local = 0;
@@ -209,19 +213,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       const int buf = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1;
       const int row = tm * 256 + static_cast<int>(rank) * kBM + row_in_half;
-      // fused QKV epilogue: the token's rotary rows are requested before the wait for the accumulator, so their latency
-      // is gone by the time they are used.  cos[d + 64] == cos[d] (the angles are cat(freqs, freqs)): 64 values each.
-      uint4 rope_c[8], rope_s[8];
-      if (args.qkv && row < args.M) {
-        const int pos = args.f.pos0 + row % args.f.S;
-        const uint4* c4 = reinterpret_cast<const uint4*>(args.f.cos_t + static_cast<size_t>(pos) * 128);
-        const uint4* s4 = reinterpret_cast<const uint4*>(args.f.sin_t + static_cast<size_t>(pos) * 128);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          rope_c[v] = __ldg(c4 + v);
-          rope_s[v] = __ldg(s4 + v);
-        }
-      }
       if (!mbar_wait(acc_full_bar(buf), acc_phase, err, DEVERR_GEMM_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBN;
@@ -234,7 +225,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         const QkvEpilogue& f = args.f;
         const int seq = row / f.S, pos = f.pos0 + row % f.S;
 #pragma unroll 1
-        for (int hh = 0; hh < 2; ++hh) {
+        for (int hh = side; hh <= side; ++hh) {  // a warp's one head
           const int head = tn * 2 + hh;
           if (head >= f.Hq + 2 * f.Hkv) break;  // uniform over the CTA
           uint32_t xp[64];                      // the head as bf16 pairs (the projection is a bf16 tensor)
@@ -282,10 +273,15 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
           }
           // out[d] = n[d] cos[d] - n[d + 64] sin[d];  out[d + 64] = n[d + 64] cos[d + 64] + n[d] sin[d + 64]
+          // cos[d + 64] == cos[d] (the angles are cat(freqs, freqs)): 64 values each.  (Asked for before the wait for the accumulator they are 64
+          // registers that eight epilogue warps do not have: prefill of 4 x 1500 tokens, 0.6B model, 8.0 ms for 7.65.)
+          const uint4* c4 = reinterpret_cast<const uint4*>(f.cos_t + static_cast<size_t>(pos) * 128);
+          const uint4* s4 = reinterpret_cast<const uint4*>(f.sin_t + static_cast<size_t>(pos) * 128);
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
-            const uint32_t cw[4] = {rope_c[v].x, rope_c[v].y, rope_c[v].z, rope_c[v].w};
-            const uint32_t sw[4] = {rope_s[v].x, rope_s[v].y, rope_s[v].z, rope_s[v].w};
+            const uint4 rc = __ldg(c4 + v), rs = __ldg(s4 + v);
+            const uint32_t cw[4] = {rc.x, rc.y, rc.z, rc.w};
+            const uint32_t sw[4] = {rs.x, rs.y, rs.z, rs.w};
             uint32_t lo[4], hi[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -297,10 +293,31 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             dst4[8 + v] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
           }
         }
+      } else if (args.y_map) {
+        // rows through shared memory and TMA (us, stored by each lane for itself -> now: 937 x 4120 x 1840 22.3 -> 18.3, 6000 x 6144 x 1024
+        // 62.2 -> 57.8, 16384 x 6144 x 4096 530 -> 518; eight warps instead of four in the epilogue: a gated unit over 1024 k was
+        // bound by it, 6000 x 6144 x 1024 115 -> 70)
+        const int row0 = tm * 256 + static_cast<int>(rank) * kBM + quarter * 32;
+        if (row0 < args.M) {
+          uint32_t v[32];
+          if (args.swiglu) {
+#pragma unroll 1
+            for (int c0 = c_first; c0 < c_first + 128 && tn * 256 + c0 < args.N; c0 += 128) {
+              pack_glu_row64(t_addr + c0, args.swiglu, v);
+              store_rows64(&tmap_y, buffer, v, (tn * 256 + c0) / 2, row0, lane);
+            }
+          } else {
+#pragma unroll 1
+            for (int c0 = c_first; c0 < c_first + 128 && tn * 256 + c0 < args.N; c0 += 64) {
+              pack_row64(t_addr + c0, args.bias, tn * 256 + c0, args.N, v);
+              store_rows64(&tmap_y, buffer, v, tn * 256 + c0, row0, lane);
+            }
+          }
+        }
       } else if (args.swiglu) {
         // columns come in groups of 128 weight rows = 64 gate + 64 up channels: 64 outputs per group
 #pragma unroll 1
-        for (int c0 = 0; c0 < kBN; c0 += 128) {
+        for (int c0 = c_first; c0 < c_first + 128; c0 += 128) {
 #pragma unroll 1
           for (int sub = 0; sub < 64; sub += 32) {
             uint32_t gr[32], ur[32];
@@ -333,7 +350,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
       } else
 #pragma unroll 1
-      for (int c0 = 0; c0 < kBN; c0 += 32) {
+      for (int c0 = c_first; c0 < c_first + 128; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(t_addr + c0, r);
         tmem_wait_ld();
@@ -372,6 +389,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(buf ? acc_empty_leader1 : acc_empty_leader0);
     }
+    if (lane == 0) bulk_wait_all();
   }
 
   // ---------------- teardown ----------------
@@ -447,7 +465,9 @@ int gemm_bf16_2cta(const bf16* x, int ldx, const bf16* w, int ldw, const bf16* b
   const int tiles = a.tiles_m * a.tiles_n;
   int pairs = sm_count() / 2;
   if (pairs > tiles) pairs = tiles;
-  return launch_kernel(gemm_bf16_2cta_kernel, dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, 2, tmx, tmw, a);
+  CUtensorMap tmy{};
+  a.y_map = !qkv && encode_store_map(&tmy, y, ldy, M, swiglu ? N / 2 : N);
+  return launch_kernel(gemm_bf16_2cta_kernel, dim3(2 * pairs), dim3(kThreads), kSmemBytes, stream, 2, tmx, tmw, tmy, a);
 }
 
 }  // namespace teeny
