@@ -5,7 +5,8 @@
 //               stages (128-byte swizzle), completion on `full` mbarriers;
 //   warp 1      MMA issuer: one elected thread issues tcgen05.mma (M=128, N=BN, K=16) four times per k-block,
 //               tcgen05.commit releases the stage (`empty`) and finally publishes the accumulator (`acc_full`);
-//   warps 2-5   epilogue: tcgen05.ld the 128 x BN f32 accumulator (thread = row), convert to bf16, store.
+//   warps 2-9   epilogue: tcgen05.ld the 128 x BN f32 accumulator (thread = row, four warps half of the columns), convert to bf16,
+//               through shared memory and TMA to Y.
 //   The accumulator is double buffered in TMEM (2 x BN columns) so the epilogue of tile t overlaps the main loop
 //   of tile t+1.
 //
@@ -20,9 +21,9 @@
 // occupy the GPU (decode: M <= 128 tokens, N of a few thousand).  These GEMMs only stream weights, so the job is to
 // get every SM pulling from HBM: K is split across a thread-block cluster (2, 4 or 8 CTAs per weight tile, one
 // k-range each, small enough that two CTAs share an SM), every CTA accumulates its partial tile in TMEM, parks it
-// in its own shared memory, and after a cluster barrier the CTAs sum the partials through distributed shared
-// memory -- each CTA reduces its own slice of the token columns, in cluster-rank order, so the result is
-// bit-reproducible.  No global scratch, no atomics.
+// in its own shared memory, and each CTA sums its own slice of the token columns, in cluster-rank order, so the
+// result is bit-reproducible: sent by the others up to 32 tokens, read through distributed shared memory above.
+// No global scratch, no atomics.
 #include <atomic>
 #include <cstdlib>
 #include <type_traits>
@@ -54,7 +55,7 @@ struct GemmArgs {
   int k_blocks;           // ceil(K / 64)
   int group;              // persistent kernel: P-tiles per raster group
   int kb_per_split;       // skinny kernel: k-blocks per cluster rank
-  int l2_ahead;           // skinny kernel: weight k-blocks asked into L2 beyond the shared-memory ring at start; -1: not the ring's either
+  int l2_ahead;           // skinny kernel: weight k-blocks asked into L2 beyond the shared-memory ring at start
   int swiglu;             // GLU kind (glu_f): W rows interleave 64 gate / 64 up channels; Y[M, N/2] = act(gate) * up
   // Tensor-parallel push (skinny kernel only): instead of Y, the f32 row sums go to slot `rank` of every rank's
   // receive buffer (peer-mapped memory, [M][N] f32 each) and each CTA then bumps every rank's arrival counter.
