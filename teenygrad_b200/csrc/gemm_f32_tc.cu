@@ -170,8 +170,9 @@ __device__ __forceinline__ bool store_columns(const F32Args& g, int m, int n, co
   return !(f.x == 0.0f && f.y == 0.0f);
 }
 
-__device__ __forceinline__ void copy16(uint32_t dst, const float* src, bool there) {  // zeros where nothing is
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+// The first `count` of four numbers (none where it is not positive) and zeros behind them.
+__device__ __forceinline__ void copy16(uint32_t dst, const float* src, int count) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(4 * max(0, min(4, count))) : "memory");
 }
 __device__ __forceinline__ void copy4(uint32_t dst, const float* src, bool there) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(there ? 4 : 0) : "memory");
@@ -201,22 +202,21 @@ __device__ __forceinline__ void sum_again_here(const F32Args& g, float* sm, int 
         copy4(d + (kA + (KN ? r * BN : r * kLd) + c) * 4, there ? g.b + (KN ? k * g.ldb + n : n * g.ldb + k) : g.b, there);
       }
     } else {
-    for (int i = tid; i < kRows * (kK / 4); i += kThreads) {
-      const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4;
-      const bool there = m0 + r < g.M && k < g.K;
-      copy16(d + (r * kLd + i % (kK / 4) * 4) * 4, there ? g.a + (m0 + r) * g.lda + k : g.a, there);
-    }
-    for (int i = tid; i < BN * (kK / 4); i += kThreads) {
-      if constexpr (KN) {
-        const int r = i / (BN / 4), n = i % (BN / 4) * 4;
-        const bool there = k0 + r < g.K && n0 + n < g.N;
-        copy16(d + (kA + r * BN + n) * 4, there ? g.b + (k0 + r) * g.ldb + n0 + n : g.b, there);
-      } else {
-        const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4;
-        const bool there = n0 + r < g.N && k < g.K;
-        copy16(d + (kA + r * kLd + i % (kK / 4) * 4) * 4, there ? g.b + (n0 + r) * g.ldb + k : g.b, there);
+      // 16 bytes at a time, cut off at the row's last number: rows that a tensor map describes start on 16 bytes, but K and N need not be multiples of
+      // four, and what lies behind a row belongs to nobody
+      for (int i = tid; i < kRows * (kK / 4); i += kThreads) {
+        const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4, count = m0 + r < g.M ? g.K - k : 0;
+        copy16(d + (r * kLd + i % (kK / 4) * 4) * 4, count > 0 ? g.a + (m0 + r) * g.lda + k : g.a, count);
       }
-    }
+      for (int i = tid; i < BN * (kK / 4); i += kThreads) {
+        if constexpr (KN) {
+          const int r = i / (BN / 4), n = i % (BN / 4) * 4, count = k0 + r < g.K ? g.N - n0 - n : 0;
+          copy16(d + (kA + r * BN + n) * 4, count > 0 ? g.b + (k0 + r) * g.ldb + n0 + n : g.b, count);
+        } else {
+          const int r = i / (kK / 4), k = k0 + i % (kK / 4) * 4, count = n0 + r < g.N ? g.K - k : 0;
+          copy16(d + (kA + r * kLd + i % (kK / 4) * 4) * 4, count > 0 ? g.b + (n0 + r) * g.ldb + k : g.b, count);
+        }
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -853,7 +853,8 @@ Choice choose(int M, int N, int K, bool kn, bool mapped, int sms) {
 
 }  // namespace
 
-// A [M][K] with k contiguous and B as [N][K] or [K][N] with its second index contiguous, rows of whole 16-byte vectors.
+// A [M][K] with k contiguous and B as [N][K] or [K][N] with its second index contiguous, any alignment, stride and length of rows: rows that a tensor
+// map cannot describe (mappable) are copied four bytes at a time.
 bool gemm_f32_tc_takes(long long sak, long long sbk, long long sbn, int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return false;
   if (sak != 1) return false;

@@ -64,3 +64,24 @@ def test_results_that_are_not_finite(ops, M, N, K, kn):
     some = torch.isfinite(f)
     b = max(48 + K // 64 + 12, K) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
     assert bool(((y.double() - e).abs() <= b)[some].all())
+
+
+@pytest.mark.parametrize("M,N", [(1290, 4100), (300, 1002), (130, 70)])  # pairs, single CTAs, K over a cluster
+@pytest.mark.parametrize("K", [1001, 1002, 1003])
+@pytest.mark.parametrize("kn", [False, True])
+def test_results_that_are_not_finite_between_padded_rows(ops, M, N, K, kn):
+    """Rows that start on 16 bytes with lengths that are no multiple of four: what is summed again ends at a row's last number as well."""
+    x = rows(M, K, 1004, 0, 1)
+    w = rows(K, N, (N + 3) // 4 * 4 + 4, 0, 2).T if kn else rows(N, K, 1004, 0, 2)
+    x[3, 7], x[M - 1, K - 1], w[N - 1, 5] = float("inf"), float("nan"), -float("inf")
+    x[9] *= 2.0 ** 50  # finite sums from 2^80 on overflow on their way
+    w[11] *= 2.0 ** 45
+    y = ops.linear_forward(x, w, None)
+    e = x.double() @ w.double().T
+    f = e.float()
+    assert torch.equal(torch.isnan(y), torch.isnan(f)) and torch.equal(torch.isinf(y), torch.isinf(f))
+    some = torch.isfinite(f)
+    assert bool(some[9, 11]) and abs(float(e[9, 11])) > 2.0 ** 90
+    b = max(48 + K // 64 + 12, K) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)  # (as above)
+    assert bool(((y.double() - e).abs() <= b)[some].all())
+    assert ops.device_error() == 0
