@@ -516,9 +516,13 @@ int attention_f32_tc(const T* q, const T* k, const T* v, T* o, float* lse, const
   constexpr int kTerms = sizeof(T) == 4 ? 3 : 1;
   Args g{};
   g.q = q; g.k = k; g.v = v; g.o = o; g.lse = lse; g.s = s;
-  // The accumulator cuts off at every MMA, which leaves a score short by 1.2e-7 of itself on average (the mean of logsumexp's error over 64 to
-  // 1400 keys, D = 64 and 128: -1.2e-7 without the factor, within 5e-8 with it)
-  g.to_log2 = static_cast<float>(static_cast<double>(s.scale) * 1.4426950408889634 * (1.0 + 1.2e-7) * (kTerms == 3 ? 0x1p-48 : 1.0));
+  // The accumulator cuts off at every MMA, which leaves a score short by part of a half-ulp on average.  What counts are the MMAs of the largest products, one
+  // for 16 dimensions up to the four of an accumulator (zeros behind the head cut nothing off); two bf16 numbers' products are exact and the first sums of
+  // them mostly so, the f32 operands' hi products meet a sum of the smaller ones from the first on.  Mean shortfall of logsumexp, 1000 keys, scores up to 4 sqrt(D),
+  // the rounding of the scale taken off, D = 8, 16, 32, 64, 128: f32 4.2, 3.8, 5.2, 6.3, 6.5e-8, bf16 1.4, 1.8, 3.7, 5.5, - e-8.
+  const int cuts = s.D >= 64 ? 4 : (s.D + 15) / 16;
+  const double shortfall = kTerms == 3 ? 3.2e-8 + 0.8e-8 * cuts : 1.4e-8 * cuts;
+  g.to_log2 = static_cast<float>(static_cast<double>(s.scale) * 1.4426950408889634 * (1.0 + shortfall) * (kTerms == 3 ? 0x1p-48 : 1.0));
   g.from_o = kTerms == 3 ? 0x1p-48f : 0x1p-24f;
   g.row_tiles = (s.Sq + kRows - 1) / kRows;
   g.vec_out = (s.o_sb | s.o_sh | s.o_ss) % static_cast<long long>(16 / sizeof(T)) == 0 && !(reinterpret_cast<uintptr_t>(o) & 15);

@@ -90,3 +90,35 @@ def test_values_behind_the_causal_edge_do_not_count(ops, D):
     o = ops.flash_attn_fwd(q, k, v, 0.125, causal=True)
     assert torch.isfinite(o[:, :, :130]).all() and torch.isnan(o[:, :, 130:]).all()
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [8, 16, 32, 48, 64, 80, 96, 112, 128])
+def test_scores_are_not_off_to_one_side(ops, dtype, D):
+    """Mean error of logsumexp over many rows, relative to the largest scores, which decide it: a score times the scale in f32 may be off by the scale's
+    rounding, a half-ulp (2^-24), for all keys alike; the mean over 30000 rows of what else is rounded stays well below a third of that."""
+    if dtype == torch.bfloat16 and D == 128:
+        pytest.skip("the bf16 kernel's head size")
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(32, 1000, D, generator=g, device="cuda").to(dtype) for _ in range(3))
+    off = []
+    for scale in (4.0, 3.7, 3.1, 2.6):
+        scale = float(torch.tensor(scale * D ** -0.5))  # as the f32 number that the kernel gets
+        s = q.double() @ k.double().transpose(1, 2) * scale
+        l = ops.flash_attention2_forward(q, k, v, scale)[1]
+        off.append(float((l.double() - torch.logsumexp(s, -1)).mean() / s.amax(-1).mean()))
+    assert max(map(abs, off)) <= 2.0 ** -24 * 4 / 3 and abs(sum(off)) / len(off) <= 2.0 ** -24, off
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [8, 16, 64, 120])
+def test_exact_scores(ops, dtype, D):
+    """Scores of one product of powers of two: nothing is cut off, and what the kernel allows for on average (up to 6.5e-8) and the roundings of scale and result
+    stay within 1.5 ulps of 2^-23."""
+    i = torch.arange(300, device="cuda")
+    q, k = (torch.zeros(40, 300, D, device="cuda", dtype=dtype) for _ in range(2))
+    q[:, i, i % D], k[:, i, i % D] = 8.0, 4.0
+    l = ops.flash_attention2_forward(q, k, torch.ones_like(k), 1.0)[1]
+    e = torch.logsumexp(q.double() @ k.double().transpose(1, 2), -1)
+    assert float(((l.double() - e) / e).abs().max()) <= 1.5 * 2.0 ** -23
+    assert ops.device_error() == 0
