@@ -15,12 +15,15 @@ _BF16, _F32 = torch.bfloat16, torch.float32
 
 
 # An operator on small tensors is bound by its host side: of 13.4 us a call, the objects behind torch.cuda.current_stream() and ctypes'
-# pointer wrappers were 4.  The raw handle and plain integers say the same.
-_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# pointer wrappers were 4.  The raw handle and plain integers say the same.  Torch gives the handle under names of its own that a build, one
+# without CUDA among them, need not have.
+_raw_stream, _current_device = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
 
 
 def _stream():
     """Handle of torch's current stream on the current device."""
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_current_device())
 
 
