@@ -475,6 +475,9 @@ int residual_norm(teeny_qwen3* m, bf16* delta, bf16* h, long long ld, bf16* y, c
                            split ? m->at<uint8_t>(m->off.y8) : nullptr, c.hidden, split ? m->at<float>(m->off.y8_scale) : nullptr);
 }
 
+// Weight of an FP8 down projection from which up to 16 rows are split into two FP8 terms for it: between the two sizes that the line was
+// measured at (3072 x 9216 and 4096 x 12288, see run_layers).
+constexpr long long kDown8Weight = 38ll << 20;
 // TEENY_FP8_DOWN_SPLIT=0 leaves the FP8 down projection on the converting kernel (for A/B timing).
 bool down8_enabled() {
   static const bool on = [] { const char* e = getenv("TEENY_FP8_DOWN_SPLIT"); return !(e && e[0] == '0'); }();
@@ -596,12 +599,20 @@ int run_layers(teeny_qwen3* m, int B, int S, int pos0, const int* pos_dev, const
     }
     TEENY_TRY(sublayer_out(attn, w.o, Hq * D, true, false));
     TEENY_TRY(normed(w.post_ln, w.gate_up, mlp_rows, mlp8, act, 2 * I, kGluSilu));
-    // (one GPU, FP8 down projection: its input as two-term FP8 costs a small kernel and saves the conversion of 50 M
-    // weight bytes next to the tensor core.  With more than 16 rows the two terms' products take longer than the
-    // conversion: 4096-wide model, us a step with the split and without, batch 8 527, 541; 16 554, 563; 24 624, 618;
-    // 32 624, 607.)
-    const bool down8 = T <= 16 && down8_enabled() && wants_x8(m, w.down, T) && m->off.a8 != m->off.a8_scale &&
-                       !(decode && rows_take(m, w.down, T, H, I));
+    // (one GPU, FP8 down projection: its input as two-term FP8 costs a small kernel and twice the products, and saves the conversion of the
+    // weight next to the tensor core, which costs as much as there is weight.  Decode step, us, with the split and without, by the weight's size
+    // (hidden x intermediate; 28, 12, 10, 10 and 8 layers):
+    //   rows    1024 x 3072   2048 x 6144   2560 x 9728   3072 x 9216   4096 x 12288
+    //   8       (few rows)    500, 499      537, 528      562, 548      527, 545
+    //   12      1010, 996     514, 512      545, 537      571, 559      538, 552
+    //   16      1044, 1026    519, 514      558, 547      586, 576      549, 565
+    //   20      1174, 1183    582, 582      614, 602      642, 630      603, 603
+    //   32      1130, 1128    567, 561      603, 587      635, 621      597, 595
+    //   48      1545, 1525    721, 707      -             -             734, 737
+    //   64      1594, 1558    755, 733      774, 773      809, 804      759, 756
+    //   128     2349, 2255    1085, 1034    -             -             1105, 1089)
+    const bool down8 = T <= 16 && static_cast<long long>(H) * I >= kDown8Weight && down8_enabled() && wants_x8(m, w.down, T) &&
+                       m->off.a8 != m->off.a8_scale && !(decode && rows_take(m, w.down, T, H, I));
     if (down8) TEENY_TRY(split_e4m3(act, I, m->at<uint8_t>(m->off.a8), I, m->at<float>(m->off.a8_scale), T, I, st));
     TEENY_TRY(sublayer_out(act, w.down, I, l + 1 < c.num_layers, down8));
   }

@@ -116,3 +116,35 @@ def test_sizes_of_the_f32_attention_tests(ops, dtype, H, Sq, Skv, D):
     names = kernels(lambda: ops.flash_attention2_forward(q, k, v, 0.1))
     other = dtype == torch.bfloat16 and D == 128
     assert len(names) == 1 and ("attention_prefill_kernel" if other else "attention_f32_tc_kernel") in names[0], names
+
+
+@pytest.mark.parametrize("hidden,inter,batch,split", [(1024, 3072, 16, False), (3072, 9216, 12, False), (4096, 12288, 1, True), (4096, 12288, 16, True), (4096, 12288, 17, False),
+                                                      (4096, 12288, 128, False), (4096, 9728, 9, True), (4096, 9664, 9, False)])
+def test_fp8_down_projection(hidden, inter, batch, split):
+    """Up to 16 rows in front of a large weight are split into two FP8 terms; a model with FP8 weights that bf16 holds gives what the bf16 model gives."""
+    from teenygrad_b200 import quant, qwen3
+    cfg = qwen3.Qwen3Config(1, hidden, 2, 1, 128, inter, 264, tied=False)
+    fp8, bf16 = {}, {}
+    for name, t in qwen3.random_weights_device(cfg, hidden + inter, "cuda"):
+        fp8[name] = bf16[name] = t
+        if t.dim() == 2:
+            fp8[name], fp8[name + "_scale"] = (t.float() * 2.0 ** 10).to(torch.float8_e4m3fn), torch.full((t.shape[0],), 2.0 ** -10, device="cuda")
+            bf16[name] = (fp8[name].float() * 2.0 ** -10).bfloat16()
+    ids = torch.arange(batch, device="cuda", dtype=torch.int32)[:, None]
+    first, picked, step = [], [], []
+    for tensors in (fp8, bf16):
+        r = qwen3.Qwen3Runner(cfg, max_batch=batch, max_len=4, max_tokens=128, max_new_tokens=2)
+        r.load_quantized(tensors, quant.Fp8Scheme("channel")) if tensors is fp8 else r.load_state_dict(tensors)
+        if tensors is fp8:
+            assert any("split_e4m3_vec_kernel" in n for n in kernels(lambda: r.prefill(ids))) == split  # noqa: B023
+        r.prefill(ids)
+        first.append(r.logits().double())
+        picked.append(r.next_ids().clone())
+        r.decode_step()
+        step.append(r.logits().double())
+        assert r.device_error() == 0
+    same = picked[0] == picked[1]  # (near ties may go to another token, which the step then goes on from)
+    assert int(same.sum()) >= 0.9 * batch
+    for a, b in (first, [x[same] for x in step]):
+        # eight bf16 tensors from the first kernel to the last, each rounded by 2^-9 at most from sums in another order
+        assert float((a - b).norm() / b.norm()) < 8 * 2.0 ** -9
