@@ -74,18 +74,6 @@ struct Args {
   int* err;
 };
 
-// the three bf16 terms of two numbers, packed
-__device__ __forceinline__ void terms3(f32x2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const f32x2 minus = pack2(-1.0f, -1.0f);
-  const float2 u = unpack2(v);
-  hi = pack_bf16x2(u.x, u.y);
-  const f32x2 r = fma2(pack2(bf16_lo(hi), bf16_hi(hi)), minus, v);
-  const float2 f = unpack2(r);
-  mid = pack_bf16x2(f.x, f.y);
-  const float2 q = unpack2(fma2(pack2(bf16_lo(mid), bf16_hi(mid)), minus, r));
-  lo = pack_bf16x2(q.x, q.y);
-}
-
 template <typename F, int... I>
 __device__ __forceinline__ void each(std::integer_sequence<int, I...>, F f) { (f(std::integral_constant<int, I>{}), ...); }
 
@@ -109,8 +97,8 @@ struct Operand {
     } else {
       const f32x2 up = pack2(kUp, kUp);
       uint2 hi, mid, lo;
-      terms3(mul2(pack2(__uint_as_float(x.x), __uint_as_float(x.y)), up), hi.x, mid.x, lo.x);
-      terms3(mul2(pack2(__uint_as_float(x.z), __uint_as_float(x.w)), up), hi.y, mid.y, lo.y);
+      bf16_terms3(mul2(pack2(__uint_as_float(x.x), __uint_as_float(x.y)), up), hi.x, mid.x, lo.x);
+      bf16_terms3(mul2(pack2(__uint_as_float(x.z), __uint_as_float(x.w)), up), hi.y, mid.y, lo.y);
       to += (d & 4) * 2;
       *reinterpret_cast<uint2*>(to) = hi;
       *reinterpret_cast<uint2*>(to + kTerm) = mid;
@@ -378,7 +366,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_f32_tc_kernel(const __g
             const float2 z = unpack2(fma2(pack2(x[e0 + 2 * e], x[e0 + 2 * e + 1]), cc, nn));
             const f32x2 p = pack2(ex2(z.x), ex2(z.y));
             sum = fma2(p, one, sum);
-            terms3(mul2(p, up), hi[e], mid[e], lo[e]);
+            bf16_terms3(mul2(p, up), hi[e], mid[e], lo[e]);
           }
           if (c == 0 && e0 == 0 && j > 0) {
             wait(P_EMPTY, (j & 1) ^ 1);

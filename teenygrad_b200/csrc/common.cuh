@@ -272,6 +272,38 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ------------------------------------------------------------------------------------------------
+// thread-block clusters
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// An arrival that orders nothing (a releasing one waits for what the thread has under way, 1000 clocks and more): for barriers whose initialisation
+// has its own fence, and for bulk copies that a barrier has counted.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// an address in this CTA's shared memory -> the same place in CTA `rank`'s
+__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+// shared memory -> another CTA's (dst and bar are its addresses); its barrier counts the bytes
+__device__ __forceinline__ void send_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// ------------------------------------------------------------------------------------------------
 // tcgen05 / tensor memory
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {  // whole warp
@@ -323,6 +355,25 @@ __device__ __forceinline__ void umma_ts_at(uint32_t d, uint32_t a, uint64_t b, u
   asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x;\n\t.reg .b64 y;\n\tadd.u32 x, %1, %5;\n\tadd.u64 y, %2, %6;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                "tcgen05.mma.cta_group::1.kind::f16 [%0], [x], y, %3, p;\n\t}"
                ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "n"(OA), "n"(OB) : "memory");
+}
+// The four K=16 steps of a 64-deep product as one block of straight-line code, D[tmem] (+)= A * B with A and B in shared memory.  Per step the
+// address field of a K-major descriptor advances by 2 (16 k = 32 bytes inside the swizzled row), that of an MN-major one by 128 (two 8-row groups
+// of 1024 bytes); the steps are compile-time immediates because a lone thread that computes addresses between its tcgen05.mma issues one only
+// every ~100 cycles.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_bf16_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accumulate_first) {
+  asm volatile(
+      "{\n\t.reg .pred p, t;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 t, %3, %3;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.u64 a, %1, %5;\n\t add.u64 b, %2, %6;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.u64 a, %1, %7;\n\t add.u64 b, %2, %8;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+      "add.u64 a, %1, %9;\n\t add.u64 b, %2, %10;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "n"(A_STEP), "n"(B_STEP), "n"(2 * A_STEP),
+        "n"(2 * B_STEP), "n"(3 * A_STEP), "n"(3 * B_STEP)
+      : "memory");
 }
 // mbarrier arrives once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -574,6 +625,17 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+// Two f32 numbers as three bf16 terms each, packed: x = hi + mid + lo, each the rounded rest of the ones before.
+__device__ __forceinline__ void bf16_terms3(f32x2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const f32x2 minus = pack2(-1.0f, -1.0f);
+  const float2 u = unpack2(v);
+  hi = pack_bf16x2(u.x, u.y);
+  const f32x2 r = fma2(pack2(bf16_lo(hi), bf16_hi(hi)), minus, v);
+  const float2 f = unpack2(r);
+  mid = pack_bf16x2(f.x, f.y);
+  const float2 q = unpack2(fma2(pack2(bf16_lo(mid), bf16_hi(mid)), minus, r));
+  lo = pack_bf16x2(q.x, q.y);
+}
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -654,7 +716,7 @@ __device__ __forceinline__ void pack_glu_row64(uint32_t taddr, int kind, uint32_
 // 128-byte swizzle; box[0] must be 64 elements.  Returns TEENY_OK or an error code.
 int encode_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                            const uint64_t* strides_bytes, const uint32_t* box);
-// the same for a tensor of bytes
+// the same for f32 numbers, for bytes
 int encode_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box);
 int encode_tensor_map_u8(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                          const uint64_t* strides_bytes, const uint32_t* box);

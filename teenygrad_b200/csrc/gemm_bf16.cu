@@ -99,27 +99,7 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_p, int tiles_q, 
   tq = r / size_p;
 }
 
-// The four K=16 steps of a 64-deep product as one block of straight-line code, D[tmem] (+)= A * B with B in shared
-// memory and A in shared memory (SS) or tensor memory (TS).  Per step the address field of a K-major shared-memory
-// descriptor advances by 2 (16 k = 32 bytes inside the swizzled row), that of an MN-major one by 128 (two 8-row groups
-// of 1024 bytes), a tensor-memory A by 8 columns (16 bf16 as pairs); the steps are compile-time immediates because a
-// lone thread that computes addresses between its tcgen05.mma issues one only every ~100 cycles.
-template <int A_STEP, int B_STEP>
-__device__ __forceinline__ void umma_bf16_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                uint32_t accumulate_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 a, b;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.eq.b32 t, %3, %3;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "add.u64 a, %1, %5;\n\t add.u64 b, %2, %6;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
-      "add.u64 a, %1, %7;\n\t add.u64 b, %2, %8;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
-      "add.u64 a, %1, %9;\n\t add.u64 b, %2, %10;\n\t tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "n"(A_STEP), "n"(B_STEP), "n"(2 * A_STEP),
-        "n"(2 * B_STEP), "n"(3 * A_STEP), "n"(3 * B_STEP)
-      : "memory");
-}
-// The same for kind::f8f6f4 with both operands FP8 (E4M3) in shared memory: four K = 32 steps over 128 k, 32 bytes each.
+// umma_bf16_ss_x4 for kind::f8f6f4 with both operands FP8 (E4M3) in shared memory: four K = 32 steps over 128 k, 32 bytes each.
 __device__ __forceinline__ void umma_f8_ss_x4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate_first) {
   asm volatile(
@@ -133,6 +113,7 @@ __device__ __forceinline__ void umma_f8_ss_x4(uint32_t d_tmem, uint64_t a_desc, 
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first)
       : "memory");
 }
+// umma_bf16_ss_x4 with A in tensor memory, 8 columns (16 bf16 as pairs) a step.
 template <int B_STEP>
 __device__ __forceinline__ void umma_bf16_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                                 uint32_t accumulate_first) {
@@ -486,33 +467,6 @@ struct SkinnyCfg {
   static_assert(!kSend || 2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs on an SM");
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// An arrival that orders nothing (a releasing one waits for what the thread has under way, 1000 clocks): for barriers whose initialisation has
-// its own fence, and for bulk copies that a barrier has counted.
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-  return a;
-}
-// shared memory -> another CTA's (dst and bar are its addresses); its barrier counts the bytes
-__device__ __forceinline__ void send_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
 // 16 bytes of CTA `rank`'s shared memory at this CTA's address `local_addr`.  Volatile (so it stays behind the cluster
 // barrier, itself a volatile asm) but without a memory clobber: consecutive loads are all in flight together.
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t local_addr, uint32_t rank) {
@@ -618,7 +572,7 @@ gemm_bf16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       }
       // ... and the weight tiles behind them are asked into L2, so that HBM keeps streaming this kernel's weights for
       // as long as the predecessor's tail lasts, not just until the ring is full
-      for (int kb = kb0 + pre; kb < min(kb1, kb0 + (args.l2_ahead < 0 ? 0 : ring + args.l2_ahead)); ++kb)
+      for (int kb = kb0 + pre; kb < min(kb1, kb0 + ring + args.l2_ahead); ++kb)
         if (one) tma_prefetch_l2_2d(&tmap_w, kb * Cfg::kKB, tile * kBM);
       pdl_wait();
       auto load_x = [&](uint32_t sq, uint32_t bar, int kb) {  // the activation tile(s) of one stage: 64 k each

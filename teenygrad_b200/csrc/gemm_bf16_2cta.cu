@@ -52,19 +52,6 @@ struct Args2 {
   int* err;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank2() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync2() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -117,7 +104,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       reinterpret_cast<volatile uint32_t*>(smem_gen + kStages * kStageBytes + kOut + 8 * (2 * kStages + 4));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank2();
+  const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   int* err = args.err;
 
@@ -140,7 +127,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync2();  // both CTAs' barriers exist before either CTA can signal the other
+  cluster_sync_all();  // both CTAs' barriers exist before either CTA can signal the other
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   pdl_wait();
@@ -204,7 +191,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     const int quarter = warp & 3, side = (warp - 2) >> 2, c_first = side * 128;
     const int row_in_half = quarter * 32 + lane;
     const uint32_t buffer = smem_base + kStages * kStageBytes + (warp - 2) * 4096;
-    const uint32_t acc_empty_leader0 = map_to_rank(acc_empty_bar(0), 0), acc_empty_leader1 = map_to_rank(acc_empty_bar(1), 0);
+    const uint32_t acc_empty_leader0 = map_rank(acc_empty_bar(0), 0), acc_empty_leader1 = map_rank(acc_empty_bar(1), 0);
     bool ok = true;
     int local = 0;
     for (int t = pair; ok && t < num_tiles; t += n_pairs, ++local) {
@@ -217,23 +204,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBN;
       if (args.qkv) {
-        // Each 128-column half of the tile is one head of the fused [q | k | v] projection and a thread holds the whole
+        // Each 128-column half of the tile is one head of the fused [q | k | v] projection, a warp has one of them and a thread holds the whole
         // head of its token: per-head RMSNorm (q, k), rotate-half rotary embedding at the token's position (q, k), then
         // q goes back into the projection buffer and k / v straight into the caches -- the rounding points are those of
         // the separate kernel (head_norm_rope, common.cuh): the projection, the normed head, each product and the sum
         // are bf16 tensors.
         const QkvEpilogue& f = args.f;
-        const int seq = row / f.S, pos = f.pos0 + row % f.S;
-#pragma unroll 1
-        for (int hh = side; hh <= side; ++hh) {  // a warp's one head
-          const int head = tn * 2 + hh;
-          if (head >= f.Hq + 2 * f.Hkv) break;  // uniform over the CTA
-          uint32_t xp[64];                      // the head as bf16 pairs (the projection is a bf16 tensor)
+        const int seq = row / f.S, pos = f.pos0 + row % f.S, head = tn * 2 + side;
+        auto store_head = [&] {
+          uint32_t xp[64];  // the head as bf16 pairs (the projection is a bf16 tensor)
           float sq4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t r[32];
-            tmem_ld_32x32(t_addr + hh * 128 + c * 32, r);
+            tmem_ld_32x32(t_addr + c_first + c * 32, r);
             tmem_wait_ld();
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
@@ -243,7 +227,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
           }
           const float sq = (sq4[0] + sq4[1]) + (sq4[2] + sq4[3]);
-          if (row >= args.M) continue;
+          if (row >= args.M) return;
           bf16* dst;
           if (head < f.Hq) {
             dst = args.y + static_cast<size_t>(row) * args.ldy + static_cast<size_t>(head) * 128;
@@ -257,7 +241,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           if (head >= f.Hq + f.Hkv) {  // v: no norm, no rotation
 #pragma unroll
             for (int v = 0; v < 16; ++v) dst4[v] = make_uint4(xp[4 * v], xp[4 * v + 1], xp[4 * v + 2], xp[4 * v + 3]);
-            continue;
+            return;
           }
           const float rr = 1.0f / sqrtf(sq * (1.0f / 128.0f) + f.eps);
           const uint4* w4 = reinterpret_cast<const uint4*>(head < f.Hq ? f.q_w : f.k_w);
@@ -292,7 +276,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             dst4[v] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             dst4[8 + v] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
           }
-        }
+        };
+        if (head < f.Hq + 2 * f.Hkv) store_head();  // (the same in all lanes: four warps have one half)
       } else if (args.y_map) {
         // rows through shared memory and TMA (us, stored by each lane for itself -> now: 937 x 4120 x 1840 22.3 -> 18.3, 6000 x 6144 x 1024
         // 62.2 -> 57.8, 16384 x 6144 x 4096 530 -> 518; eight warps instead of four in the epilogue: a gated unit over 1024 k was
@@ -301,10 +286,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         if (row0 < args.M) {
           uint32_t v[32];
           if (args.swiglu) {
-#pragma unroll 1
-            for (int c0 = c_first; c0 < c_first + 128 && tn * 256 + c0 < args.N; c0 += 128) {
-              pack_glu_row64(t_addr + c0, args.swiglu, v);
-              store_rows64(&tmap_y, buffer, v, (tn * 256 + c0) / 2, row0, lane);
+            if (tn * 256 + c_first < args.N) {
+              pack_glu_row64(t_addr + c_first, args.swiglu, v);
+              store_rows64(&tmap_y, buffer, v, (tn * 256 + c_first) / 2, row0, lane);
             }
           } else {
 #pragma unroll 1
@@ -315,35 +299,32 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           }
         }
       } else if (args.swiglu) {
-        // columns come in groups of 128 weight rows = 64 gate + 64 up channels: 64 outputs per group
+        // columns come in groups of 128 weight rows = 64 gate + 64 up channels: 64 outputs per group, a warp has one
 #pragma unroll 1
-        for (int c0 = c_first; c0 < c_first + 128; c0 += 128) {
-#pragma unroll 1
-          for (int sub = 0; sub < 64; sub += 32) {
-            uint32_t gr[32], ur[32];
-            tmem_ld_32x32(t_addr + c0 + sub, gr);
-            tmem_ld_32x32(t_addr + c0 + 64 + sub, ur);
-            tmem_wait_ld();
-            const int ocol0 = (tn * 256 + c0) / 2 + sub;
-            if (row < args.M) {
-              bf16* dst = args.y + static_cast<size_t>(row) * args.ldy + ocol0;
-              const bool vec_ok = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) && (ocol0 + 32 <= args.N / 2);
+        for (int sub = 0; sub < 64; sub += 32) {
+          uint32_t gr[32], ur[32];
+          tmem_ld_32x32(t_addr + c_first + sub, gr);
+          tmem_ld_32x32(t_addr + c_first + 64 + sub, ur);
+          tmem_wait_ld();
+          const int ocol0 = (tn * 256 + c_first) / 2 + sub;
+          if (row < args.M) {
+            bf16* dst = args.y + static_cast<size_t>(row) * args.ldy + ocol0;
+            const bool vec_ok = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) && (ocol0 + 32 <= args.N / 2);
 #pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                float f[8];
+            for (int v = 0; v < 4; ++v) {
+              float f[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                f[e] = glu_f(args.swiglu, __uint_as_float(gr[v * 8 + e]), __uint_as_float(ur[v * 8 + e]));
+              if (vec_ok) {
+                uint4 o;
+                o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
+                o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
+                *reinterpret_cast<uint4*>(dst + v * 8) = o;
+              } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
-                  f[e] = glu_f(args.swiglu, __uint_as_float(gr[v * 8 + e]), __uint_as_float(ur[v * 8 + e]));
-                if (vec_ok) {
-                  uint4 o;
-                  o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
-                  o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-                  *reinterpret_cast<uint4*>(dst + v * 8) = o;
-                } else {
-#pragma unroll
-                  for (int e = 0; e < 8; ++e)
-                    if (ocol0 + v * 8 + e < args.N / 2) dst[v * 8 + e] = __float2bfloat16_rn(f[e]);
-                }
+                  if (ocol0 + v * 8 + e < args.N / 2) dst[v * 8 + e] = __float2bfloat16_rn(f[e]);
               }
             }
           }
@@ -396,7 +377,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   pdl_trigger();
   tc_fence_before();
   __syncthreads();
-  cluster_sync2();  // the peer may still be signalling this CTA's barriers / reading its shared memory
+  cluster_sync_all();  // the peer may still be signalling this CTA's barriers / reading its shared memory
   if (warp == 2) {
     if (*reinterpret_cast<volatile int*>(err) != 0) {
       const uint64_t t0 = global_timer_ns();

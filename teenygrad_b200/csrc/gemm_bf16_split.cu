@@ -46,41 +46,6 @@ struct SplitArgs {
   int* err;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-// Relaxed: the barriers' initialisation has a fence of its own, and that something has arrived orders nothing else.  (A release took 1000
-// clocks and more, waiting for what the thread had under way.)
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-  return a;
-}
-// shared memory -> another CTA's, at the same offset plus `to`; its barrier counts the bytes
-__device__ __forceinline__ void send(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void umma_x4(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 x, y;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, %3, %3;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "add.u64 x, %1, 2;\n\tadd.u64 y, %2, 2;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, t;\n\t"
-      "add.u64 x, %1, 4;\n\tadd.u64 y, %2, 4;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, t;\n\t"
-      "add.u64 x, %1, 6;\n\tadd.u64 y, %2, 6;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, t;\n\t}"
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate_first) : "memory");
-}
-
 // Pieces of 4 weight rows of a token, the S parts added in the order of k.
 template <int S>
 __device__ __forceinline__ void finish(const SplitArgs& g, const float4* own, const float4* got, int rank, int m0, int tile, int columns) {
@@ -201,7 +166,7 @@ gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (S > 1) {
     if (tid == 0) mbar_expect_tx(received, (S - 1) * columns * (kBM * 4));
     __syncwarp();
-    cluster_arrive();  // this CTA's barriers exist
+    cluster_arrive_relaxed();  // this CTA's barriers exist
   }
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_at);
   if (warp != 0) pdl_wait();
@@ -222,7 +187,7 @@ gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     for (int i = 0; i < n; ++i) {
       if (!ready && !mbar_wait(full(s), ph, g.err, DEVERR_GEMM_MMA)) { ok = false; break; }
       tc_fence_after();
-      if (one) umma_x4(tmem, dw + off, dx + off, make_idesc_bf16(kBM, BN, false, false), i ? 1u : 0u);
+      if (one) umma_bf16_ss_x4<2, 2>(tmem, dw + off, dx + off, make_idesc_bf16(kBM, BN, false, false), i ? 1u : 0u);
       if (i + g.stages < n && one) umma_commit(empty(s));
       off += C::kStage / 16;
       if (++s == g.stages) { s = 0; ph ^= 1; off = 0; }
@@ -256,12 +221,12 @@ gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     if (S > 1 && warp == 2 && lane < S && lane != rank && !gave_up) {  // each other CTA gets the columns that it finishes
       const int q = lane, from = first_of(q), bytes = (first_of(q + 1) - from) * (kBM * 4);
       if (bytes > 0)
-        send(map_rank(base + g.ring + (rank - (rank > q)) * bytes, q), base + from * (kBM * 4), bytes, map_rank(received, q));
+        send_bulk(map_rank(base + g.ring + (rank - (rank > q)) * bytes, q), base + from * (kBM * 4), bytes, map_rank(received, q));
     }
     bool ok = true;
     if (S > 1 && columns > 0) ok = mbar_wait(received, 0, g.err, DEVERR_GEMM_EPILOGUE);
     __syncwarp();
-    if (S > 1) cluster_arrive();  // what was sent here has arrived
+    if (S > 1) cluster_arrive_relaxed();  // what was sent here has arrived
     if (ok) {
       const float4* own = reinterpret_cast<const float4*>(part + c0 * kBM);
       const float4* got = reinterpret_cast<const float4*>(reinterpret_cast<uint8_t*>(part) + g.ring);
@@ -277,7 +242,7 @@ gemm_bf16_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       }
     }
   } else if (S > 1) {
-    cluster_arrive();
+    cluster_arrive_relaxed();
   }
   __syncwarp();
   if (warp == 1) {

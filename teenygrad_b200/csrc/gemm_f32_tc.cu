@@ -62,19 +62,6 @@ struct F32Args {
   int* err;
 };
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t map_rank(uint32_t local, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
-  return a;
-}
-// shared memory -> another CTA's; its barrier counts the bytes
-__device__ __forceinline__ void send(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
 template <int OA, int OB>
 __device__ __forceinline__ void umma_ts_pair_at(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x;\n\t.reg .b64 y;\n\tadd.u32 x, %1, %5;\n\tadd.u64 y, %2, %6;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -87,16 +74,9 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
                ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
 }
 
-// two numbers -> the three bf16 terms of kUp times them, packed
+// the three terms of kUp times two numbers
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const f32x2 minus = pack2(-1.0f, -1.0f), v = mul2(pack2(x, y), pack2(kUp, kUp));
-  const float2 u = unpack2(v);
-  hi = pack_bf16x2(u.x, u.y);
-  const f32x2 r = fma2(pack2(bf16_lo(hi), bf16_hi(hi)), minus, v);
-  const float2 f = unpack2(r);
-  mid = pack_bf16x2(f.x, f.y);
-  const float2 q = unpack2(fma2(pack2(bf16_lo(mid), bf16_hi(mid)), minus, r));
-  lo = pack_bf16x2(q.x, q.y);
+  bf16_terms3(mul2(pack2(x, y), pack2(kUp, kUp)), hi, mid, lo);
 }
 
 // Results (m, n .. n + 3); whether one of them is not finite.
@@ -524,11 +504,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // Every CTA is behind its main loop, so what the others send may take the place of its stages: a CTA finishes kBM / split rows of
     // the tile and gets them from the others by bulk copies (remote loads took 2000 clocks), relaxed arrivals: the barrier above
     // has seen every reader.
-    cluster_arrive();
+    cluster_arrive_relaxed();
     cluster_wait();
     const int bytes = rows * C::kPitch * 4;
     if (warp == kSplitWarps && lane < g.split && lane != rank && !gave_up)
-      send(map_rank(base + C::kPart + (rank - (rank > lane)) * bytes, lane), base + lane * bytes, bytes, map_rank(received, lane));
+      send_bulk(map_rank(base + C::kPart + (rank - (rank > lane)) * bytes, lane), base + lane * bytes, bytes, map_rank(received, lane));
     __syncwarp();
     if (mbar_wait(received, 0, g.err, DEVERR_GEMM_EPILOGUE)) {
       // the parts added in the order of k
@@ -549,7 +529,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     __syncwarp();
-    cluster_arrive();
+    cluster_arrive_relaxed();
     cluster_wait();  // nobody leaves, or takes its shared memory for something else, while what it sent is on its way
     if (tid == 0) gave_up = *reinterpret_cast<volatile int*>(g.err) != 0;
     __syncthreads();
@@ -620,7 +600,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
+  cluster_arrive_relaxed();
   cluster_wait();  // both CTAs' barriers exist
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(gen + C::kStages + 104);
@@ -743,7 +723,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();
+  cluster_arrive_relaxed();
   cluster_wait();  // neither CTA leaves while the other's MMAs read its terms
   if (tid == 0) gave_up = *reinterpret_cast<volatile int*>(g.err) != 0;
   __syncthreads();

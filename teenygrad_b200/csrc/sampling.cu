@@ -8,21 +8,18 @@
 //      sequentially in f32;
 //   3. nucleus = the shortest prefix with c_{n-1} >= top_p * c_last (at least one candidate);
 //   4. the sample is the first candidate i < n with c_i > u * c_{n-1}, u in [0, 1) given per row by the caller.
-// bf16 logits have 65536 possible values, so the k-th largest value is found exactly with two 256-bin histograms
-// (high byte, then low byte inside the deciding bin).
 //
-// Bound: latency; a row is 300 KB and its logits have just been written.  A row is cut over a thread-block cluster (up to
-// 8 CTAs while the grid stays within one CTA per SM), each CTA histograms its slice with 16-byte loads that later passes
-// find in L1, the cluster adds the histograms through distributed shared memory.  Everything at or above the threshold
-// goes into a list per CTA; the first CTA sorts their union, which also orders the ties at the threshold (a row with
-// thousands of them, such as a masked one, is collected in index order instead).  One thread does the running sums,
-// so that the result does not depend on a reduction tree; the cut and the pick are searches over them.
+// Bound: latency; a row is 300 KB and its logits have just been written.  A row is cut over a thread-block cluster (up to four CTAs, see
+// sample_parts), which read their slices with 16-byte loads that later passes find in L1.  Each thread takes the largest of its columns' keys
+// (packed pairs), and each of the row's P CTAs finds the ceil(K / P)-th largest of its 1024, a bit at a time by barriers that count.  The smallest
+// of these P bounds is reached by at least K entries of the row, so every one of the top K is among the entries not below it, of which there are
+// little more than K: only the threads whose largest reaches it look at their columns again.  The entries go into a list per CTA; the first CTA sorts
+// their union.  One thread does the running sums, so that the result does not depend on a reduction tree; the cut and the pick are searches over them.
 //
-// Mostly no histogram is needed: logits share a handful of exponents, so that a warp's 32 increments of the high byte's bins mostly hit the
-// same one or two.  Instead each thread takes the largest of its columns' keys (packed pairs), and each of the row's P CTAs finds the
-// ceil(K / P)-th largest of its 1024, a bit at a time by barriers that count.  The smallest of these P bounds is reached by at least K
-// entries of the row, so every one of the top K is among the entries not below it, of which there are little more than K: only the threads whose
-// largest reaches it look at their columns again.  Where they do not fit the list (ties), or the threads are too few, the histograms decide.
+// Where they do not fit the list (ties), or the threads are too few, histograms decide: bf16 logits have 65536 possible values, so two 256-bin
+// histograms (high byte, then low byte inside the deciding bin), which the cluster adds through distributed shared memory, give the k-th
+// largest value exactly; what is at or above it goes into the lists (a row with thousands of ties, such as a masked one, is collected in index order
+// instead).  For every row they are slower: logits share a handful of exponents, and a warp's 32 increments of the high byte's bins mostly hit the same one or two.
 // Measured on B200, before (histograms, bitonic sort) and now: 32 x 151936, top-k 50 17.0 -> 11.8 us, top-k 1000 36.4 -> 19.8; 8 x 151936 16.4 -> 11.5;
 // 64 x 151936 22.8 -> 13.9; 64 x 32768 13.0 -> 8.7; 5 x 1000 8.4 -> 6.7.
 #include <atomic>
@@ -36,6 +33,7 @@ namespace {
 
 constexpr int kSampleThreads = 1024;
 constexpr int kMaxTopK = 1024;
+constexpr int kMaxParts = 4;  // CTAs of a row (sample_parts)
 
 // bf16 bit pattern -> 16-bit key whose unsigned order is the float order (NaNs sort above +inf; not expected here)
 __device__ __forceinline__ unsigned sort_key(unsigned short bits) {
@@ -112,14 +110,6 @@ __device__ __forceinline__ void pick_from_sorted(const unsigned long long* cand,
   }
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // address of `local` (an address in this CTA's shared memory) in the shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_smem(const void* local, uint32_t rank) {
   uint32_t a;
@@ -275,18 +265,18 @@ sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int col
   const unsigned K = static_cast<unsigned>(min(top_k, cols));
   const int slice = ((cols + parts - 1) / parts + 7) & ~7;
   const int begin = min(cols, static_cast<int>(rank) * slice), end = min(cols, begin + slice);
-  auto sync_row = [&] { if (parts > 1) cluster_sync(); else __syncthreads(); };
+  auto sync_row = [&] { if (parts > 1) cluster_sync_all(); else __syncthreads(); };
   // the row's histogram from all CTAs', then the bin that holds entry number `want` from the top
   auto decide = [&](int level, unsigned want) {
     sync_row();
     if (tid < 256) {
       unsigned n = 0;
       if (parts > 1) {
-        unsigned v[8];
+        unsigned v[kMaxParts];
 #pragma unroll
-        for (int p = 0; p < 8; ++p) v[p] = p < parts ? ld_peer_u32(peer_smem(&sh.hist[level][tid], p)) : 0u;
+        for (int p = 0; p < kMaxParts; ++p) v[p] = p < parts ? ld_peer_u32(peer_smem(&sh.hist[level][tid], p)) : 0u;
 #pragma unroll
-        for (int p = 0; p < 8; ++p) n += v[p];
+        for (int p = 0; p < kMaxParts; ++p) n += v[p];
       } else {
         n = sh.hist[level][tid];
       }
@@ -323,12 +313,12 @@ sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int col
       if (__syncthreads_count(top >= (bound | bit)) >= want) bound |= bit;
     if (parts > 1) {
       if (tid == 0) sh.bound = bound;
-      cluster_sync();
-      unsigned v[8];
+      cluster_sync_all();
+      unsigned v[kMaxParts];
 #pragma unroll
-      for (int p = 0; p < 8; ++p) v[p] = p < parts ? ld_peer_u32(peer_smem(&sh.bound, p)) : bound;
+      for (int p = 0; p < kMaxParts; ++p) v[p] = p < parts ? ld_peer_u32(peer_smem(&sh.bound, p)) : bound;
 #pragma unroll
-      for (int p = 0; p < 8; ++p) bound = min(bound, v[p]);
+      for (int p = 0; p < kMaxParts; ++p) bound = min(bound, v[p]);
     }
     if (top >= bound) {
       auto list = [&](int i, unsigned k) {
@@ -349,23 +339,23 @@ sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int col
       }
     }
     sync_row();
-    unsigned n[8], total = 0;  // (a list that ran over has a count beyond it)
+    unsigned n[kMaxParts], total = 0;  // (a list that ran over has a count beyond it)
 #pragma unroll
-    for (int p = 0; p < 8; ++p) n[p] = p < parts ? (parts > 1 ? ld_peer_u32(peer_smem(&sh.count, p)) : sh.count) : 0u;
+    for (int p = 0; p < kMaxParts; ++p) n[p] = p < parts ? (parts > 1 ? ld_peer_u32(peer_smem(&sh.count, p)) : sh.count) : 0u;
 #pragma unroll
-    for (int p = 0; p < 8; ++p) total += n[p];
+    for (int p = 0; p < kMaxParts; ++p) total += n[p];
     found = total <= kSampleList;
     if (found) {
       if (rank == 0) {
         unsigned at = 0;
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
+        for (int p = 0; p < kMaxParts; ++p) {
           if (p >= parts) break;
           for (unsigned i = tid; i < n[p]; i += kSampleThreads) sh.cand[at + i] = parts > 1 ? ld_peer_u64(peer_smem(&sh.list[i], p)) : sh.list[i];
           at += n[p];
         }
       }
-      if (parts > 1) cluster_sync(); else __syncthreads();  // nobody leaves while its list is being read
+      if (parts > 1) cluster_sync_all(); else __syncthreads();  // nobody leaves while its list is being read
       if (rank != 0) return;
       entries = total;
       lowest = bound;
@@ -401,10 +391,10 @@ sample_top_k_top_p_kernel(const bf16* __restrict__ logits, long long ld, int col
         }
       }
       entries = total;
-      if (parts > 1) cluster_sync();  // nobody leaves while its list is being read
+      if (parts > 1) cluster_sync_all();  // nobody leaves while its list is being read
       if (rank != 0) return;
     } else {
-      if (parts > 1) cluster_sync();  // nor while its histogram is
+      if (parts > 1) cluster_sync_all();  // nor while its histogram is
       if (rank != 0) return;
       // in index order: everything above the threshold, and the first need_eq entries equal to it
       const unsigned need_eq = K - above;
@@ -475,7 +465,7 @@ bool sample_by_bound(int cols, int top_k, int parts) {
 int sample_parts(int rows, int cols, int top_k) {
   const int sms = sm_count();
   const bool two = 2LL * rows <= sms, four = 9LL * rows <= 2 * sms;
-  int parts = !two || cols < 65536 ? 1 : (four && cols >= 98304 ? 4 : 2);
+  int parts = !two || cols < 65536 ? 1 : (four && cols >= 98304 ? kMaxParts : 2);
   while ((parts == 1 ? two : parts == 2 && four) && !sample_by_bound(cols, top_k, parts) && sample_by_bound(cols, top_k, 2 * parts)) parts *= 2;
   return parts;
 }
