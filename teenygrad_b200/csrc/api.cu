@@ -205,7 +205,7 @@ int matmul_forward_entry_point_f32(const float* a, const float* b, float* c, int
       !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
          reinterpret_cast<uintptr_t>(scratch)) & 15) &&
       scratch_bytes >= gemm_f32_split_scratch_bytes(M, N, K) &&
-      gemm_f32_split_clocks(M, N, K) < gemm_f32_clocks(a, K, 1, b, N, 1, M, N, K))
+      gemm_f32_split_clocks(M, N, K) < gemm_f32_clocks(a, K, 1, b, N, 1, c, N, 1, M, N, K))
     return gemm_f32_split(a, b, c, M, N, K, scratch, scratch_bytes, S(stream));
   return gemm_f32(a, K, 1, b, N, 1, nullptr, c, N, 1, M, N, K, S(stream));
 }

@@ -198,9 +198,11 @@ gemm_simt_kernel(const Operand<T> a, const Operand<T> b, const T* __restrict__ b
 // multiply-adds per clock that a tile reaches on a full SM, and the clocks that one of its slices takes when a chain of slices is all
 // there is.
 struct Choice { int bm, bn, kg; double rate, slice; };
+constexpr double kEndsChain = 2800.0, kEndsPipe = 5000.0;  // start and end of a launch that a chain, or rounds of tiles, bounds
 constexpr Choice kChoices[] = {{128, 128, 1, 92.0, 3500.0}, {64, 64, 2, 75.0, 2060.0}, {32, 64, 3, 55.0, 2130.0}, {16, 32, 6, 31.0, 1650.0}};
 
-// The tile that is estimated to end first: rounds of tiles over the SMs at the tile's rate, or the chain of slices if that is longer.
+// The tile that is estimated to end first: rounds of tiles over the SMs at the tile's rate, or the chain of slices if that is longer.  To `least`, which is
+// compared with the tensor cores' estimate, comes what a launch takes besides.
 // 1000 x 4096 x 1024: 128 x 128 at 199 us (64 x 64: 210); 512^3: 32 x 64 at 16.5 us (64 x 64: 23, 16 x 32: 23).  The one 64 x 64 tile
 // with 4 x 4 sums per thread that served every size before took 308 us and 50 us.  (Call by call, as in the table above; back to back in a
 // graph a call takes 2.4 us less: 14.1 for 512^3.)
@@ -208,6 +210,7 @@ constexpr Choice kChoices[] = {{128, 128, 1, 92.0, 3500.0}, {64, 64, 2, 75.0, 20
 // hold 128 sums each do not keep up with (1000 x 4096 x 1024, odd rows: 368 us with 128 x 128, 281 with 64 x 64; f32 216 and 242).
 int choose(long long M, long long N, long long K, int sms, double& least, int first = 0) {
   int best = first;
+  double ends = 0.0;
   least = 0.0;
   for (int i = first; i < 4; ++i) {
     const Choice& x = kChoices[i];
@@ -215,8 +218,9 @@ int choose(long long M, long long N, long long K, int sms, double& least, int fi
     const double pipe = static_cast<double>((tiles + sms - 1) / sms) * x.bm * x.bn * K / x.rate;
     const double chain = static_cast<double>((K + kTK * x.kg - 1) / (kTK * x.kg)) * x.slice;
     const double t = pipe > chain ? pipe : chain;
-    if (i == first || t < least) { least = t; best = i; }
+    if (i == first || t < least) { least = t; best = i; ends = pipe > chain ? kEndsPipe : kEndsChain; }
   }
+  least += ends;
   return best;
 }
 
@@ -256,11 +260,12 @@ int launch(const T* a, long long sam, long long sak, const T* b, long long sbk, 
 
 }  // namespace
 
-double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K) {
+double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, const float* c, long long scm,
+                       long long scn, int M, int N, int K) {
   double here;
   choose(M, N, K, sm_count(), here);
   if (!gemm_f32_tc_takes(sak, sbk, sbn, M, N, K)) return here;
-  const double there = gemm_f32_tc_clocks(a, sam, b, sbk, sbn, M, N, K);
+  const double there = gemm_f32_tc_clocks(a, sam, b, sbk, sbn, c, scm, scn, M, N, K);
   return there < here ? there : here;
 }
 
@@ -268,11 +273,13 @@ int gemm_f32(const float* a, long long sam, long long sak, const float* b, long 
              const float* bias, float* c, long long scm, long long scn, int M, int N, int K, cudaStream_t stream) {
   // On the tensor cores where that is estimated to end first, and always with a smaller error: from about 1 M multiply-adds per
   // SM on.  Back to back, [N][K]: 64 x 512 x 512 6.8 us here, 8.0 there; 34 x 288 x 536 7.2, 9.0; 512^3 14.1, 8.6; 64 x 4096 x 4096 93,
-  // 33.5; 300 x 700 x 2000 45.7, 14.5; 1000 x 2048 x 2048 236, 54.
+  // 33.5; 300 x 700 x 2000 45.7, 14.5; 1000 x 2048 x 2048 236, 54; [K][N]: 3490 x 136 x 136 11.9, 8.2; 1051 x 592 x 104 10.1, 7.3; rows
+  // of C off 32 bytes: 1325 x 801 x 88 9.4, 11.3.  Of 434 calls of random sizes with 16-byte rows the slower kernel is taken by more than 5 % in 19 (42 without the ends of
+  // a launch here and the stores of such rows there).
   if (a && b && c && gemm_f32_tc_takes(sak, sbk, sbn, M, N, K)) {
     double here;
     choose(M, N, K, sm_count(), here);
-    if (gemm_f32_tc_clocks(a, sam, b, sbk, sbn, M, N, K) < here) return gemm_f32_tc(a, sam, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
+    if (gemm_f32_tc_clocks(a, sam, b, sbk, sbn, c, scm, scn, M, N, K) < here) return gemm_f32_tc(a, sam, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
   }
   return launch<float>(a, sam, sak, b, sbk, sbn, bias, c, scm, scn, M, N, K, stream);
 }

@@ -163,11 +163,13 @@ int gemm_f32_split(const float* a, const float* b, float* c, int M, int N, int K
 // (k contiguous); B with either index contiguous.
 bool gemm_f32_tc_takes(long long sak, long long sbk, long long sbn, int M, int N, int K);
 int gemm_f32_tc_prepare();
-double gemm_f32_tc_clocks(const float* a, long long sam, const float* b, long long sbk, long long sbn, int M, int N, int K);  // estimated
+double gemm_f32_tc_clocks(const float* a, long long sam, const float* b, long long sbk, long long sbn, const float* c, long long scm, long long scn, int M,
+                          int N, int K);  // estimated
 int gemm_f32_tc(const float* a, long long sam, const float* b, long long sbk, long long sbn, const float* bias, float* c, long long scm,
                 long long scn, int M, int N, int K, cudaStream_t stream);
 // f32 GEMM with true f32 accuracy, on the tensor cores or the CUDA cores, whichever is estimated to end first (gemm_f32_clocks).  b_is_nk: B given as [N, K] (linear layout) instead of [K, N].
-double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, int M, int N, int K);
+double gemm_f32_clocks(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn, const float* c, long long scm,
+                       long long scn, int M, int N, int K);
 int gemm_f32(const float* a, long long sam, long long sak, const float* b, long long sbk, long long sbn,
              const float* bias, float* c, long long scm, long long scn, int M, int N, int K, cudaStream_t stream);
 // bf16 GEMM on CUDA cores for shapes the TMA path cannot take (unaligned strides / pointers).

@@ -84,6 +84,8 @@ def padded(M, K, ld, first, seed):
     ("gemm_f32_tc_kernelILi128ELb0ELb1EE", 600, 1000, 1001, 1001, 1004, 0), ("gemm_f32_tc_kernelILi128ELb0ELb1EE", 1290, 4100, 515, 515, 515, 3),
     ("gemm_f32_tc_kernelILi64ELb0ELb1EE", 300, 300, 2003, 2004, 2004, 1), ("gemm_f32_tc_kernelILi64ELb0ELb1EE", 300, 300, 2003, 0, 2003, 0),
     ("gemm_f32_tc_kernelILi32ELb0ELb1EE", 17, 70, 4001, 4005, 4001, 2), ("gemm_f32_tc_kernelILi32ELb0ELb1EE", 130, 70, 2003, 2003, 2003, 0),
+    # few chunks, where a launch's start and end decide; results that are not whole sectors
+    ("gemm_f32_tc_kernelILi64ELb1ELb0EE", 3490, 136, 136, 136, 136, 0), ("gemm_simt_kernel", 1325, 801, 88, 88, 88, 0), ("gemm_simt_kernel", 10, 776, 488, 488, 488, 0),
     # [K][N]: ldb is the stride of k
     ("gemm_f32_pair_kernelILb1EE", 1290, 4097, 579, 580, 4100, 0), ("gemm_f32_tc_kernelILi128ELb1ELb0EE", 300, 1002, 1001, 1004, 1004, 0),
     ("gemm_f32_tc_kernelILi64ELb1ELb0EE", 130, 1001, 2003, 2004, 1004, 4),
@@ -101,8 +103,8 @@ def test_f32_linears(ops, kernel, M, N, K, lda, ldb, first):
     ops.linear_forward(x, w, bias, out=out)
     e, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
     # a sum of 64 k is cut off at most 24 times by 2^-23 of the products' sizes, the sums of K / 64 such and of up to eight parts are rounded, and the
-    # terms left out are below 3 * 2^-24
-    assert bool(((out.double() - e - bias.double()).abs() <= (48 + K // 64 + 12) * 2.0 ** -24 * size + 2.0 ** -23 * (e.abs() + bias.double().abs())).all())
+    # terms left out are below 3 * 2^-24; f32 multiply-adds in one chain round K times
+    assert bool(((out.double() - e - bias.double()).abs() <= max(48 + K // 64 + 12, K if "simt" in kernel else 0) * 2.0 ** -24 * size + 2.0 ** -23 * (e.abs() + bias.double().abs())).all())
     assert ops.device_error() == 0
 
 
