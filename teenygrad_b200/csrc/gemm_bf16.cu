@@ -1092,11 +1092,19 @@ int gemm_bf16(const bf16* x, int ldx, const bf16* w, int ldw, bool w_is_kn, cons
   const int sms = sm_count();
   LargeChoice large{};
   if (!w_is_kn && !push && (M > kSwapMaxM || !w_early)) {
-    const bool lines = ldx % 64 == 0 && ldw % 64 == 0 && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 127);
+    const auto rows_on = [&](int bytes) { return ldx * 2 % bytes == 0 && ldw * 2 % bytes == 0 && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & (bytes - 1)); };
+    const bool lines = rows_on(128);
     const SplitChoice split = gemm_bf16_split_choose(M, N, K, lines, sms);
     if (M > kSwapMaxM) large = choose_large(M, N, ceil_div(K, kBK), sms);
-    if (!lines) large.us *= 1.25;  // 654 x 2128 x 2104 18.5 us (estimated 14.2), 937 x 4120 x 1840 22.2 (17.5), 2011 x 800 x 6744 46.7 (34.7)
-    if (split.bn && (M <= kSwapMaxM || split.us < large.us)) return gemm_bf16_split(x, ldx, w, ldw, bias, y, ldy, M, N, K, split.bn, split.split, swiglu, stream);
+    // Rows that start off 128 bytes: the split tiles' estimate is then for rows off the 32-byte sectors too, which cost a row of a tile a fifth sector, and a quarter too
+    // high for rows on them.  So the others' go up as much; off the sectors narrow tiles suffer more, and pairs, whose CTAs load half as much, little (measured
+    // against the estimates, rows on sectors and off them: narrow 0.98, 1.33, pairs 0.94, 1.10, split 0.80, 1.03): 350 x 6464 x 8104 pairs 54.9 us, split 67.7, 1278 x
+    // 2384 x 3464 29.2 and 36.0; 1158 x 1680 x 2760 narrow 23.4, split 20.4.  Of 372 calls the slower kernel is taken by 3 % or more in 24 (38 with 1.25 for all).
+    if (!lines) large.us *= rows_on(32) ? 1.25 : (large.kind == kLargeNarrow ? 1.35 : (large.kind == kLargeWide ? 1.1 : 1.06));
+    // Up to 16 tokens the decode GEMM, two CTAs an SM, is ahead where clusters of two do not find place and single CTAs leave much of the GPU idle, if there is
+    // enough K: 3 x 10816 x 4032 14.1 us split, 12.0 there, 6 x 10048 x 9152 33.0 and 31.4, 9 x 10112 x 3264 14.4 and 14.5; 20 to 31 tokens 0.94 to 1.08 of it
+    const bool idle = M <= 16 && split.split == 1 && 100 * ceil_div(N, kBM) <= 60 * sms && K >= 2688;
+    if (split.bn && (M <= kSwapMaxM ? !idle : split.us < large.us)) return gemm_bf16_split(x, ldx, w, ldw, bias, y, ldy, M, N, K, split.bn, split.split, swiglu, stream);
   }
   GemmArgs a{};
   a.M = M; a.N = N; a.K = K; a.ldy = ldy; a.y = y; a.y32 = y32; a.bias = bias;

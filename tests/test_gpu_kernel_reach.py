@@ -28,7 +28,9 @@ def check_product(y, x, w, bias=None):
     ("gemm_bf16_kernelILi128ELb0ELb0EE", 1290, 6152, 264), ("gemm_bf16_kernelILi128ELb0ELb0EE", 4100, 3000, 72), ("gemm_bf16_kernelILi128ELb0ELb0EE", 257, 6152, 4104),
     ("gemm_bf16_kernelILi256ELb0ELb0EE", 257, 12296, 2056), ("gemm_bf16_kernelILi256ELb0ELb0EE", 1290, 6152, 520),
     ("gemm_bf16_2cta_kernel", 700, 9224, 1032), ("gemm_bf16_2cta_kernel", 2000, 2056, 8200), ("gemm_bf16_2cta_kernel", 3001, 3000, 264),
-    ("gemm_bf16_split_kernelILi32EE", 129, 1000, 1032), ("gemm_bf16_split_kernelILi32EE", 200, 136, 2056),
+    ("gemm_bf16_2cta_kernel", 350, 6464, 8104), ("gemm_bf16_2cta_kernel", 1278, 2384, 3464),  # rows off the 32-byte sectors, which pairs mind least
+    ("gemm_bf16_skinny_kernelILi16ELb0ELb0EE", 3, 10816, 4032), ("gemm_bf16_skinny_kernelILi16ELb0ELb0EE", 16, 9601, 2696),
+    ("gemm_bf16_split_kernelILi32EE", 17, 9601, 2696), ("gemm_bf16_split_kernelILi32EE", 129, 1000, 1032), ("gemm_bf16_split_kernelILi32EE", 200, 136, 2056),
     ("gemm_bf16_split_kernelILi64EE", 257, 520, 2056), ("gemm_bf16_split_kernelILi64EE", 129, 520, 8200), ("gemm_bf16_split_kernelILi64EE", 999, 1000, 264),
     ("gemm_bf16_split_kernelILi128EE", 700, 2056, 264), ("gemm_bf16_split_kernelILi128EE", 385, 520, 4104), ("gemm_bf16_split_kernelILi128EE", 200, 6152, 520),
     ("gemm_bf16_split_kernelILi192EE", 129, 3000, 4104), ("gemm_bf16_split_kernelILi192EE", 257, 4104, 2056), ("gemm_bf16_split_kernelILi192EE", 1290, 2056, 520),
