@@ -21,8 +21,9 @@
 // Bound: the issue slots.  A tile of 128 keys (D = 64) is 3100 clocks of the tensor pipe at its best and about 3400 issue slots of each scheduler, half of them
 // the split of K and V, which every CTA of a head repeats; 5200 are taken, the chain being the split of a key tile, its 24 MMAs, and the next split into
 // the same place (both operands of one tile twice do not fit beside Q).  With two places for K and one for V a tile took 7000 clocks.
-// Measured on B200 against the CUDA-core kernel, f32, 32 heads x 1000 x 1000: D = 64 279 -> 61 us, error against 64 bits 6.0e-7 -> 1.9e-7, D = 128 561 -> 130 us,
-// 6.0e-7 -> 1.9e-7; 8 heads x 300 x 300, D = 64 37 -> 15.5 us, 3.6e-7 -> 1.7e-7; bf16, 32 heads x 1000 x 1000, D = 64 312 -> 41 us.
+// Measured on B200 back to back against the CUDA-core kernel, f32, 32 heads x 1000 x 1000: D = 64 278 -> 59.5 us (called alone 288 -> 66.7), error against 64 bits
+// 6.0e-7 -> 1.9e-7, D = 128 560 -> 131 us, 6.0e-7 -> 1.9e-7; 8 heads x 300 x 300, D = 64 37 -> 15.8 us, 3.6e-7 -> 1.7e-7; bf16, 32 heads x 1000 x 1000, D = 64 312 ->
+// 41 us.  Tensor pipe 42 % active (D = 128 39 %).  f32 with D = 128 spills 36 bytes a thread (stored; 88 loaded), the others none.
 #include <atomic>
 #include <cmath>
 #include <type_traits>

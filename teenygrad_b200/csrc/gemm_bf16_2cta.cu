@@ -12,8 +12,10 @@
 //   warp 1   MMA issuer (leader only).  commit -> `empty` barrier of both CTAs; after the last k-block -> `acc_full`
 //            of both CTAs.
 //   warp 2   allocates / frees tensor memory (both CTAs, cta_group::2).
-//   warps 2-5 epilogue (both CTAs): tcgen05.ld the CTA's 128 x 256 f32 half, bf16, 16-byte stores; then arrive on
-//            the leader's `acc_empty` (the peer does so through a cluster-mapped address).
+//   warps 2-9 epilogue (both CTAs, four warps 128 columns): tcgen05.ld the CTA's 128 x 256 f32 half, bf16, through shared memory and TMA to Y
+//            (16-byte stores where no map describes it); then arrive on the leader's `acc_empty` (the peer does so through a
+//            cluster-mapped address).  Ten warps have 168 registers a thread; the fused QKV epilogue, which holds a head's 64 packed
+//            words, spills 184 bytes (stored; 340 loaded) once a tile.
 // Two accumulators in tensor memory (2 x 256 columns) let the epilogue of tile t overlap the main loop of tile t+1.
 #include <atomic>
 

@@ -13,8 +13,8 @@
 //     470 clocks to issue by a lone lane, now 255, which is what its four MMAs take);
 //   * the ring is requested before tensor memory is there and the CTA meets; eight warps move the sums, by code for each cluster width.
 // 128 x 4096 x 4096 now: last MMA done 6000, parted 6700, received 8700, stored 10100, gone 10500.
-// Measured back to back on B200 (M x N x K, us, before -> now): 32 x 4096 x 4096 10.8 -> 8.6, 64 x 4096 x 4096 12.4 -> 9.6, 128 x 4096 x 4096 15.4 -> 11.9, 128 x 1024 x 1024
-// 8.2 -> 4.5, 151 x 1944 x 704 11.0 -> 4.9, 512 x 1024 x 3072 12.9 -> 7.6, 512 x 6144 x 1024 13.8 -> 9.1, 1349 x 912 x 832 10.9 -> 6.5, 16 x 1120 x 8048 9.0 -> 6.3.
+// Measured back to back on B200 (M x N x K, us, before -> now): 32 x 4096 x 4096 10.2 -> 6.5, 64 x 4096 x 4096 11.3 -> 7.7, 128 x 4096 x 4096 13.9 -> 8.6 (called alone 16.4 ->
+// 12.3), 151 x 1944 x 704 11.2 -> 4.8, 512 x 1024 x 3072 12.7 -> 7.7.
 #include <atomic>
 #include <cmath>
 

@@ -15,9 +15,10 @@
 // Tried: the splitting warps in two teams of four, each every other chunk, to hide the latency: 64 k of 128, 64 and 32 columns 2400, 1540 and 1200 clocks instead
 // of 2680, 1670 and 1560, but a launch's first chunk later, 1000 x 4096 x 1024 40.6 us for 38.2, 512^3 9.3 for 8.8.  Two terms of B as one MMA of
 // twice the columns in narrow tiles: no faster, errors up to 15 % larger.
-// Measured (f32 rows split by the warps that loaded them, one CTA to a tile -> now): 1000 x 4096 x 1024 72 -> 43 us, 2048 x 4096 x 4096 473 -> 271,
-// 2048 x 2048 x 2048 [K][N] 121 -> 72, 594 x 780 x 652 25 -> 12.8, 300 x 700 x 2000 17 -> 14.5, 512^3 9.65 -> 8.6; error against 64 bits the same or smaller (8e-8 to
-// 1.3e-7; f32 multiply-adds 1.2e-6 for 2048 x 4096 x 4096).
+// Measured back to back (f32 rows split by the warps that loaded them, one CTA to a tile -> now): 1000 x 4096 x 1024 63 -> 39 us (with bias called alone 74 -> 50),
+// 2048 x 4096 x 4096 478 -> 273, 2048 x 2048 x 2048 [K][N] 123 -> 72, 594 x 780 x 652 25 -> 13.3, 300 x 700 x 2000 16.8 -> 15.1, 512^3 9.6 -> 8.8; error against 64 bits the
+// same or smaller (8e-8 to 1.3e-7; f32 multiply-adds 1.2e-6 for 2048 x 4096 x 4096).  Tensor pipe 92 % active with 128 tiles on 74 pairs.  The pairs' kernel spills
+// 112 bytes a thread (stored; 284 loaded) with B as [N][K], 56 (96) with [K][N]: their roles have 80 and 176 registers.
 //
 // bf16 has the exponents of f32 but only eight bits, so the terms of a small number would run out of exponent: the third below 2^-110, all
 // three below 2^-134.  Both operands are therefore taken times 2^24, with which every term of every f32 number, the smallest subnormal
