@@ -16,9 +16,9 @@ def kernels(f):
     with torch.cuda.graph(graph):
         f()
     raw = driver.CUgraph(graph.raw_cuda_graph())
-    nodes, _ = _done(driver.cuGraphGetNodes(raw, _done(driver.cuGraphGetNodes(raw, 0))[1])), None
+    count = _done(driver.cuGraphGetNodes(raw, 0))[1]
     names = []
-    for node in nodes[0]:
+    for node in _done(driver.cuGraphGetNodes(raw, count))[0]:
         if _done(driver.cuGraphNodeGetType(node))[0] != driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
             continue
         p, = _done(driver.cuGraphKernelNodeGetParams(node))
